@@ -38,7 +38,7 @@ enum : uint8_t { COL_INVARIANT = 0, COL_MASKED = 1, COL_VARIANT = 2 };
 struct InstDev {
     int T, internal, minage, nleaves, nnodes, nseqs, seqlen, ntrees;
     int block0;           // first block of this instance in the batch
-    int pad;
+    int maxS;             // states of its largest local tree (at least 1)
     long long cell0;      // forward-table offset of column 0
     long long col0;       // offset into per-column arrays
     long long seq0;       // offset of the column-major sequences [seqlen][nseqs]
@@ -99,7 +99,9 @@ struct BatchDev {
     double *gts;                 // [total M] get_time(a, b, c, same_node=true) rows
     double *inv_lk;              // [total states] invariant-site emission per state
     int *determ;                 // [total states] switch: target of state j of prev tree
-    double *determprob;          // [total states]
+    double *determprob;          // [total states]; FP32 path: once a tree's table is built, a
+                                 // slot's first float holds the move as a complement, 1 - p,
+                                 // when p >= 1/2, else -p (sign bit set)
     int2 *srcs;                  // [nblocks] {recombsrc, recoalsrc}
     double *recombrow, *recoalrow;  // [total states] dense rows over this block's states
     int *gptr;                   // [total states + nblocks] gather CSR pointers

@@ -13,6 +13,7 @@
 
 #include <cuda_runtime.h>
 
+#include "f2.cuh"
 #include "kernels.h"
 
 namespace awg {
@@ -39,32 +40,6 @@ template <> struct BTab<float> {
           rrow(d.recombrow32), crow(d.recoalrow32), t2d(d.t2d32), fw(d.fw32) {}
     __device__ float t2(long long idx, float) const { return t2d[idx]; }
 };
-
-// FP32 pair arithmetic for the dominant path of the FP32 backward step (the same reason
-// and transforms as the forward's: the column's fixed point within a tree would otherwise
-// move by the step's rounding over one minus the chain's contraction).
-struct F2 {
-    float hi, lo;
-};
-__device__ __forceinline__ F2 f2_renorm(float a, float b) {  // |a| >= |b|
-    const float s = a + b;
-    return F2{s, b - (s - a)};
-}
-__device__ __forceinline__ F2 f2_keep(F2 x, float r) {  // x * (1 - r), 0 <= r < 1
-    const float t = x.hi * r;
-    const float h = x.hi - t;
-    return f2_renorm(h, ((x.hi - h) - t) + x.lo);
-}
-__device__ __forceinline__ F2 f2_mul(F2 x, float e) {
-    const float p = x.hi * e;
-    return f2_renorm(p, fmaf(x.hi, e, -p) + x.lo * e);
-}
-__device__ __forceinline__ F2 f2_add(F2 x, float s) {
-    const float h = x.hi + s;
-    const float bb = h - x.hi;
-    const float err = (x.hi - (h - bb)) + (s - bb);
-    return f2_renorm(h, err + x.lo);
-}
 
 template <typename F>
 __device__ __forceinline__ F warp_sum(F v) {
@@ -262,7 +237,7 @@ __global__ void k_backward(BatchDev d, int maxS, double *bw_out) {
             const int2 src = d.srcs[I.block0 + bi];
             const int *determ = d.determ + B.prev_state0;
             const F *dp = tab.dprob + B.prev_state0;
-            const double *dp64 = d.determprob + B.prev_state0;
+            const float2 *mv = (const float2 *)(d.determprob + B.prev_state0);
             const F *rr = tab.rrow + B.state0;
             const F *cr = tab.crow + B.state0;
             for (int j = tid; j < n1; j += blockDim.x) {
@@ -274,9 +249,8 @@ __global__ void k_backward(BatchDev d, int maxS, double *bw_out) {
                         if (row[k] > F(0)) s += row[k] * g[k];
                 } else if (determ[j] >= 0) {
                     if constexpr (BTab<F>::split) {
-                        const double pj = dp64[j];
                         const F2 x{g[determ[j]], glo[determ[j]]};
-                        const F2 y = pj >= 0.5 ? f2_keep(x, (float)(1.0 - pj)) : f2_mul(x, (float)pj);
+                        const F2 y = f2_move(x, mv[j].x);
                         s = y.hi;
                         slo = y.lo;
                     } else {

@@ -333,7 +333,7 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
     const size_t o_bw = w.add(want_bw ? sizeof(double) * CELLS : 0);
     const size_t o_path = w.add(want_path ? sizeof(int) * COLS : 0);
     // FP32 traceback: the forward columns' time-bin sums
-    const bool want_bins = fp32 && want_path && forward_writes_bins(plan.maxS, plan.maxM, plan.maxT, cfg.kpt);
+    const bool want_bins = fp32 && want_path && forward_writes_bins(plan.maxS);
     const size_t o_bins = w.add(want_bins ? sizeof(float) * MAXT * COLS : 0);
     const size_t o_err = w.add(4 * sizeof(int));
     const size_t o_queue = w.add(sizeof(int) * 2 * MAXG);  // work counters of the groups

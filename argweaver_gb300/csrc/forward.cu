@@ -34,6 +34,7 @@
 
 #include <cstdlib>
 
+#include "f2.cuh"
 #include "kernels.h"
 
 namespace awg {
@@ -409,45 +410,6 @@ __global__ void __launch_bounds__(512) k_forward(BatchDev d, int maxS, int maxM,
 // holds its sub-partition's FP64 pipe for about 64 cycles and a dependent FP64 step costs a
 // few hundred cycles, so the plain FP64 path is shaped to issue few FP64 instructions in
 // short dependent chains.
-// FP32 pair arithmetic (value = hi + lo, |lo| <= ulp(hi) / 2) for the dominant path of
-// the FP32 forward step. Within a tree the normalised column converges to the fixed point
-// of the step; a rounding error of the step shifts that fixed point by about the error
-// divided by (1 - the chain's contraction), and with stay probabilities near 1 the
-// contraction is slow. The stay, emission and rescaling factors, which carry almost all of
-// a state's mass from column to column, therefore run on pairs built from error-free
-// transforms (Fast2Sum, and products split by FMA); the mass moving in from other states
-// (a few percent) stays plain FP32.
-struct F2 {
-    float hi, lo;
-};
-__device__ __forceinline__ F2 f2_renorm(float a, float b) {  // |a| >= |b|
-    const float s = a + b;
-    return F2{s, b - (s - a)};
-}
-// (x.hi + x.lo) * (1 - r), 0 <= r < 1 (x.lo * r dropped: below the pair's precision)
-__device__ __forceinline__ F2 f2_keep(F2 x, float r) {
-    const float t = x.hi * r;
-    const float h = x.hi - t;
-    return f2_renorm(h, ((x.hi - h) - t) + x.lo);
-}
-// x * e
-__device__ __forceinline__ F2 f2_mul(F2 x, float e) {
-    const float p = x.hi * e;
-    return f2_renorm(p, fmaf(x.hi, e, -p) + x.lo * e);
-}
-// x + s (any magnitudes: two-sum)
-__device__ __forceinline__ F2 f2_add(F2 x, float s) {
-    const float h = x.hi + s;
-    const float bb = h - x.hi;
-    const float err = (x.hi - (h - bb)) + (s - bb);
-    return f2_renorm(h, err + x.lo);
-}
-// x + y, both pairs
-__device__ __forceinline__ F2 f2_add2(F2 x, F2 y) {
-    const F2 s = f2_add(x, y.hi);
-    return f2_renorm(s.hi, s.lo + y.lo);
-}
-
 constexpr int NRW = 4;                      // reduction warps of the register variant
 constexpr int RBINS = (MAXT - 1 + NRW - 1) / NRW;  // time bins per reduction warp (<= 8)
 
@@ -727,13 +689,11 @@ __global__ void __launch_bounds__(512) k_forward_reg(BatchDev d, int maxS, int m
                     // pairs: the previous column's values with their low parts, each
                     // deterministic move by its FP64 probability (kept as a complement near
                     // 1), the recombination rows (a small inflow) plain, then the emission
-                    const double *dp64 = d.determprob + B.prev_state0;
+                    const float2 *mv = (const float2 *)(d.determprob + B.prev_state0);
                     F2 a{0.0f, 0.0f};
                     for (int p = gp[k]; p < gp[k + 1]; p++) {
                         const int j = gi[p];
-                        const double pj = dp64[j];
-                        const F2 xj{prev[j], lastlo[j]};
-                        a = f2_add2(a, pj >= 0.5 ? f2_keep(xj, (float)(1.0 - pj)) : f2_mul(xj, (float)pj));
+                        a = f2_add2(a, f2_move(F2{prev[j], lastlo[j]}, mv[j].x));
                     }
                     if (src.x != -1 && rr[k] > F(0)) a = f2_add(a, prev[src.x] * rr[k]);
                     if (src.y != -1 && cr[k] > F(0)) a = f2_add(a, prev[src.y] * cr[k]);
@@ -1271,13 +1231,6 @@ void launch(const BatchDev &d, cudaStream_t s, int want_kpt) {
 
 }  // namespace
 
-bool forward_writes_bins(int maxS, int maxM, int maxT, int kpt) {
-    (void)maxM;
-    (void)maxT;
-    const int k = reg_kpt(imax(maxS, 1), kpt);
-    return 32 * NRW + imax(32, ((imax(maxS, 1) + k - 1) / k + 31) / 32 * 32) <= 512;
-}
-
 void launch_forward_dense(const BatchDev &d, cudaStream_t s) {
     const int maxS = imax(d.maxS, 1);
     const size_t smem = 2 * (size_t)maxS * sizeof(double) + 2 * (size_t)maxS * sizeof(int);
@@ -1288,8 +1241,8 @@ void launch_forward_dense(const BatchDev &d, cudaStream_t s) {
 }
 
 void launch_forward(const BatchDev &d, bool fp32, cudaStream_t s, int kpt) {
-    if (fp32) launch<float>(d, s, kpt);
-    else launch<double>(d, s, kpt);
+    if (!fp32) launch<double>(d, s, kpt);
+    else if (!launch_forward32(d, s, kpt)) launch_old<float>(d, d.maxM, s);
 }
 
 }  // namespace awg

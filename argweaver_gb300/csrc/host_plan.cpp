@@ -320,7 +320,7 @@ bool plan_layout(const awg_problem *probs, int n, HostPlan &plan, std::string &e
         InstDev &I = plan.inst[q];
         I.T = p.ntimes; I.internal = p.internal ? 1 : 0; I.minage = p.minage;
         I.nleaves = nleaves; I.nnodes = p.nnodes; I.nseqs = nemit; I.seqlen = p.seqlen;
-        I.ntrees = p.ntrees; I.block0 = o.blk; I.pad = 0;
+        I.ntrees = p.ntrees; I.block0 = o.blk; I.maxS = tot[q].maxS;
         I.cell0 = o.cell; I.col0 = o.col; I.seq0 = o.seq; I.model0 = (long long)q * MODEL_STRIDE;
 
         model_arrays(p.times, p.popsizes, p.ntimes, p.rho, p.mu, p.infsites_penalty,

@@ -38,7 +38,9 @@ int dense_tables(const BatchDev &d, int kind, const int *rows, int nr, const int
 // Whether K3 writes the FP32 columns' time-bin sums (BatchDev::bins32) for a batch of these
 // largest sizes (the register-resident variant does; the fallback for the largest trees
 // does not).
-bool forward_writes_bins(int maxS, int maxM, int maxT, int kpt = 0);
+bool forward_writes_bins(int maxS);
+// K3, FP32, where a CTA takes trees of this size (else false: nothing launched).
+bool launch_forward32(const BatchDev &d, cudaStream_t s, int kpt);
 // K4: stochastic traceback, one warp per instance; FP32 with bins32 set: the decomposed draw.
 void launch_traceback(const BatchDev &d, bool fp32, cudaStream_t s);
 // K5: backward pass fused with the posterior marginals, one CTA per instance.
