@@ -204,8 +204,9 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
     plan = HostPlan();
     if (!plan_layout(probs, n, plan, err, false)) return -1;  // bytes: checked by plan_fill
 
-    bool want_path = false, want_post = false, want_bw = false;
+    bool want_path = false, want_post = false, want_bw = false, want_fw = false;
     for (int q = 0; q < n; q++) {
+        want_fw |= outs[q].forward != nullptr;
         want_path |= outs[q].path != nullptr;
         want_post |= outs[q].posterior != nullptr;
         if (opt.backward && opt.backward[q]) want_bw = true;
@@ -522,7 +523,7 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
                 cudaStream_t gs = C.gstream[g];
                 EQ(cudaEventRecord(C.gev[2 * g], s));
                 EQ(cudaStreamWaitEvent(gs, C.gev[2 * g], 0));
-                launch_forward(dg, fp32, gs, cfg.kpt);
+                launch_forward(dg, fp32, gs, cfg.kpt, want_fw);
                 EQ(cudaGetLastError());
                 if (want_path) {
                     launch_traceback(dg, fp32, gs);
@@ -540,7 +541,7 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
             EQ(cudaGetLastError());
             launch_varemit(d, fp32, s, qp(1), cfg.chunk);
             EQ(cudaGetLastError());
-            launch_forward(d, fp32, s, cfg.kpt);
+            launch_forward(d, fp32, s, cfg.kpt, want_fw);
             EQ(cudaGetLastError());
             if (want_path) {
                 launch_traceback(d, fp32, s);
@@ -566,7 +567,7 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         if (E.graphs && C.graphs) {
             // everything a launch depends on: buffers, counts, groups and schedule knobs
             std::vector<long long> sig = {(long long)(uintptr_t)D, (long long)fp32, want_path,
-                                          want_post, want_bw, want_bins, plan.ninst, plan.nblocks,
+                                          want_post, want_bw, want_fw, want_bins, plan.ninst, plan.nblocks,
                                           plan.maxS, plan.maxT, plan.maxnodes, plan.maxM,
                                           cfg.kpt, cfg.chunk, cfg.group_div, cfg.persistent, ng,
                                           (long long)total, d.emit64, d.vardf};
@@ -679,7 +680,7 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         CKL("emission kernel");
         if (T) CK(cudaEventRecord(C.ev[3], s));
         if (opt.dense) launch_forward_dense(d, s);
-        else launch_forward(d, fp32, s, cfg.kpt);
+        else launch_forward(d, fp32, s, cfg.kpt, want_fw);
         CKL("forward kernel");
         if (T) CK(cudaEventRecord(C.ev[4], s));
         if (want_path) {

@@ -21,9 +21,11 @@ void launch_varemit(const BatchDev &d, bool want32, cudaStream_t s, int *queue =
 // Whether K2's carve with FP64 per-state factors and 8-byte scratch (needed for FP64 and
 // double-float emissions) fits this largest tree.
 bool varemit_full_carve_fits(int maxnodes, int maxS);
-// K3: forward pass, one CTA per instance; kpt: states per owner thread of the
-// register-resident variant (0: chosen by the state count).
-void launch_forward(const BatchDev &d, bool fp32, cudaStream_t s, int kpt = 0);
+// K3: forward pass, one CTA per instance; kpt: at least this many states per owner thread of
+// the FP32 kernel (0: chosen by the state count). table: the FP64 table is to be read, so its
+// columns are normalised (else each is left on a power-of-two scale of its own, which the
+// traceback and the posterior do not see).
+void launch_forward(const BatchDev &d, bool fp32, cudaStream_t s, int kpt = 0, bool table = true);
 // K3 with the reference's dense test step (arghmm_forward_block_slow), FP64.
 void launch_forward_dense(const BatchDev &d, cudaStream_t s);
 
@@ -39,8 +41,11 @@ int dense_tables(const BatchDev &d, int kind, const int *rows, int nr, const int
 // largest sizes (the register-resident variant does; the fallback for the largest trees
 // does not).
 bool forward_writes_bins(int maxS);
-// K3, FP32, where a CTA takes trees of this size (else false: nothing launched).
+// The forms of K3 and K5 for trees that a CTA's owner threads hold (else false: nothing
+// launched).
 bool launch_forward32(const BatchDev &d, cudaStream_t s, int kpt);
+bool launch_forward64(const BatchDev &d, cudaStream_t s, bool table);
+bool launch_backward_chain(const BatchDev &d, bool fp32, double *bw_out, cudaStream_t s);
 // K4: stochastic traceback, one warp per instance; FP32 with bins32 set: the decomposed draw.
 void launch_traceback(const BatchDev &d, bool fp32, cudaStream_t s);
 // K5: backward pass fused with the posterior marginals, one CTA per instance.
