@@ -1,23 +1,21 @@
-// K4: stochastic traceback, one warp per instance (stochastic_traceback,
-// sample_thread.cpp:522-569; sample_hmm_posterior :470-503; sample_hmm_posterior_step
-// :506-519; sample, common.h:272-290).
+// K4: stochastic traceback (stochastic_traceback, sample_thread.cpp:522-569;
+// sample_hmm_posterior :470-503; sample_hmm_posterior_step :506-519; sample,
+// common.h:272-290). Column i draws path[i] from A[j] = fw[i][j] * P(j -> path[i+1]) with the
+// uniform u[i]: the first j whose running sum reaches u[i] * sum(A). Three kernels, one block
+// per instance:
+//   k_traceback64     FP64: the reference's scan, a CTA testing many columns at once
+//   k_traceback_split FP32: the draw decomposed by the structure of the transition
+//   k_traceback       FP32 where the decomposed draw's tables do not fit: the scan, one warp
 //
-// Column i draws path[i] from A[j] = fw[i][j] * P(j -> path[i+1]) with the uniform u[i]:
-// the first j whose running sum reaches u[i] * sum(A). The warp splits the states into 32
-// contiguous chunks (lane t sums chunk t with two accumulators, even and odd states); chunk
-// sums are scanned across lanes and the chunk that holds the pick is rescanned by all
-// lanes at once.
-//
-// Speculation over columns: the transition row P(. -> k) changes only when the sampled
-// state does, which is rare inside a local tree. The warp therefore samples G columns at
-// once under the current row, every column's sums computed exactly as if it were alone,
-// and keeps the draws up to and including the first one that leaves state k; the rest are
-// redone under the new row. The path is the same as one column at a time, draw for draw.
-//
-// The forward table is read from HBM once, newest column first: columns stream into a
-// shared-memory ring DEPTH columns ahead of the sampler with 16-byte cp.async (a column's
-// start is rounded down to 16 bytes and the slot keeps the offset), each column's uniform
-// beside it, so HBM latency overlaps the sampling of earlier groups.
+// The scan by one warp splits the states into 32 contiguous chunks (lane t sums chunk t with
+// two accumulators, even and odd states); chunk sums are scanned across lanes and the chunk
+// that holds the pick is rescanned by all lanes at once. The transition row P(. -> k) changes
+// only when the sampled state does, which is rare inside a local tree, so the warp samples G
+// columns at once under the current row, every column's sums computed exactly as if it were
+// alone, and keeps the draws up to and including the first one that leaves state k; the rest
+// are redone under the new row. Columns stream into a shared-memory ring DEPTH columns ahead
+// of the sampler with 16-byte cp.async (a column's start is rounded down to 16 bytes and the
+// slot keeps the offset), each column's uniform beside it.
 
 #include <cuda_runtime.h>
 
@@ -29,16 +27,6 @@ namespace awg {
 namespace {
 
 template <typename F> struct TTab;
-template <> struct TTab<double> {
-    static constexpr bool split = false;
-    const float *rstay = nullptr;
-    const double *tm, *gts, *dprob, *rrow, *crow, *fw;
-    __device__ explicit TTab(const BatchDev &d)
-        : tm(d.tm), gts(d.gts), dprob(d.determprob), rrow(d.recombrow), crow(d.recoalrow),
-          fw(d.fw64) {}
-    // same-node entry: get_time(a, b, c, minage, true)
-    __device__ double same(long long idx, double) const { return gts[idx]; }
-};
 template <> struct TTab<float> {
     static constexpr bool split = true;  // t2d32 excludes the diagonal's stay term
     const float *rstay;
@@ -124,18 +112,7 @@ __device__ int warp_sample(int n, double u, W w) {
     return finish_sample<F>(n, chunk, incl, (F)u * total, lo, hi, lane, w);
 }
 
-// QL: four lanes per column (G = 8): lane 4g + q runs quarter q of column g's states in
-// order, keeping each running sum in shared memory, so that a column's draw needs a 4-lane
-// scan and a binary search of the stored sums instead of a 32-lane scan and a rescan; the
-// fewer warp-wide FP64 instructions suit the FP64 path, whose every warp instruction holds
-// the sub-partition's FP64 pipe for about 64 cycles. For trees of up to QL_MAXS states.
-constexpr int QL_MAXS = 256;
-
-// The order of non-negative values as integers (their bit patterns order the same way).
-__device__ __forceinline__ long long order_key(double x) { return __double_as_longlong(x); }
-__device__ __forceinline__ long long order_key(float x) { return __float_as_int(x); }
-
-template <typename F, int G, int DEPTH, bool QL>
+template <typename F, int G, int DEPTH>
 __global__ void k_traceback(BatchDev d, int maxS, int slot_elems) {
     extern __shared__ double dyn_d[];
     F *ring = (F *)dyn_d;                                   // [DEPTH][slot_elems], 16-B slots
@@ -143,8 +120,6 @@ __global__ void k_traceback(BatchDev d, int maxS, int slot_elems) {
     F *trans = (F *)(uring + DEPTH);                        // [maxS]
     int *stime = (int *)(trans + maxS + (maxS & 1));        // [maxS] state times of the tree
     int *snode = stime + maxS;                              // [maxS]
-    // QL: [G][maxS + 1] running sums (after the ints, 8-byte aligned)
-    F *pre = (F *)((char *)dyn_d + (((char *)(snode + maxS) - (char *)dyn_d + 15) & ~(size_t)15));
     __shared__ F tmS[MAXT * MAXT];
     const TTab<F> tab(d);
     const int qi = cta_instance(d);
@@ -251,56 +226,7 @@ __global__ void k_traceback(BatchDev d, int maxS, int slot_elems) {
 #pragma unroll
             for (int g = 0; g < G; g++) cg[g] = column(B, c0 - imin(g, ng - 1));
             int res[G];
-            if constexpr (QL) {
-                static_assert(G == 8, "four lanes per column of eight");
-                const int g = lane >> 2, q = lane & 3;
-                const int qs = (Sm + 3) >> 2;
-                const int qlo = imin(q * qs, Sm), qhi = imin(qlo + qs, Sm);
-                const int mycol = c0 - imin(g, ng - 1);
-                const F *cp = column(B, mycol);
-                F *pg = pre + g * (maxS + 1);
-                F run = 0;
-                for (int j = qlo; j < qhi; j++) {
-                    run = fma(cp[j], trans[j], run);
-                    pg[j] = run;
-                }
-                // inclusive scan of the quarters' sums within the column's four lanes
-                F incl = run;
-                F v = __shfl_up_sync(0xffffffffu, incl, 1);
-                if (q >= 1) incl += v;
-                v = __shfl_up_sync(0xffffffffu, incl, 2);
-                if (q >= 2) incl += v;
-                F excl = __shfl_up_sync(0xffffffffu, incl, 1);
-                if (q == 0) excl = 0;
-                const F total = __shfl_sync(0xffffffffu, incl, lane | 3);
-                const F pick = (F)uring[mycol % DEPTH] * total;
-                const unsigned hit = __ballot_sync(0xffffffffu, incl >= pick && qhi > qlo);
-                __syncwarp();  // the running sums are stored
-                int mine = Sm - 1;
-                const unsigned gh = (hit >> (4 * g)) & 15u;
-                if (gh && q == __ffs(gh) - 1) {
-                    // the first state whose running sum reaches the pick: stored sum >=
-                    // pick - (the sums of the quarters before); none (rounding): the
-                    // quarter's last state
-                    const long long key = order_key(pick - excl);
-                    int a = qlo, b = qhi - 1;
-                    if (order_key(pg[b]) >= key) {
-                        while (a < b) {
-                            const int mid = (a + b) >> 1;
-                            if (order_key(pg[mid]) >= key) b = mid;
-                            else a = mid + 1;
-                        }
-                    }
-                    mine = b;
-                }
-#pragma unroll
-                for (int gg = 0; gg < G; gg++) {
-                    const unsigned hq = (hit >> (4 * gg)) & 15u;
-                    const int src = hq ? 4 * gg + __ffs(hq) - 1 : 4 * gg;
-                    const int r = __shfl_sync(0xffffffffu, mine, src);
-                    res[gg] = hq ? r : Sm - 1;
-                }
-            } else {
+            {
             // every column's chunk sums under the current row, as warp_sample forms them
             F l0[G], l1[G];
 #pragma unroll
@@ -905,6 +831,276 @@ __global__ void __launch_bounds__(32) k_traceback_split(BatchDev d, int maxS) {
     __syncwarp();
 }
 
+// ---------------------------------------------------------------------------------------
+// FP64 path: the reference's scan, tested for many columns at once by a CTA.
+//
+// Inside a tree the draw of column i depends on the later column only through its state k, and
+// mostly stays at k: the first state whose running sum reaches u sum(A) is k when the sum before
+// k is below the pick and the sum through k reaches it. Those sums do not depend on the other
+// columns' draws, so the CTA tests up to 64 columns at once: four lanes take a column (8,
+// 16 or 32 where the lot has fewer), lane q the states congruent to q, and butterfly steps
+// combine them. The first column that
+// leaves k, if any, is drawn by one warp exactly as a column on its own; the columns after it
+// are tested again under the new state's row.
+//
+// What bounds it: the FP64 pipe (64 cycles a warp's instruction). Four lanes a column with all
+// 32 lanes at work cost S / 32 FMAs a column plus a sixteenth of an instruction for each
+// butterfly step; one warp per instance (8 columns at a time, each summed in order and resolved
+// by a binary search) took 980 cycles a column at 99 states and 4,100 at 483, on one
+// sub-partition of the four.
+//
+// A tree's columns (as many as a buffer holds) and their uniforms arrive by bulk copies, the
+// next lot's while this one is drawn. A tree switch has few sources of nonzero weight (the drawn
+// state's gather list and the breakpoint's two states), taken in state order.
+constexpr int TW = 8;  // warps of k_traceback64
+
+__global__ void __launch_bounds__(32 * TW) k_traceback64(BatchDev d, int buf_bytes) {
+    extern __shared__ __align__(16) unsigned char dyn_b[];
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int LOT = 8 * TW, u_bytes = 8 * LOT + 32;  // columns of a lot at most
+    double *const trans = (double *)(dyn_b + 2 * buf_bytes + 2 * u_bytes);  // [maxS]
+    __shared__ double tmS[MAXT * MAXT];
+    __shared__ uint64_t bar[2];
+    __shared__ int first, drawn;
+    const int qi = cta_instance(d);
+    const InstDev I = d.inst[qi];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int *path = d.path + I.col0;
+    const double *u = d.uniforms + I.col0;
+    bool failed = false;
+
+    if (tid == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+
+    // lots: columns [lo, hi] of tree bi, from the last tree's last column down
+    struct Lot {
+        int bi, lo, hi, off, uoff;  // off, uoff: where column lo's values begin in the buffer
+    };
+    auto lot_at = [&](int bi, int hi) {
+        const BlockDev &B = d.blocks[I.block0 + bi];
+        const int Sm = imax(B.S, 1), cap = (buf_bytes - 16) / (8 * Sm);
+        return Lot{bi, imax(B.start, hi - imin(cap, LOT) + 1), hi, 0, 0};
+    };
+    auto fetch = [&](Lot &t, int b) {
+        const BlockDev &B = d.blocks[I.block0 + t.bi];
+        const int Sm = imax(B.S, 1), n = t.hi - t.lo + 1;
+        const Rounded<8> rt(d.fw64 + B.cell0 + (size_t)(t.lo - B.start) * Sm, (long long)n * Sm);
+        const Rounded<8> ru(u + t.lo, n);
+        t.off = rt.off;
+        t.uoff = ru.off;
+        if (tid == 0) {
+            mbar_expect_tx(&bar[b], rt.bytes + ru.bytes);
+            bulk_g2s(dyn_b + (size_t)b * buf_bytes, rt.a16, rt.bytes, &bar[b]);
+            bulk_g2s(dyn_b + 2 * buf_bytes + b * u_bytes, ru.a16, ru.bytes, &bar[b]);
+        }
+    };
+
+    Lot cur = lot_at(I.ntrees - 1, I.seqlen - 1);
+    fetch(cur, 0);
+    int state = 0, n = 0;        // state of the column after; lots done
+    bool pending = false;        // a lot in flight when the loop ends
+    bool fresh = true;           // the state's row is to be built
+    while (true) {
+        const int b = n & 1;
+        const BlockDev &B = d.blocks[I.block0 + cur.bi];
+        const int S = B.S, Sm = imax(S, 1), start = B.start, len = B.len;
+        // the next lot, into the other buffer (its last readers passed the barrier below)
+        Lot next = cur;
+        const bool more = cur.lo > 0;
+        if (more) {
+            next = cur.lo > start ? lot_at(cur.bi, cur.lo - 1) : lot_at(cur.bi - 1, cur.lo - 1);
+            fetch(next, b ^ 1);
+        }
+        const bool top = cur.hi == start + len - 1;  // the tree's last column is in this lot
+        if (top && S > 0) {
+            const double *tmg = d.tm + (size_t)(I.block0 + cur.bi) * MAXT * MAXT;
+            for (int e = tid; e < (I.T - 1) * MAXT; e += 32 * TW) tmS[e] = tmg[e];
+        }
+        const bool landed = mbar_wait(&bar[b], (unsigned)((n >> 1) & 1));
+        if (__syncthreads_or(!landed)) {
+            failed = true;
+            pending = more;
+            break;
+        }
+        const double *buf = (const double *)(dyn_b + (size_t)b * buf_bytes) + cur.off;
+        const double *ub = (const double *)(dyn_b + 2 * buf_bytes + b * u_bytes) + cur.uoff;
+        auto column = [&](int c) { return buf + (size_t)(c - cur.lo) * Sm; };
+        int c0 = cur.hi;
+
+        if (top) {
+            // the tree's last column, by warp 0
+            if (warp == 0) {
+                const double *c = column(c0);
+                const double uc = ub[c0 - cur.lo];
+                int x;
+                if (cur.bi == I.ntrees - 1) {
+                    // the last column of all (sample_thread.cpp:534-539); a given last state
+                    // (conditioned sampling) takes no draw
+                    const int given = d.last_state ? d.last_state[qi] : -1;
+                    x = given >= 0 ? given : warp_sample<double>(Sm, uc, [&](int j) { return c[j]; });
+                } else {
+                    // through the switch into the next tree (sample_hmm_posterior_step)
+                    const int nb = I.block0 + cur.bi + 1, k = state;
+                    const BlockDev &N = d.blocks[nb];
+                    const int2 src = d.srcs[nb];
+                    const int *gp = d.gptr + N.gptr0 + k;
+                    const int p0 = gp[0], ng = gp[1] - p0;
+                    const double *dp = d.determprob + N.prev_state0;
+                    const double rr = d.recombrow[N.state0 + k], cr = d.recoalrow[N.state0 + k];
+                    const bool hx = src.x != -1 && src.x != src.y, hy = src.y != -1;
+                    if (ng + 2 <= 32) {
+                        // lane e: the e-th source of the gather list, then the two states
+                        int j = -1;
+                        double wt = 0.0;
+                        if (lane < ng) {
+                            j = d.gidx[N.prev_state0 + p0 + lane];
+                            wt = c[j] * dp[j];
+                        } else if (lane == ng && hx) {
+                            j = src.x;
+                            wt = c[j] * rr;
+                        } else if (lane == ng + 1 && hy) {
+                            j = src.y;
+                            wt = c[j] * cr;
+                        }
+                        // their order by state, then the running sum in that order
+                        int pos = 0;
+                        for (int e = 0; e < ng + 2; e++) {
+                            const int je = __shfl_sync(FULL, j, e);
+                            pos += je >= 0 && je < j;
+                        }
+                        const int live = __popc(__ballot_sync(FULL, j >= 0));
+                        double run = 0.0, mine = 0.0;
+                        for (int r = 0; r < live; r++) {
+                            const unsigned at = __ballot_sync(FULL, j >= 0 && pos == r);
+                            run += __shfl_sync(FULL, wt, __ffs(at) - 1);
+                            if (j >= 0 && pos == r) mine = run;
+                        }
+                        const double pick = uc * run;
+                        // the first state of all reaches a pick of zero
+                        const unsigned hit = __ballot_sync(FULL, j >= 0 && mine >= pick);
+                        if (pick <= 0.0) {
+                            x = 0;
+                        } else if (hit) {
+                            int best = (hit >> lane & 1) ? j : 0x7fffffff;
+                            best = __reduce_min_sync(FULL, best);
+                            x = best;
+                        } else {
+                            x = imax(N.S1, 1) - 1;
+                        }
+                    } else {
+                        const int *determ = d.determ + N.prev_state0;
+                        x = warp_sample<double>(imax(N.S1, 1), uc, [&](int j) {
+                            const double g = j == src.y ? cr : j == src.x ? rr : determ[j] == k ? dp[j] : 0.0;
+                            return c[j] * g;
+                        });
+                    }
+                }
+                if (lane == 0) {
+                    path[c0] = x;
+                    drawn = x;
+                }
+            }
+            __syncthreads();
+            state = drawn;
+            c0--;
+        }
+        if (S == 0) {
+            // fully specified tree: its single state carries over
+            for (int c = cur.lo + tid; c <= c0; c += 32 * TW) path[c] = 0;
+            state = 0;
+            c0 = cur.lo - 1;
+        }
+        fresh |= top;
+        while (c0 >= cur.lo) {
+            if (fresh) {
+                // trans[j] = TransMatrix::get(j, k) (trans.h:64-83)
+                const StateInfo sk = d.sinfo[B.state0 + state];
+                const long long row = B.t2_0 + d.t2off[B.state0 + state];
+                for (int j = tid; j < S; j += 32 * TW) {
+                    const StateInfo sj = d.sinfo[B.state0 + j];
+                    trans[j] = sj.node == sk.node ? d.gts[row + (long long)(j - sk.j1) * sk.m]
+                                                  : tmS[sj.time * MAXT + sk.time];
+                }
+                fresh = false;
+            }
+            const int ncols = imin(LOT, c0 - cur.lo + 1), k = state;
+            // lanes a column: 4, 8, 16 or 32, so that few columns still keep every warp busy
+            const int lb = ncols > LOT / 2 ? 2 : ncols > LOT / 4 ? 3 : ncols > LOT / 8 ? 4 : 5;
+            if (tid == 0) first = ncols;
+            __syncthreads();  // trans, first
+            const int g = tid >> lb, lanes = 1 << lb, q = tid & (lanes - 1);
+            if ((tid & ~31) >> lb < ncols) {
+                const int mc = c0 - imin(g, ncols - 1);
+                const double *cp = column(mc);
+                double before = 0.0, after = 0.0;
+                int j = q;
+#pragma unroll 4
+                for (; j < k; j += lanes) before = fma(cp[j], trans[j], before);
+                j += j == k ? lanes : 0;
+#pragma unroll 4
+                for (; j < S; j += lanes) after = fma(cp[j], trans[j], after);
+                for (int o = 1; o < lanes; o <<= 1) {
+                    before += __shfl_xor_sync(FULL, before, o);
+                    after += __shfl_xor_sync(FULL, after, o);
+                }
+                const double through = fma(cp[k], trans[k], before);
+                const double pick = ub[mc - cur.lo] * (through + after);
+                const bool leave = g < ncols && !((k == 0 || before < pick) && pick <= through);
+                const unsigned l = __ballot_sync(FULL, leave);
+                if (l && lane == 0) atomicMin(&first, (tid + __ffs(l) - 1) >> lb);
+            }
+            __syncthreads();
+            const int r = first;
+            if (tid < r) path[c0 - tid] = k;
+            if (r < ncols) {
+                // the column that leaves, drawn as one on its own
+                if (warp == 0) {
+                    const double *cp = column(c0 - r);
+                    const int x = warp_sample<double>(S, ub[c0 - r - cur.lo], [&](int j) { return cp[j] * trans[j]; });
+                    if (lane == 0) {
+                        path[c0 - r] = x;
+                        drawn = x;
+                    }
+                }
+                __syncthreads();
+                fresh = drawn != state;
+                state = drawn;
+                c0 -= r + 1;
+            } else {
+                c0 -= r;
+            }
+            __syncthreads();  // first, drawn and trans are read
+        }
+        if (!more) break;
+        __syncthreads();  // this lot's buffer is read
+        cur = next;
+        n++;
+    }
+    if (failed && tid == 0) {
+        report_error(d.err, ERR_WAIT_LIMIT, qi, -1, -1);
+        // the copies in flight, before the memory is released
+        mbar_wait(&bar[n & 1], (unsigned)((n >> 1) & 1));
+        if (pending) mbar_wait(&bar[(n & 1) ^ 1], (unsigned)(((n + 1) >> 1) & 1));
+    }
+    __syncthreads();
+}
+
+void launch64(const BatchDev &d, cudaStream_t s) {
+    // a lot of the largest tree in a buffer, where two buffers leave room for a second CTA on the
+    // SM; else as many columns as two buffers hold, at least one
+    const size_t col = 8 * (size_t)imax(d.maxS, 1);
+    const size_t n = 8 * TW * col <= 44 * 1024 ? 8 * TW : imax(imin((int)(100 * 1024 / col), 8 * TW), 1);
+    const size_t buf = (n * col + 16 + 15) & ~(size_t)15;
+    const size_t smem = 2 * buf + 2 * (8 * 8 * TW + 32) + col;
+    if (!raise_dynamic_smem(k_traceback64, smem)) return;  // the launch reports it
+    k_traceback64<<<d.ninst, 32 * TW, smem, s>>>(d, (int)buf);
+    note_launch();
+}
+
 template <int NCH>
 bool launch_split(const BatchDev &d, cudaStream_t s, size_t budget) {
     const int maxS = imax(d.maxS, 1);
@@ -918,18 +1114,16 @@ bool launch_split(const BatchDev &d, cudaStream_t s, size_t budget) {
     return true;
 }
 
-template <typename F, int G, int DEPTH, bool QL = false>
+template <typename F, int G, int DEPTH>
 bool launch_cfg(const BatchDev &d, cudaStream_t s, size_t budget) {
     const int maxS = imax(d.maxS, 1);
-    if (QL && maxS > QL_MAXS) return false;
     const int slot_elems = (int)(((size_t)maxS * sizeof(F) + 32 + 15) / 16 * 16 / sizeof(F));
-    size_t smem = (size_t)DEPTH * slot_elems * sizeof(F) + DEPTH * sizeof(double) +
+    const size_t smem = (size_t)DEPTH * slot_elems * sizeof(F) + DEPTH * sizeof(double) +
                   (size_t)(maxS + 1) * sizeof(F) + 2 * (size_t)maxS * sizeof(int) + 16;
-    if (QL) smem = (smem + 15) / 16 * 16 + (size_t)G * (maxS + 1) * sizeof(F);
     if (smem > budget) return false;
     // opt in; static shared memory counts against 48 KB too
-    if (!raise_dynamic_smem(k_traceback<F, G, DEPTH, QL>, smem)) return true;  // the launch reports it
-    k_traceback<F, G, DEPTH, QL><<<d.ninst, 32, smem, s>>>(d, maxS, slot_elems);
+    if (!raise_dynamic_smem(k_traceback<F, G, DEPTH>, smem)) return true;  // the launch reports it
+    k_traceback<F, G, DEPTH><<<d.ninst, 32, smem, s>>>(d, maxS, slot_elems);
     note_launch();
     return true;
 }
@@ -946,9 +1140,6 @@ void launch(const BatchDev &d, cudaStream_t s) {
             if (launch_split<3>(d, s, 224 * 1024)) return;
         }
     }
-    if constexpr (sizeof(F) == 8) {
-        if (launch_cfg<F, 8, 24, true>(d, s, two)) return;
-    }
     if (launch_cfg<F, 8, 24>(d, s, two)) return;
     if (launch_cfg<F, 4, 12>(d, s, two)) return;
     if (launch_cfg<F, 4, 12>(d, s, one)) return;
@@ -960,7 +1151,7 @@ void launch(const BatchDev &d, cudaStream_t s) {
 
 void launch_traceback(const BatchDev &d, bool fp32, cudaStream_t s) {
     if (fp32) launch<float>(d, s);
-    else launch<double>(d, s);
+    else launch64(d, s);
 }
 
 }  // namespace awg
