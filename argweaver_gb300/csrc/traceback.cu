@@ -1,21 +1,15 @@
 // K4: stochastic traceback (stochastic_traceback, sample_thread.cpp:522-569;
 // sample_hmm_posterior :470-503; sample_hmm_posterior_step :506-519; sample,
 // common.h:272-290). Column i draws path[i] from A[j] = fw[i][j] * P(j -> path[i+1]) with the
-// uniform u[i]: the first j whose running sum reaches u[i] * sum(A). Three kernels, one block
+// uniform u[i]: the first j whose running sum reaches u[i] * sum(A). Two kernels, one block
 // per instance:
-//   k_traceback64     FP64: the reference's scan, a CTA testing many columns at once
+//   k_traceback_lots  the reference's scan, a CTA drawing or testing many columns at once: FP64,
+//                     and FP32 where the decomposed draw's tables do not fit
 //   k_traceback_split FP32: the draw decomposed by the structure of the transition
-//   k_traceback       FP32 where the decomposed draw's tables do not fit: the scan, one warp
 //
 // The scan by one warp splits the states into 32 contiguous chunks (lane t sums chunk t with
 // two accumulators, even and odd states); chunk sums are scanned across lanes and the chunk
-// that holds the pick is rescanned by all lanes at once. The transition row P(. -> k) changes
-// only when the sampled state does, which is rare inside a local tree, so the warp samples G
-// columns at once under the current row, every column's sums computed exactly as if it were
-// alone, and keeps the draws up to and including the first one that leaves state k; the rest
-// are redone under the new row. Columns stream into a shared-memory ring DEPTH columns ahead
-// of the sampler with 16-byte cp.async (a column's start is rounded down to 16 bytes and the
-// slot keeps the offset), each column's uniform beside it.
+// that holds the pick is rescanned.
 
 #include <cuda_runtime.h>
 
@@ -27,33 +21,21 @@ namespace awg {
 namespace {
 
 template <typename F> struct TTab;
-template <> struct TTab<float> {
-    static constexpr bool split = true;  // t2d32 excludes the diagonal's stay term
-    const float *rstay;
-    const float *tm, *t2d, *dprob, *rrow, *crow, *fw;
+template <> struct TTab<double> {
+    const double *tm, *rows, *dprob, *rrow, *crow, *fw;
     __device__ explicit TTab(const BatchDev &d)
-        : rstay(d.rstay32), tm(d.tm32), t2d(d.t2d32), dprob(d.determprob32),
-          rrow(d.recombrow32), crow(d.recoalrow32), fw(d.fw32) {}
-    __device__ float same(long long idx, float tmab) const { return t2d[idx] + tmab; }
+        : tm(d.tm), rows(d.gts), dprob(d.determprob), rrow(d.recombrow), crow(d.recoalrow), fw(d.fw64) {}
+    // same-node entry: get_time(a, b, c, minage, true)
+    __device__ static double same(double v, double) { return v; }
 };
-
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-
-// Elements between a column's 16-byte-aligned start and the column itself.
-template <typename F>
-__device__ __forceinline__ int col_offset(const F *p) {
-    return (int)(((uintptr_t)p & 15) / sizeof(F));
-}
+template <> struct TTab<float> {
+    const float *rstay;  // rows exclude the diagonal's stay term
+    const float *tm, *rows, *dprob, *rrow, *crow, *fw;
+    __device__ explicit TTab(const BatchDev &d)
+        : rstay(d.rstay32), tm(d.tm32), rows(d.t2d32), dprob(d.determprob32),
+          rrow(d.recombrow32), crow(d.recoalrow32), fw(d.fw32) {}
+    __device__ static float same(float v, float tmab) { return v + tmab; }
+};
 
 // Inclusive lane scan.
 template <typename F>
@@ -112,279 +94,124 @@ __device__ int warp_sample(int n, double u, W w) {
     return finish_sample<F>(n, chunk, incl, (F)u * total, lo, hi, lane, w);
 }
 
-template <typename F, int G, int DEPTH>
-__global__ void k_traceback(BatchDev d, int maxS, int slot_elems) {
-    extern __shared__ double dyn_d[];
-    F *ring = (F *)dyn_d;                                   // [DEPTH][slot_elems], 16-B slots
-    double *uring = (double *)(ring + (size_t)DEPTH * slot_elems);  // [DEPTH] uniforms
-    F *trans = (F *)(uring + DEPTH);                        // [maxS]
-    int *stime = (int *)(trans + maxS + (maxS & 1));        // [maxS] state times of the tree
-    int *snode = stime + maxS;                              // [maxS]
-    __shared__ F tmS[MAXT * MAXT];
-    const TTab<F> tab(d);
-    const int qi = cta_instance(d);
-    const InstDev I = d.inst[qi];
-    const int lane = threadIdx.x;
-    int *path = d.path + I.col0;
-    const double *u = d.uniforms + I.col0;
-    const int L = I.seqlen;
-
-    // prefetch cursor: next column to copy (descending), its tree's fields in registers
-    int pcol = L - 1, pblk = I.ntrees - 1;
-    int pS = imax(d.blocks[I.block0 + pblk].S, 1), pstart = d.blocks[I.block0 + pblk].start;
-    long long pcell = d.blocks[I.block0 + pblk].cell0;
-    auto issue = [&]() {
-        if (pcol >= 0) {
-            const F *src = tab.fw + pcell + (size_t)(pcol - pstart) * pS;
-            const char *a16 = (const char *)((uintptr_t)src & ~(uintptr_t)15);
-            const int nbytes = (int)((const char *)(src + pS) - a16);
-            char *dst = (char *)(ring + (size_t)(pcol % DEPTH) * slot_elems);
-            for (int q = lane; q * 16 < nbytes; q += 32) cp_async16(dst + q * 16, a16 + q * 16);
-            if (lane == 0) cp_async8(uring + pcol % DEPTH, u + pcol);
-            pcol--;
-            if (pblk > 0 && pcol < pstart) {
-                pblk--;
-                pS = imax(d.blocks[I.block0 + pblk].S, 1);
-                pstart = d.blocks[I.block0 + pblk].start;
-                pcell = d.blocks[I.block0 + pblk].cell0;
-            }
-        }
-        cp_commit();  // one group per column, empty ones included
-    };
-    // Invariant: before a group starting at column c0 is sampled, columns c0 .. c0-DEPTH+1
-    // have been issued, one commit group each, oldest first.
-    for (int q = 0; q < DEPTH; q++) issue();
-
-    // a column's values in its ring slot
-    auto column = [&](const BlockDev &B, int col) -> const F * {
-        const int Sm = imax(B.S, 1);
-        const F *g = tab.fw + B.cell0 + (size_t)(col - B.start) * Sm;
-        return ring + (size_t)(col % DEPTH) * slot_elems + col_offset(g);
-    };
-
-    int col = L - 1;
-    int state;  // path[col + 1] of the column being sampled
-    // last column (sample_thread.cpp:534-539)
-    {
-        const BlockDev &Bl = d.blocks[I.block0 + I.ntrees - 1];
-        cp_wait<DEPTH - 1>();
-        __syncwarp();
-        const F *c = column(Bl, col);
-        // a given last state (conditioned sampling) takes no draw
-        const int given = d.last_state ? d.last_state[qi] : -1;
-        const int x = given >= 0 ? given
-                                 : warp_sample<F>(imax(Bl.S, 1), uring[col % DEPTH], [&](int j) { return c[j]; });
-        if (lane == 0) path[col] = x;
-        state = x;
-        __syncwarp();
-        issue();
-    }
-    for (int bi = I.ntrees - 1; bi >= 0; bi--) {
-        const int blk = I.block0 + bi;
-        const BlockDev B = d.blocks[blk];
-        const int S = B.S, Sm = imax(S, 1);
-        const int chunk = (Sm + 31) >> 5;
-        const int lo = imin(lane * chunk, Sm), hi = imin(lo + chunk, Sm);
-        // stage the tree's state times/nodes and tmatrix
-        for (int j = lane; j < S; j += 32) {
-            const StateInfo si = d.sinfo[B.state0 + j];
-            stime[j] = si.time;
-            snode[j] = si.node;
-        }
-        const F *tmg = tab.tm + (size_t)blk * MAXT * MAXT;
-        for (int e = lane; e < (I.T - 1) * MAXT; e += 32) tmS[e] = tmg[e];
-        __syncwarp();
-        // trans[j] = TransMatrix::get(j, k) (trans.h:64-83)
-        auto build_row = [&](int k) {
-            if (S == 0) {
-                if (lane == 0) trans[0] = F(1);
-            } else {
-                const StateInfo sk = d.sinfo[B.state0 + k];
-                const long long row = B.t2_0 + d.t2off[B.state0 + k];
-                const F stay = TTab<F>::split ? F(1) - tab.rstay[(size_t)blk * MAXT + sk.time] : F(0);
-                for (int j = lane; j < S; j += 32) {
-                    const F tmab = tmS[stime[j] * MAXT + sk.time];
-                    F t = tmab;
-                    if (snode[j] == sk.node) {
-                        t = tab.same(row + (long long)(j - sk.j1) * sk.m, tmab);
-                        if (j == k) t += stay;
-                    }
-                    trans[j] = t;
-                }
-            }
-            __syncwarp();
-        };
-        build_row(state);
-
-        // within the tree: columns B.start + B.len - 2 down to B.start, G at a time
-        int c0 = B.start + B.len - 2;
-        while (c0 >= B.start) {
-            const int ng = imin(G, c0 - B.start + 1);
-            cp_wait<DEPTH - G>();
-            __syncwarp();
-            const F *cg[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) cg[g] = column(B, c0 - imin(g, ng - 1));
-            int res[G];
-            {
-            // every column's chunk sums under the current row, as warp_sample forms them
-            F l0[G], l1[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) l0[g] = l1[g] = F(0);
-            int j = lo;
-            for (; j + 1 < hi; j += 2) {
-                const F t0 = trans[j], t1 = trans[j + 1];
-#pragma unroll
-                for (int g = 0; g < G; g++) {
-                    l0[g] = fma(cg[g][j], t0, l0[g]);
-                    l1[g] = fma(cg[g][j + 1], t1, l1[g]);
-                }
-            }
-            if (j < hi) {
-                const F t0 = trans[j];
-#pragma unroll
-                for (int g = 0; g < G; g++) l0[g] = fma(cg[g][j], t0, l0[g]);
-            }
-            F incl[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) incl[g] = l0[g] + l1[g];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-                for (int g = 0; g < G; g++) {
-                    const F v = __shfl_up_sync(0xffffffffu, incl[g], o);
-                    if (lane >= o) incl[g] += v;
-                }
-            }
-            // every column's draw, all G interleaved (finish_sample's steps, column-wise)
-            F pick[G], carry[G];
-            int slo[G], shi[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) {
-                F excl = __shfl_up_sync(0xffffffffu, incl[g], 1);
-                if (lane == 0) excl = 0;
-                const F total = __shfl_sync(0xffffffffu, incl[g], 31);
-                pick[g] = (F)uring[(c0 - imin(g, ng - 1)) % DEPTH] * total;
-                const unsigned hit = __ballot_sync(0xffffffffu, incl[g] >= pick[g] && hi > lo);
-                const int src = hit ? __ffs(hit) - 1 : 0;
-                slo[g] = imin(src * chunk, Sm);
-                shi[g] = hit ? imin(slo[g] + chunk, Sm) : slo[g];  // empty: no rescan
-                carry[g] = __shfl_sync(0xffffffffu, excl, src);
-                res[g] = hit ? shi[g] - 1 : Sm - 1;
-            }
-            unsigned open = 0;  // columns whose pick is not found yet
-#pragma unroll
-            for (int g = 0; g < G; g++)
-                if (shi[g] > slo[g]) open |= 1u << g;
-            if (chunk <= 16) {
-                // short chunks: lane g rescans column g's chosen chunk in order, one product
-                // and one add per state, the G columns side by side (a 32-lane scan per column
-                // costs five warp-wide adds however few states the chunk holds: on the FP64
-                // path each holds the sub-partition's FP64 pipe for about 64 cycles)
-                int mine = 0;
-                if (lane < G) {
-                    F mpick = 0, run = 0;
-                    int mslo = 0, mshi = 0;
-                    const F *mc = cg[0];
-#pragma unroll
-                    for (int g = 0; g < G; g++)
-                        if (lane == g) {
-                            mpick = pick[g];
-                            run = carry[g];
-                            mslo = slo[g];
-                            mshi = (open >> g) & 1 ? shi[g] : slo[g];
-                            mine = res[g];
-                            mc = cg[g];
-                        }
-                    for (int jj = mslo; jj < mshi; jj++) {
-                        run += mc[jj] * trans[jj];
-                        if (run >= mpick) {
-                            mine = jj;
-                            break;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int g = 0; g < G; g++) res[g] = __shfl_sync(0xffffffffu, mine, g);
-                open = 0;
-            }
-            for (int b = 0; open; b += 32) {
-                F x[G];
-#pragma unroll
-                for (int g = 0; g < G; g++) {
-                    const int jj = slo[g] + b + lane;
-                    x[g] = ((open >> g) & 1) && jj < shi[g] ? cg[g][jj] * trans[jj] : F(0);
-                }
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
+// G columns under one row, each as warp_sample draws it on its own (fused products), side by side:
+// values cg[g][j], weights trans[j], j < n, uniforms ug.
+template <typename F, int G>
+__device__ void warp_sample_group(int n, const F *const (&cg)[G], const F *trans, const double (&ug)[G], int (&res)[G]) {
+    const int lane = threadIdx.x & 31;
+    const int chunk = (n + 31) >> 5;
+    const int lo = imin(lane * chunk, n), hi = imin(lo + chunk, n);
+                // every column's chunk sums under the current row, as warp_sample forms them
+                F l0[G], l1[G];
+    #pragma unroll
+                for (int g = 0; g < G; g++) l0[g] = l1[g] = F(0);
+                int j = lo;
+                for (; j + 1 < hi; j += 2) {
+                    const F t0 = trans[j], t1 = trans[j + 1];
+    #pragma unroll
                     for (int g = 0; g < G; g++) {
-                        const F v = __shfl_up_sync(0xffffffffu, x[g], o);
-                        if (lane >= o) x[g] += v;
+                        l0[g] = fma(cg[g][j], t0, l0[g]);
+                        l1[g] = fma(cg[g][j + 1], t1, l1[g]);
                     }
                 }
-#pragma unroll
+                if (j < hi) {
+                    const F t0 = trans[j];
+    #pragma unroll
+                    for (int g = 0; g < G; g++) l0[g] = fma(cg[g][j], t0, l0[g]);
+                }
+                F incl[G];
+    #pragma unroll
+                for (int g = 0; g < G; g++) incl[g] = l0[g] + l1[g];
+    #pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+    #pragma unroll
+                    for (int g = 0; g < G; g++) {
+                        const F v = __shfl_up_sync(0xffffffffu, incl[g], o);
+                        if (lane >= o) incl[g] += v;
+                    }
+                }
+                // every column's draw, all G interleaved (finish_sample's steps, column-wise)
+                F pick[G], carry[G];
+                int slo[G], shi[G];
+    #pragma unroll
                 for (int g = 0; g < G; g++) {
-                    if (!((open >> g) & 1)) continue;
-                    const int jj = slo[g] + b + lane;
-                    const unsigned got =
-                        __ballot_sync(0xffffffffu, jj < shi[g] && carry[g] + x[g] >= pick[g]);
-                    if (got) {
-                        res[g] = slo[g] + b + __ffs(got) - 1;
-                        open &= ~(1u << g);
-                    } else {
-                        carry[g] += __shfl_sync(0xffffffffu, x[g], 31);
-                        if (slo[g] + b + 32 >= shi[g]) open &= ~(1u << g);
+                    F excl = __shfl_up_sync(0xffffffffu, incl[g], 1);
+                    if (lane == 0) excl = 0;
+                    const F total = __shfl_sync(0xffffffffu, incl[g], 31);
+                    pick[g] = (F)ug[g] * total;
+                    const unsigned hit = __ballot_sync(0xffffffffu, incl[g] >= pick[g] && hi > lo);
+                    const int src = hit ? __ffs(hit) - 1 : 0;
+                    slo[g] = imin(src * chunk, n);
+                    shi[g] = hit ? imin(slo[g] + chunk, n) : slo[g];  // empty: no rescan
+                    carry[g] = __shfl_sync(0xffffffffu, excl, src);
+                    res[g] = hit ? shi[g] - 1 : n - 1;
+                }
+                unsigned open = 0;  // columns whose pick is not found yet
+    #pragma unroll
+                for (int g = 0; g < G; g++)
+                    if (shi[g] > slo[g]) open |= 1u << g;
+                if (chunk <= 16) {
+                    // short chunks: lane g rescans column g's chosen chunk in order, one product
+                    // and one add per state, the G columns side by side (a 32-lane scan per column
+                    // costs five warp-wide adds however few states the chunk holds: on the FP64
+                    // path each holds the sub-partition's FP64 pipe for about 64 cycles)
+                    int mine = 0;
+                    if (lane < G) {
+                        F mpick = 0, run = 0;
+                        int mslo = 0, mshi = 0;
+                        const F *mc = cg[0];
+    #pragma unroll
+                        for (int g = 0; g < G; g++)
+                            if (lane == g) {
+                                mpick = pick[g];
+                                run = carry[g];
+                                mslo = slo[g];
+                                mshi = (open >> g) & 1 ? shi[g] : slo[g];
+                                mine = res[g];
+                                mc = cg[g];
+                            }
+                        for (int jj = mslo; jj < mshi; jj++) {
+                            run += mc[jj] * trans[jj];
+                            if (run >= mpick) {
+                                mine = jj;
+                                break;
+                            }
+                        }
+                    }
+    #pragma unroll
+                    for (int g = 0; g < G; g++) res[g] = __shfl_sync(0xffffffffu, mine, g);
+                    open = 0;
+                }
+                for (int b = 0; open; b += 32) {
+                    F x[G];
+    #pragma unroll
+                    for (int g = 0; g < G; g++) {
+                        const int jj = slo[g] + b + lane;
+                        x[g] = ((open >> g) & 1) && jj < shi[g] ? cg[g][jj] * trans[jj] : F(0);
+                    }
+    #pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+    #pragma unroll
+                        for (int g = 0; g < G; g++) {
+                            const F v = __shfl_up_sync(0xffffffffu, x[g], o);
+                            if (lane >= o) x[g] += v;
+                        }
+                    }
+    #pragma unroll
+                    for (int g = 0; g < G; g++) {
+                        if (!((open >> g) & 1)) continue;
+                        const int jj = slo[g] + b + lane;
+                        const unsigned got =
+                            __ballot_sync(0xffffffffu, jj < shi[g] && carry[g] + x[g] >= pick[g]);
+                        if (got) {
+                            res[g] = slo[g] + b + __ffs(got) - 1;
+                            open &= ~(1u << g);
+                        } else {
+                            carry[g] += __shfl_sync(0xffffffffu, x[g], 31);
+                            if (slo[g] + b + 32 >= shi[g]) open &= ~(1u << g);
+                        }
                     }
                 }
-            }
-            }
-            // keep the draws in column order up to the first that leaves the current state
-            int r = 0, x = state;
-#pragma unroll
-            for (int g = 0; g < G; g++) {
-                if (g < ng && x == state) {
-                    x = res[g];
-                    if (lane == 0) path[c0 - g] = x;
-                    r = g + 1;
-                }
-            }
-            __syncwarp();
-            for (int q = 0; q < r; q++) issue();
-            c0 -= r;
-            if (x != state) {
-                state = x;
-                build_row(state);
-            }
-        }
-        if (bi > 0) {
-            // switch into this tree (sample_hmm_posterior_step)
-            col = B.start - 1;
-            const BlockDev &P = d.blocks[blk - 1];
-            const int k = state;
-            const int n1 = imax(B.S1, 1);
-            const int2 src = d.srcs[blk];
-            const int *determ = d.determ + B.prev_state0;
-            const F *dp = tab.dprob + B.prev_state0;
-            const F rr = tab.rrow[B.state0 + k], cr = tab.crow[B.state0 + k];
-            cp_wait<DEPTH - 1>();
-            __syncwarp();
-            const F *c = column(P, col);
-            auto w = [&](int j) -> F {
-                F g;
-                if (j == src.y) g = cr;
-                else if (j == src.x) g = rr;
-                else g = (determ[j] == k) ? dp[j] : F(0);
-                return c[j] * g;
-            };
-            const int x = warp_sample<F>(n1, uring[col % DEPTH], w);
-            if (lane == 0) path[col] = x;
-            state = x;
-            __syncwarp();
-            issue();
-        }
-    }
-    cp_wait<0>();
 }
 
 // ---------------------------------------------------------------------------------------
@@ -659,7 +486,7 @@ __global__ void __launch_bounds__(32) k_traceback_split(BatchDev d, int maxS) {
                 const long long row = B.t2_0 + t2off[k];
                 const float stay = 1.0f - rst[sk.time];
                 __syncwarp();
-                t2row[lane] = lane < km ? tab.t2d[row + (long long)lane * km] + (lane == ys ? stay : 0.0f) : 0.0f;
+                t2row[lane] = lane < km ? tab.rows[row + (long long)lane * km] + (lane == ys ? stay : 0.0f) : 0.0f;
                 tmcol[lane] = lane < NB ? tmS[lane * MAXT + sk.time] : 0.0f;
                 __syncwarp();
 #pragma unroll
@@ -832,7 +659,7 @@ __global__ void __launch_bounds__(32) k_traceback_split(BatchDev d, int maxS) {
 }
 
 // ---------------------------------------------------------------------------------------
-// FP64 path: the reference's scan, tested for many columns at once by a CTA.
+// The reference's scan, for many columns at once by a CTA.
 //
 // Inside a tree the draw of column i depends on the later column only through its state k, and
 // mostly stays at k: the first state whose running sum reaches u sum(A) is k when the sum before
@@ -842,8 +669,11 @@ __global__ void __launch_bounds__(32) k_traceback_split(BatchDev d, int maxS) {
 // combine them. The first column that
 // leaves k, if any, is drawn by one warp exactly as a column on its own; the columns after it
 // are tested again under the new state's row.
+// In FP32 every column of a round is drawn as one on its own, up to four by a warp (the same sums
+// in the same order whatever the round), and the draws are kept up to the first that leaves k:
+// 0.49 us a column at 1572 states, where one warp per instance took 2.09.
 //
-// What bounds it: the FP64 pipe (64 cycles a warp's instruction). Four lanes a column with all
+// What bounds it in FP64: the FP64 pipe (64 cycles a warp's instruction). Four lanes a column with all
 // 32 lanes at work cost S / 32 FMAs a column plus a sixteenth of an instruction for each
 // butterfly step; one warp per instance (8 columns at a time, each summed in order and resolved
 // by a binary search) took 980 cycles a column at 99 states and 4,100 at 483, on one
@@ -852,16 +682,25 @@ __global__ void __launch_bounds__(32) k_traceback_split(BatchDev d, int maxS) {
 // A tree's columns (as many as a buffer holds) and their uniforms arrive by bulk copies, the
 // next lot's while this one is drawn. A tree switch has few sources of nonzero weight (the drawn
 // state's gather list and the breakpoint's two states), taken in state order.
-constexpr int TW = 8;  // warps of k_traceback64
+constexpr int TW = 8;  // warps of k_traceback_lots
+template <int N>
+struct Cols {
+    static constexpr int value = N;
+};
+template <typename F>
+constexpr int LOT = sizeof(F) == 8 ? 8 * TW : 4 * TW;  // columns of a lot and a round at most
 
-__global__ void __launch_bounds__(32 * TW) k_traceback64(BatchDev d, int buf_bytes) {
+template <typename F>
+__global__ void __launch_bounds__(32 * TW) k_traceback_lots(BatchDev d, int buf_bytes) {
+    constexpr bool wide = sizeof(F) == 8;
     extern __shared__ __align__(16) unsigned char dyn_b[];
     constexpr unsigned FULL = 0xffffffffu;
-    constexpr int LOT = 8 * TW, u_bytes = 8 * LOT + 32;  // columns of a lot at most
-    double *const trans = (double *)(dyn_b + 2 * buf_bytes + 2 * u_bytes);  // [maxS]
-    __shared__ double tmS[MAXT * MAXT];
+    constexpr int u_bytes = 8 * LOT<F> + 32, E = sizeof(F);
+    const TTab<F> tab(d);
+    F *const trans = (F *)(dyn_b + 2 * buf_bytes + 2 * u_bytes);  // [maxS]
+    __shared__ F tmS[MAXT * MAXT];
     __shared__ uint64_t bar[2];
-    __shared__ int first, drawn;
+    __shared__ int first, drawn, draws[LOT<F>];
     const int qi = cta_instance(d);
     const InstDev I = d.inst[qi];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -882,13 +721,13 @@ __global__ void __launch_bounds__(32 * TW) k_traceback64(BatchDev d, int buf_byt
     };
     auto lot_at = [&](int bi, int hi) {
         const BlockDev &B = d.blocks[I.block0 + bi];
-        const int Sm = imax(B.S, 1), cap = (buf_bytes - 16) / (8 * Sm);
-        return Lot{bi, imax(B.start, hi - imin(cap, LOT) + 1), hi, 0, 0};
+        const int Sm = imax(B.S, 1), cap = (buf_bytes - 16) / (E * Sm);
+        return Lot{bi, imax(B.start, hi - imin(cap, LOT<F>) + 1), hi, 0, 0};
     };
     auto fetch = [&](Lot &t, int b) {
         const BlockDev &B = d.blocks[I.block0 + t.bi];
         const int Sm = imax(B.S, 1), n = t.hi - t.lo + 1;
-        const Rounded<8> rt(d.fw64 + B.cell0 + (size_t)(t.lo - B.start) * Sm, (long long)n * Sm);
+        const Rounded<E> rt(tab.fw + B.cell0 + (size_t)(t.lo - B.start) * Sm, (long long)n * Sm);
         const Rounded<8> ru(u + t.lo, n);
         t.off = rt.off;
         t.uoff = ru.off;
@@ -917,7 +756,7 @@ __global__ void __launch_bounds__(32 * TW) k_traceback64(BatchDev d, int buf_byt
         }
         const bool top = cur.hi == start + len - 1;  // the tree's last column is in this lot
         if (top && S > 0) {
-            const double *tmg = d.tm + (size_t)(I.block0 + cur.bi) * MAXT * MAXT;
+            const F *tmg = tab.tm + (size_t)(I.block0 + cur.bi) * MAXT * MAXT;
             for (int e = tid; e < (I.T - 1) * MAXT; e += 32 * TW) tmS[e] = tmg[e];
         }
         const bool landed = mbar_wait(&bar[b], (unsigned)((n >> 1) & 1));
@@ -926,22 +765,37 @@ __global__ void __launch_bounds__(32 * TW) k_traceback64(BatchDev d, int buf_byt
             pending = more;
             break;
         }
-        const double *buf = (const double *)(dyn_b + (size_t)b * buf_bytes) + cur.off;
+        const F *buf = (const F *)(dyn_b + (size_t)b * buf_bytes) + cur.off;
         const double *ub = (const double *)(dyn_b + 2 * buf_bytes + b * u_bytes) + cur.uoff;
         auto column = [&](int c) { return buf + (size_t)(c - cur.lo) * Sm; };
         int c0 = cur.hi;
 
         if (top) {
-            // the tree's last column, by warp 0
+            // the tree's last column, by warp 0; FP32: its weights through the switch by all
+            if (!wide && cur.bi < I.ntrees - 1) {
+                const int nb = I.block0 + cur.bi + 1;
+                const BlockDev &N = d.blocks[nb];
+                const int2 src = d.srcs[nb];
+                const int *determ = d.determ + N.prev_state0;
+                const F *c = column(c0), *dp = tab.dprob + N.prev_state0;
+                const F rr = tab.rrow[N.state0 + state], cr = tab.crow[N.state0 + state];
+                for (int j = tid; j < imax(N.S1, 1); j += 32 * TW) {
+                    const F g = j == src.y ? cr : j == src.x ? rr : determ[j] == state ? dp[j] : F(0);
+                    trans[j] = c[j] * g;
+                }
+                __syncthreads();
+            }
             if (warp == 0) {
-                const double *c = column(c0);
+                const F *c = column(c0);
                 const double uc = ub[c0 - cur.lo];
                 int x;
                 if (cur.bi == I.ntrees - 1) {
                     // the last column of all (sample_thread.cpp:534-539); a given last state
                     // (conditioned sampling) takes no draw
                     const int given = d.last_state ? d.last_state[qi] : -1;
-                    x = given >= 0 ? given : warp_sample<double>(Sm, uc, [&](int j) { return c[j]; });
+                    x = given >= 0 ? given : warp_sample<F>(Sm, uc, [&](int j) { return c[j]; });
+                } else if (!wide) {
+                    x = warp_sample<F>(Sm, uc, [&](int j) { return trans[j]; });
                 } else {
                     // through the switch into the next tree (sample_hmm_posterior_step)
                     const int nb = I.block0 + cur.bi + 1, k = state;
@@ -949,13 +803,13 @@ __global__ void __launch_bounds__(32 * TW) k_traceback64(BatchDev d, int buf_byt
                     const int2 src = d.srcs[nb];
                     const int *gp = d.gptr + N.gptr0 + k;
                     const int p0 = gp[0], ng = gp[1] - p0;
-                    const double *dp = d.determprob + N.prev_state0;
-                    const double rr = d.recombrow[N.state0 + k], cr = d.recoalrow[N.state0 + k];
+                    const F *dp = tab.dprob + N.prev_state0;
+                    const F rr = tab.rrow[N.state0 + k], cr = tab.crow[N.state0 + k];
                     const bool hx = src.x != -1 && src.x != src.y, hy = src.y != -1;
                     if (ng + 2 <= 32) {
                         // lane e: the e-th source of the gather list, then the two states
                         int j = -1;
-                        double wt = 0.0;
+                        F wt = F(0);
                         if (lane < ng) {
                             j = d.gidx[N.prev_state0 + p0 + lane];
                             wt = c[j] * dp[j];
@@ -973,16 +827,16 @@ __global__ void __launch_bounds__(32 * TW) k_traceback64(BatchDev d, int buf_byt
                             pos += je >= 0 && je < j;
                         }
                         const int live = __popc(__ballot_sync(FULL, j >= 0));
-                        double run = 0.0, mine = 0.0;
+                        F run = F(0), mine = F(0);
                         for (int r = 0; r < live; r++) {
                             const unsigned at = __ballot_sync(FULL, j >= 0 && pos == r);
                             run += __shfl_sync(FULL, wt, __ffs(at) - 1);
                             if (j >= 0 && pos == r) mine = run;
                         }
-                        const double pick = uc * run;
+                        const F pick = (F)uc * run;
                         // the first state of all reaches a pick of zero
                         const unsigned hit = __ballot_sync(FULL, j >= 0 && mine >= pick);
-                        if (pick <= 0.0) {
+                        if (pick <= F(0)) {
                             x = 0;
                         } else if (hit) {
                             int best = (hit >> lane & 1) ? j : 0x7fffffff;
@@ -993,8 +847,8 @@ __global__ void __launch_bounds__(32 * TW) k_traceback64(BatchDev d, int buf_byt
                         }
                     } else {
                         const int *determ = d.determ + N.prev_state0;
-                        x = warp_sample<double>(imax(N.S1, 1), uc, [&](int j) {
-                            const double g = j == src.y ? cr : j == src.x ? rr : determ[j] == k ? dp[j] : 0.0;
+                        x = warp_sample<F>(imax(N.S1, 1), uc, [&](int j) {
+                            const F g = j == src.y ? cr : j == src.x ? rr : determ[j] == k ? dp[j] : F(0);
                             return c[j] * g;
                         });
                     }
@@ -1020,38 +874,73 @@ __global__ void __launch_bounds__(32 * TW) k_traceback64(BatchDev d, int buf_byt
                 // trans[j] = TransMatrix::get(j, k) (trans.h:64-83)
                 const StateInfo sk = d.sinfo[B.state0 + state];
                 const long long row = B.t2_0 + d.t2off[B.state0 + state];
+                F stay = F(0);
+                if constexpr (!wide) stay = F(1) - tab.rstay[(size_t)(I.block0 + cur.bi) * MAXT + sk.time];
                 for (int j = tid; j < S; j += 32 * TW) {
                     const StateInfo sj = d.sinfo[B.state0 + j];
-                    trans[j] = sj.node == sk.node ? d.gts[row + (long long)(j - sk.j1) * sk.m]
-                                                  : tmS[sj.time * MAXT + sk.time];
+                    const F tmab = tmS[sj.time * MAXT + sk.time];
+                    F t = tmab;
+                    if (sj.node == sk.node) {
+                        t = TTab<F>::same(tab.rows[row + (long long)(j - sk.j1) * sk.m], tmab);
+                        if (!wide && j == state) t += stay;
+                    }
+                    trans[j] = t;
                 }
-                fresh = false;
             }
-            const int ncols = imin(LOT, c0 - cur.lo + 1), k = state;
-            // lanes a column: 4, 8, 16 or 32, so that few columns still keep every warp busy
-            const int lb = ncols > LOT / 2 ? 2 : ncols > LOT / 4 ? 3 : ncols > LOT / 8 ? 4 : 5;
+            fresh = false;
+            const int ncols = imin(LOT<F>, c0 - cur.lo + 1), k = state;
             if (tid == 0) first = ncols;
             __syncthreads();  // trans, first
-            const int g = tid >> lb, lanes = 1 << lb, q = tid & (lanes - 1);
-            if ((tid & ~31) >> lb < ncols) {
-                const int mc = c0 - imin(g, ncols - 1);
-                const double *cp = column(mc);
-                double before = 0.0, after = 0.0;
-                int j = q;
-#pragma unroll 4
-                for (; j < k; j += lanes) before = fma(cp[j], trans[j], before);
-                j += j == k ? lanes : 0;
-#pragma unroll 4
-                for (; j < S; j += lanes) after = fma(cp[j], trans[j], after);
-                for (int o = 1; o < lanes; o <<= 1) {
-                    before += __shfl_xor_sync(FULL, before, o);
-                    after += __shfl_xor_sync(FULL, after, o);
+            if constexpr (wide) {
+                // lanes a column: 4, 8, 16 or 32, so that few columns still keep every warp busy
+                const int lb = ncols > LOT<F> / 2 ? 2 : ncols > LOT<F> / 4 ? 3 : ncols > LOT<F> / 8 ? 4 : 5;
+                const int g = tid >> lb, lanes = 1 << lb, q = tid & (lanes - 1);
+                if ((tid & ~31) >> lb < ncols) {
+                    const int mc = c0 - imin(g, ncols - 1);
+                    const double *cp = column(mc);
+                    double before = 0.0, after = 0.0;
+                    int j = q;
+    #pragma unroll 4
+                    for (; j < k; j += lanes) before = fma(cp[j], trans[j], before);
+                    j += j == k ? lanes : 0;
+    #pragma unroll 4
+                    for (; j < S; j += lanes) after = fma(cp[j], trans[j], after);
+                    for (int o = 1; o < lanes; o <<= 1) {
+                        before += __shfl_xor_sync(FULL, before, o);
+                        after += __shfl_xor_sync(FULL, after, o);
+                    }
+                    const double through = fma(cp[k], trans[k], before);
+                    const double pick = ub[mc - cur.lo] * (through + after);
+                    const bool leave = g < ncols && !((k == 0 || before < pick) && pick <= through);
+                    const unsigned l = __ballot_sync(FULL, leave);
+                    if (l && lane == 0) atomicMin(&first, (tid + __ffs(l) - 1) >> lb);
                 }
-                const double through = fma(cp[k], trans[k], before);
-                const double pick = ub[mc - cur.lo] * (through + after);
-                const bool leave = g < ncols && !((k == 0 || before < pick) && pick <= through);
-                const unsigned l = __ballot_sync(FULL, leave);
-                if (l && lane == 0) atomicMin(&first, (tid + __ffs(l) - 1) >> lb);
+            } else {
+                // up to 4 columns a warp, as few as keep the warps busy
+                auto draw = [&](auto tag) {
+                    constexpr int G = decltype(tag)::value;
+                    const int g0 = G * warp;
+                    if (g0 >= ncols) return;
+                    const F *cg[G];
+                    double ug[G];
+                    int res[G];
+#pragma unroll
+                    for (int g = 0; g < G; g++) {
+                        const int mc = c0 - imin(g0 + g, ncols - 1);
+                        cg[g] = column(mc);
+                        ug[g] = ub[mc - cur.lo];
+                    }
+                    warp_sample_group<F, G>(S, cg, trans, ug, res);
+#pragma unroll
+                    for (int g = G - 1; g >= 0; g--)
+                        if (lane == 0 && g0 + g < ncols && res[g] != k) {
+                            atomicMin(&first, g0 + g);
+                            draws[g0 + g] = res[g];
+                        }
+                };
+                if (ncols <= TW) draw(Cols<1>{});
+                else if (ncols <= 2 * TW) draw(Cols<2>{});
+                else draw(Cols<4>{});
             }
             __syncthreads();
             const int r = first;
@@ -1059,8 +948,13 @@ __global__ void __launch_bounds__(32 * TW) k_traceback64(BatchDev d, int buf_byt
             if (r < ncols) {
                 // the column that leaves, drawn as one on its own
                 if (warp == 0) {
-                    const double *cp = column(c0 - r);
-                    const int x = warp_sample<double>(S, ub[c0 - r - cur.lo], [&](int j) { return cp[j] * trans[j]; });
+                    int x = 0;
+                    if constexpr (wide) {
+                        const F *cp = column(c0 - r);
+                        x = warp_sample<F>(S, ub[c0 - r - cur.lo], [&](int j) { return cp[j] * trans[j]; });
+                    } else {
+                        x = draws[r];
+                    }
                     if (lane == 0) {
                         path[c0 - r] = x;
                         drawn = x;
@@ -1089,15 +983,16 @@ __global__ void __launch_bounds__(32 * TW) k_traceback64(BatchDev d, int buf_byt
     __syncthreads();
 }
 
-void launch64(const BatchDev &d, cudaStream_t s) {
+template <typename F>
+void launch_lots(const BatchDev &d, cudaStream_t s) {
     // a lot of the largest tree in a buffer, where two buffers leave room for a second CTA on the
     // SM; else as many columns as two buffers hold, at least one
-    const size_t col = 8 * (size_t)imax(d.maxS, 1);
-    const size_t n = 8 * TW * col <= 44 * 1024 ? 8 * TW : imax(imin((int)(100 * 1024 / col), 8 * TW), 1);
+    const size_t col = sizeof(F) * (size_t)imax(d.maxS, 1);
+    const size_t n = LOT<F> * col <= 44 * 1024 ? LOT<F> : imax(imin((int)(100 * 1024 / col), LOT<F>), 1);
     const size_t buf = (n * col + 16 + 15) & ~(size_t)15;
-    const size_t smem = 2 * buf + 2 * (8 * 8 * TW + 32) + col;
-    if (!raise_dynamic_smem(k_traceback64, smem)) return;  // the launch reports it
-    k_traceback64<<<d.ninst, 32 * TW, smem, s>>>(d, (int)buf);
+    const size_t smem = 2 * buf + 2 * (8 * LOT<F> + 32) + col;
+    if (!raise_dynamic_smem(k_traceback_lots<F>, smem)) return;  // the launch reports it
+    k_traceback_lots<F><<<d.ninst, 32 * TW, smem, s>>>(d, (int)buf);
     note_launch();
 }
 
@@ -1114,44 +1009,18 @@ bool launch_split(const BatchDev &d, cudaStream_t s, size_t budget) {
     return true;
 }
 
-template <typename F, int G, int DEPTH>
-bool launch_cfg(const BatchDev &d, cudaStream_t s, size_t budget) {
-    const int maxS = imax(d.maxS, 1);
-    const int slot_elems = (int)(((size_t)maxS * sizeof(F) + 32 + 15) / 16 * 16 / sizeof(F));
-    const size_t smem = (size_t)DEPTH * slot_elems * sizeof(F) + DEPTH * sizeof(double) +
-                  (size_t)(maxS + 1) * sizeof(F) + 2 * (size_t)maxS * sizeof(int) + 16;
-    if (smem > budget) return false;
-    // opt in; static shared memory counts against 48 KB too
-    if (!raise_dynamic_smem(k_traceback<F, G, DEPTH>, smem)) return true;  // the launch reports it
-    k_traceback<F, G, DEPTH><<<d.ninst, 32, smem, s>>>(d, maxS, slot_elems);
-    note_launch();
-    return true;
-}
-
-template <typename F>
-void launch(const BatchDev &d, cudaStream_t s) {
-    // the deepest speculation whose ring leaves room for two CTAs per SM, else one
-    constexpr size_t two = 100 * 1024, one = 200 * 1024;
-    if constexpr (sizeof(F) == 4) {
-        if (d.bins32) {
-            if (launch_split<4>(d, s, 112 * 1024)) return;
-            if (launch_split<3>(d, s, 112 * 1024)) return;
-            if (launch_split<4>(d, s, 224 * 1024)) return;
-            if (launch_split<3>(d, s, 224 * 1024)) return;
-        }
-    }
-    if (launch_cfg<F, 8, 24>(d, s, two)) return;
-    if (launch_cfg<F, 4, 12>(d, s, two)) return;
-    if (launch_cfg<F, 4, 12>(d, s, one)) return;
-    if (launch_cfg<F, 2, 6>(d, s, one)) return;
-    launch_cfg<F, 1, 3>(d, s, 227 * 1024);
-}
-
 }  // namespace
 
 void launch_traceback(const BatchDev &d, bool fp32, cudaStream_t s) {
-    if (fp32) launch<float>(d, s);
-    else launch64(d, s);
+    if (!fp32) {
+        launch_lots<double>(d, s);
+        return;
+    }
+    // the decomposed draw with the deepest ring that leaves room for two CTAs per SM, else one
+    if (d.bins32 && (launch_split<4>(d, s, 112 * 1024) || launch_split<3>(d, s, 112 * 1024) ||
+                     launch_split<4>(d, s, 224 * 1024) || launch_split<3>(d, s, 224 * 1024)))
+        return;
+    launch_lots<float>(d, s);
 }
 
 }  // namespace awg
