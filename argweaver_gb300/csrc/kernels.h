@@ -18,8 +18,10 @@ void launch_tables(const BatchDev &d, bool want32, cudaStream_t s, int *queue = 
 // K2: emissions of variant columns (Felsenstein pruning); as K1.
 void launch_varemit(const BatchDev &d, bool want32, cudaStream_t s, int *queue = nullptr,
                     int chunk = 1);
-// Whether K2's carve with FP64 per-state factors and 8-byte scratch (needed for FP64 and
-// double-float emissions) fits this largest tree.
+// K2 for an FP32 batch whose variant columns are formed in double-float (BatchDev::vardf).
+void launch_varemit_df(const BatchDev &d, cudaStream_t s, int *queue, int chunk);
+// Whether K2's carve with FP64 per-state factors and 8-byte scratch fits this largest tree: an
+// FP32 batch then forms its variant columns in double-float.
 bool varemit_full_carve_fits(int maxnodes, int maxS);
 // K3: forward pass, one CTA per instance; kpt: at least this many states per owner thread of
 // the FP32 kernel (0: chosen by the state count). table: the FP64 table is to be read, so its

@@ -22,6 +22,7 @@
 #include <cmath>
 #include <cstdio>
 
+#include "emit_common.cuh"
 #include "kernels.h"
 #include "tree_util.cuh"
 
@@ -1076,23 +1077,6 @@ __global__ void __launch_bounds__(TAB_THREADS) k_tables(BatchDev d, int want32) 
     tables_tree(d, cta_block(d), want32);
 }
 
-// Work queue of a persistent per-tree kernel: units of `chunk` consecutive trees in the
-// batch's tree order (largest instances first), taken by CTAs with an atomic counter.
-struct WorkQueue {
-    int *counter;
-    int nunits, chunk;
-};
-
-// Takes the next unit for the whole CTA; -1 when the queue is empty.
-__device__ __forceinline__ int next_unit(const WorkQueue &q) {
-    __shared__ int unit;
-    __syncthreads();  // the previous unit's reads of `unit` are done
-    if (threadIdx.x == 0) unit = atomicAdd(q.counter, 1);
-    __syncthreads();
-    const int u = unit;
-    return u < q.nunits ? u : -1;
-}
-
 // K1 as a persistent kernel: as many CTAs as fit on the GPU at once, each taking units of
 // trees until the queue is empty (work-stealing over (instance, tree-chunk) units).
 __global__ void __launch_bounds__(TAB_THREADS) k_tables_ws(BatchDev d, int want32, WorkQueue q) {
@@ -1107,6 +1091,9 @@ __global__ void __launch_bounds__(TAB_THREADS) k_tables_ws(BatchDev d, int want3
 
 // ---------------------------------------------------------------------------------------
 // K2: emissions of variant columns (calc_emissions' non-invariant branch, emit.cpp:822-844)
+// of the FP64 path, and of FP32 batches whose largest tree leaves no room for double-float
+// (about 1,800 states at 259 nodes; the others take emit_df.cu's kernel: 6.28 ms here and
+// 1.26 ms there for 840 trees of 150 to 200 leaves).
 //
 // One CTA per local tree. Once per tree: the branch mutation probabilities, the per-state
 // factors of the three split branches (prob_branch, emit.cpp:787-805, FP64), and two level
@@ -1153,154 +1140,15 @@ __device__ __forceinline__ void jc_apply_x(const R *x, R m, R nm, R *y) {
 template <typename R>
 __device__ __forceinline__ R cprod(R a, R b) { return (a + b) - a * b; }
 
-// Double-float: value = hi + lo, |lo| <= ulp(hi) / 2, about 48 significant bits, from
-// FP32 error-free transforms (Knuth's two-sum; the product's error by fused multiply-add).
-// The FP32 path's variant-column emissions are formed in it: the forward posterior amplifies
-// an error of those emissions thousands-fold on the columns where they differ little between
-// states, so they must reach FP32 as correctly rounded ratios to the column's largest. FP32
-// forms left the posterior up to 6.6e-5 from FP64's (9.1e-5 with only the partials in
-// double-float); double-float, 3.1e-6 (k = 64, 100,000 columns).
-struct df {
-    float hi, lo;
-    __device__ __forceinline__ df() : hi(0.f), lo(0.f) {}
-    __device__ __forceinline__ df(double x) : hi((float)x), lo((float)(x - (double)(float)x)) {}
-    // small integer constants (0, 1, 4 in the emission forms) without the FP64 split
-    __device__ __forceinline__ df(int x) : hi((float)x), lo(0.0f) {}
-    __device__ __forceinline__ df(float h, float l) : hi(h), lo(l) {}
-    __device__ __forceinline__ explicit operator double() const { return (double)hi + (double)lo; }
-};
-__device__ __forceinline__ df df_fast2(float a, float b) {  // |a| >= |b|
-    const float s = __fadd_rn(a, b);
-    return df(s, __fsub_rn(b, __fsub_rn(s, a)));
-}
-__device__ __forceinline__ df operator+(df a, df b) {
-    const float s = __fadd_rn(a.hi, b.hi);
-    const float bb = __fsub_rn(s, a.hi);
-    const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fsub_rn(b.hi, bb));
-    return df_fast2(s, __fadd_rn(e, __fadd_rn(a.lo, b.lo)));
-}
-__device__ __forceinline__ df operator-(df a) { return df(-a.hi, -a.lo); }
-__device__ __forceinline__ df operator-(df a, df b) { return a + (-b); }
-__device__ __forceinline__ df operator*(df a, df b) {
-    const float p = __fmul_rn(a.hi, b.hi);
-    const float e = __fmaf_rn(a.hi, b.hi, -p);
-    return df_fast2(p, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, e)));
-}
-__device__ __forceinline__ df &operator+=(df &a, df b) { return a = a + b; }
-__device__ __forceinline__ bool operator<(df a, df b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
-// a + b for a, b >= 0 (every sum of the emission passes: partials, branch probabilities and
-// their products): the larger high part first makes Dekker's fast two-sum exact, three adds
-// where the two-sum of arbitrary signs takes six
-__device__ __forceinline__ df df_addp(df a, df b) {
-    const float big = fmaxf(a.hi, b.hi), small = fminf(a.hi, b.hi);
-    const float s = __fadd_rn(big, small);
-    const float e = __fsub_rn(small, __fsub_rn(s, big));
-    return df_fast2(s, __fadd_rn(e, __fadd_rn(a.lo, b.lo)));
-}
-// a * b + c, a, b, c >= 0 (the JC69 steps of the emission passes)
-__device__ __forceinline__ df fma(df a, df b, df c) { return df_addp(a * b, c); }
-__device__ __forceinline__ df fmax(df a, df b) { return a < b ? b : a; }
-__device__ __forceinline__ df __shfl_xor_sync(unsigned mask, df v, int o) {
-    return df(::__shfl_xor_sync(mask, v.hi, o), ::__shfl_xor_sync(mask, v.lo, o));
-}
-// the built-in overloads stay visible beside the double-float ones
-using ::fmax;
-using ::fma;
-using ::__shfl_xor_sync;
-
 // Per-tree context of K2 shared by the column passes.
-struct EmitCtx {
-    const int4 *nd;
+struct EmitCtx : TreeLevels {
     const double *muts, *nomuts, *pm;  // branch and per-state split-branch probabilities
     const float *muts32, *nomuts32;    // FP32 copies (converted once per tree)
     const float *pm32;                 // [S][8]: mut0..2, nomut0..2, 1 - 4 mut0, unused
-    const int *snode, *inl, *inp, *outl, *outp;
+    const int *snode;
     const uint8_t *sfloor;  // per state: a split branch of it was raised to mintime
-    int nlev_in, nlev_out, mainr, node1, S, ns, nleaves, n;
-    bool internal;
-    // The FP32 path's double-float forms (BatchDev::vardf): muts, nomuts and pm then hold
-    // double-float values, 8 bytes each in the same slots, so that the steps read them with
-    // no conversion (a conversion from double runs on the FP64 pipe, in every step)
-    __device__ __forceinline__ df dmut(int j) const { return ((const df *)muts)[j]; }
-    __device__ __forceinline__ df dnomut(int j) const { return ((const df *)nomuts)[j]; }
-    __device__ __forceinline__ df dpm(size_t i) const { return ((const df *)pm)[i]; }
+    int S;
 };
-
-__device__ __forceinline__ int base_bit(uint8_t ch) {
-    if (ch == 'N') return 0;
-    return 1 << ((ch == 'A' || ch == 'a') ? 0 : (ch == 'C' || ch == 'c') ? 1
-                 : (ch == 'G' || ch == 'g') ? 2 : 3);
-}
-
-// Infinite-sites validity of one variant column's nodes (get_infinite_sites_states,
-// emit.cpp:454-589, with parsimony_ancestral_set :898-953) by one warp over the level
-// schedules: Fitch sets by height, then refined from the main root down (any order with
-// children first, then parents first, gives the reference's sets). A state on node j keeps
-// the model when the threaded base (the cut subtree's set) meets the set of j or of its
-// parent. Node j's flag is bit j / 32 of lane j % 32's word; all flags are 1 when the
-// column cannot break the model. sets, anc: n bytes each of the warp's scratch.
-__device__ unsigned infsites_nodes(const EmitCtx &c, const uint8_t *chars, uint8_t *sets,
-                                   uint8_t *anc) {
-    constexpr unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int4 *nd = c.nd;
-    int all = 0, subset = 0, mainset = 0;
-    for (int x = lane; x < c.inp[1]; x += 32) {
-        const int j = c.inl[x];
-        const int b = base_bit(chars[j]);
-        sets[j] = (uint8_t)b;
-        if (!c.internal) {
-            all |= b;
-        } else {
-            int u = j;
-            for (int s = 0; u != -1 && u != c.node1 && s < c.n; s++) u = nd[u].x;
-            if (u == c.node1) subset |= b;
-            else mainset |= b;
-        }
-    }
-    all = __reduce_or_sync(FULL, all);
-    subset = __reduce_or_sync(FULL, subset);
-    mainset = __reduce_or_sync(FULL, mainset);
-    __syncwarp();
-    for (int h = 1; h < c.nlev_in; h++) {
-        for (int x = c.inp[h] + lane; x < c.inp[h + 1]; x += 32) {
-            const int j = c.inl[x];
-            const int l = sets[nd[j].y], r = sets[nd[j].z];
-            sets[j] = (uint8_t)((l & r) ? (l & r) : (l | r));
-        }
-        __syncwarp();
-    }
-    const int cset = c.internal ? sets[c.node1] : base_bit(chars[c.nleaves]);
-    if (c.internal ? !(subset & mainset) : !(cset & all)) return FULL;
-    for (int h = 0; h < c.nlev_out; h++) {
-        for (int x = c.outp[h] + lane; x < c.outp[h + 1]; x += 32) {
-            const int j = c.outl[x];
-            if (j == c.mainr) {
-                anc[j] = sets[j];
-            } else {
-                const int ps = anc[nd[j].x] & sets[j];
-                anc[j] = (uint8_t)(ps ? ps : sets[j]);
-            }
-        }
-        __syncwarp();
-    }
-    unsigned word = FULL;
-    for (int w = 0; w * 32 + lane < c.n && w < 32; w++) {
-        const int j = w * 32 + lane;
-        int u = j;  // in the main tree (the only nodes with states)
-        for (int s = 0; u != -1 && u != c.mainr && s < c.n; s++) u = nd[u].x;
-        if (u != c.mainr) continue;
-        const bool ok = (cset & anc[j]) || (j != c.mainr && (cset & anc[nd[j].x]));
-        if (!ok) word &= ~(1u << w);
-    }
-    __syncwarp();
-    return word;
-}
-
-// Whether state k's node keeps the infinite-sites model (all lanes call it).
-__device__ __forceinline__ bool state_ok(unsigned word, int node) {
-    return (__shfl_sync(0xffffffffu, word, node & 31) >> (node >> 5)) & 1;
-}
 
 // Column forms of the partials and emissions:
 //   REF  FP64, the reference's order of operations (plain path)
@@ -1332,15 +1180,12 @@ __device__ R emit_column(const EmitCtx &c, const uint8_t *chars, int X, R (*in)[
         else leaf_partial<R>(ch, v);
     };
     constexpr bool F32 = std::is_same<R, float>::value;
-    constexpr bool DF = std::is_same<R, df>::value;
     auto bm = [&](int j) -> R {
         if constexpr (F32) return c.muts32[j];
-        else if constexpr (DF) return c.dmut(j);
         else return (R)c.muts[j];
     };
     auto bn = [&](int j) -> R {
         if constexpr (F32) return c.nomuts32[j];
-        else if constexpr (DF) return c.dnomut(j);
         else return (R)c.nomuts[j];
     };
     auto step = [&](const R *x, R m, R nm, R *y) {
@@ -1425,8 +1270,7 @@ __device__ R emit_column(const EmitCtx &c, const uint8_t *chars, int X, R (*in)[
             q[0] = qa.x; q[1] = qa.y; q[2] = qa.z; q[3] = qa.w; q[4] = qb.x; q[5] = qb.y; q[6] = qb.z;
         } else {
             for (int t = 0; t < 6; t++) {
-                if constexpr (DF) q[t] = c.dpm(6 * (size_t)k + t);
-                else q[t] = (R)c.pm[6 * k + t];
+                q[t] = (R)c.pm[6 * k + t];
             }
             q[6] = R(1) - R(4) * q[0];
         }
@@ -1510,129 +1354,6 @@ __device__ R emit_column(const EmitCtx &c, const uint8_t *chars, int X, R (*in)[
     }
     __syncwarp();
     return ref;
-}
-
-// A column whose observed calls all show one base X (it varies only through missing calls),
-// in double-float by one warp: 4 e_k into eb[S], returns the largest. Every partial is then
-// symmetric in the other three bases (the leaves' are (1, 0) or, missing, (1, 1); JC69 treats
-// the three alike), so it is kept as the pair (x_X, x_other): half the work of the four-base
-// form, the same sums. The FP32 path's columns of this kind (about 26% of all columns at
-// 0.5% missing calls, 87% of the variant ones) are where the forward posterior amplifies an
-// emission error most: their emissions differ little between states.
-__device__ df emit_near_df(const EmitCtx &c, const uint8_t *chars, int X, df (*in)[2],
-                           df (*out)[2], df *eb) {
-    const int lane = threadIdx.x & 31;
-    const int4 *nd = c.nd;
-    // JC69 over a branch with m (to each other base), nm (no change)
-    auto step = [](const df *x, df m, df nm, df *y) {
-        const df dd = nm - m, ms = m * df_addp(x[0], df(3.0f, 0.0f) * x[1]);
-        y[0] = df_addp(dd * x[0], ms);
-        y[1] = df_addp(dd * x[1], ms);
-    };
-    auto leaf = [](uint8_t ch, df *v) {  // observed calls are X here
-        v[0] = df(1.0f, 0.0f);
-        v[1] = ch == 'N' ? df(1.0f, 0.0f) : df();
-    };
-    (void)X;
-    for (int x = lane; x < c.inp[1]; x += 32) leaf(chars[c.inl[x]], in[c.inl[x]]);
-    __syncwarp();
-    for (int h = 1; h < c.nlev_in; h++) {
-        for (int x = c.inp[h] + lane; x < c.inp[h + 1]; x += 32) {
-            const int j = c.inl[x];
-            const int c1 = nd[j].y, c2 = nd[j].z;
-            df p1[2], p2[2];
-            step(in[c1], c.dmut(c1), c.dnomut(c1), p1);
-            step(in[c2], c.dmut(c2), c.dnomut(c2), p2);
-            in[j][0] = p1[0] * p2[0];
-            in[j][1] = p1[1] * p2[1];
-        }
-        __syncwarp();
-    }
-    for (int h = 0; h < c.nlev_out; h++) {
-        for (int x = c.outp[h] + lane; x < c.outp[h + 1]; x += 32) {
-            const int j = c.outl[x];
-            if (j == c.mainr) {
-                out[j][0] = out[j][1] = df(1.0f, 0.0f);
-                continue;
-            }
-            const int p = nd[j].x;
-            const int sib = nd[p].y == j ? nd[p].z : nd[p].y;
-            df p1[2];
-            step(in[sib], c.dmut(sib), c.dnomut(sib), p1);
-            if (p != c.mainr) {
-                df p2[2];
-                step(out[p], c.dmut(p), c.dnomut(p), p2);
-                out[j][0] = p1[0] * p2[0];
-                out[j][1] = p1[1] * p2[1];
-            } else {
-                out[j][0] = p1[0];
-                out[j][1] = p1[1];
-            }
-        }
-        __syncwarp();
-    }
-    df in2[2];
-    if (c.internal) {
-        in2[0] = in[c.node1][0];
-        in2[1] = in[c.node1][1];
-    } else {
-        leaf(chars[c.nleaves], in2);
-    }
-    auto state_v = [&](int k) -> df {
-        const int node2 = c.snode[k];
-        const size_t q = 6 * (size_t)k;  // mut0..2, nomut0..2
-        df p1[2], p2[2], t[2];
-        step(in2, c.dpm(q), c.dpm(q + 3), p1);
-        step(in[node2], c.dpm(q + 1), c.dpm(q + 4), p2);
-        if (node2 != c.mainr) {
-            df p3[2];
-            step(out[node2], c.dpm(q + 2), c.dpm(q + 5), p3);
-            t[0] = p2[0] * p3[0];
-            t[1] = p2[1] * p3[1];
-        } else {
-            t[0] = p2[0];
-            t[1] = p2[1];
-        }
-        return df_addp(p1[0] * t[0], df(3.0f, 0.0f) * (p1[1] * t[1]));
-    };
-    // two states per lane at a time: independent chains the scheduler can interleave (the
-    // second one repeats the last state where it would run past S)
-    df ref = df();
-    for (int k0 = lane; k0 < c.S; k0 += 64) {
-        const int k1 = k0 + 32 < c.S ? k0 + 32 : k0;
-        const df v0 = state_v(k0), v1 = state_v(k1);
-        eb[k0] = v0;
-        eb[k1] = v1;
-        ref = fmax(ref, fmax(v0, v1));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ref = fmax(ref, __shfl_xor_sync(0xffffffffu, ref, o));
-    __syncwarp();
-    return ref;
-}
-
-// FP32 path: a tree's share of the log-likelihood's emission references, lneref per
-// invariant column and log(vref) per variant column (the instance's column 0, the prior, has
-// none), summed by one warp in a fixed order. The logarithms are taken here, a lane per
-// column, not by one lane per column in the emission passes: there an FP64 log holds the
-// warp's FP64 pipe for a few thousand cycles per column.
-__device__ void block_log_offset(const BatchDev &d, const BlockDev &B, const InstDev &I, int blk,
-                                 int lane) {
-    const uint8_t *cls = d.colclass + I.col0 + B.start;
-    const int *cvar = d.colvar + I.col0 + B.start;
-    const double lner = d.lneref[blk];
-    double s = 0.0;
-    if (B.S > 0) {
-        for (int i = lane; i < B.len; i += 32) {
-            if (B.b == 0 && i == 0) continue;
-            const uint8_t c = cls[i];
-            if (c == COL_INVARIANT) s += lner;
-            else if (c == COL_VARIANT) s += log(d.vref[B.vrow0 + cvar[i]]);
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) d.blkext[blk] = s;
 }
 
 // Variant-column emissions of one local tree, by the whole CTA (nwarps warps).
@@ -1726,11 +1447,6 @@ __device__ __forceinline__ void varemit_tree(const BatchDev &d, int blk, int nwa
         return;
     }
     for (int i = tid; i < n; i += blockDim.x) nd[i] = d.nodes[B.nodes0 + i];
-    // FP32 path with double-float variant columns: every variant column takes that form
-    // (penalised ones too), so the split-branch factors are stored as double-float and no
-    // FP32 form's copies are made
-    const bool f32forms = FP32OUT && !d.vardf;
-    const bool dfpm = FP32OUT && d.vardf;
     const bool refill = bc->inst != B.inst;  // read by all before anyone rewrites it
     __syncthreads();
     if (refill) {
@@ -1758,14 +1474,9 @@ __device__ __forceinline__ void varemit_tree(const BatchDev &d, int blk, int nwa
                 m0 = branch_nomut(e);
             }
         }
-        if (dfpm) {
-            ((df *)muts)[i] = df(m1);
-            ((df *)nomuts)[i] = df(m0);
-        } else {
-            muts[i] = m1;
-            nomuts[i] = m0;
-        }
-        if (f32forms) {
+        muts[i] = m1;
+        nomuts[i] = m0;
+        if (FP32OUT) {
             muts32[i] = (float)m1;
             nomuts32[i] = (float)m0;
         }
@@ -1791,20 +1502,13 @@ __device__ __forceinline__ void varemit_tree(const BatchDev &d, int blk, int nwa
                          : branch_exp(fmax(coal_time - time1, mintime), mu);
         e[1] = age2 < T ? bc->e[age2][a] : branch_exp(fmax(coal_time - time2, mintime), mu);
         e[2] = parent != -1 ? bc->e[a][pidx] : bc->ez[a];
-        if (dfpm) {  // branch_mut / branch_nomut in double-float: one FP64 split each
-            const df quarter(0.25f, 0.0f), one(1.0f, 0.0f), three(3.0f, 0.0f);
-            for (int x = 0; x < 3; x++) {
-                const df ex(e[x]);
-                ((df *)pm)[6 * k + x] = quarter * (one - ex);
-                ((df *)pm)[6 * k + 3 + x] = quarter * (one + three * ex);
-            }
-        } else if (!lean) {
+        if (!lean) {
             for (int x = 0; x < 3; x++) {
                 pm[6 * k + x] = branch_mut(e[x]);
                 pm[6 * k + 3 + x] = branch_nomut(e[x]);
             }
         }
-        if (f32forms) {
+        if (FP32OUT) {
             for (int x = 0; x < 3; x++) {
                 pm32[8 * k + x] = (float)branch_mut(e[x]);
                 pm32[8 * k + 3 + x] = (float)branch_nomut(e[x]);
@@ -1847,9 +1551,8 @@ __device__ __forceinline__ void varemit_tree(const BatchDev &d, int blk, int nwa
     }
     __syncthreads();
 
-    const EmitCtx ctx{nd,      muts,     nomuts,   pm,   muts32,  nomuts32, pm32, snode,
-                      inl,     inp,      outl,     outp, sfloor,  nlev_in,  nlev_out,
-                      mainr,   node1,    S,        I.nseqs, I.nleaves, n,   internal};
+    const EmitCtx ctx{{nd, inl, inp, outl, outp, nlev_in, nlev_out, mainr, node1, I.nleaves, n, internal},
+                      muts, nomuts, pm, muts32, nomuts32, pm32, snode, sfloor, S};
     double *wscr = (double *)((char *)scratch + (size_t)warp * n * 8 * esz);
     double *eb = (double *)(ebuf + (size_t)warp * maxS * esz);  // read as float when lean
     const uint8_t *cls = d.colclass + I.col0 + B.start;
@@ -1900,7 +1603,7 @@ __device__ __forceinline__ void varemit_tree(const BatchDev &d, int blk, int nwa
                 if (penalised) penalise(eb);
                 double *row = d.varemit + B.var0 + (size_t)vrow * S;
                 for (int k = lane; k < S; k += 32) row[k] = eb[k];
-            } else if (penalised && !d.vardf) {
+            } else if (penalised) {
                 // FP64 emissions, penalised, then relative to the column's largest
                 const int X0 = 0;
                 emit_column<double, EM_F64>(ctx, chars, X0, (double (*)[4])wscr,
@@ -1943,7 +1646,7 @@ __device__ __forceinline__ void varemit_tree(const BatchDev &d, int blk, int nwa
                     near = !__any_sync(0xffffffffu, other);
                 }
                 float *row = d.var32 + B.var0 + (size_t)vrow * S;
-                if (near && !d.vardf) {
+                if (near) {
                     float *fs = (float *)wscr, *fe = (float *)eb;
                     const float dref = emit_column<float, EM_REL>(ctx, chars, X, (float (*)[4])fs,
                                                                   (float (*)[4])fs + n, fe);
@@ -1953,53 +1656,6 @@ __device__ __forceinline__ void varemit_tree(const BatchDev &d, int blk, int nwa
                         row[k] = c <= 0.5f ? c : -((1.f - fe[k]) * inv1);
                     }
                     if (lane == 0) d.vref[B.vrow0 + vrow] = .25 * (1.0 - (double)dref);
-                } else if (d.vardf) {
-                    // the forward posterior amplifies an error of a variant column's
-                    // emissions thousands-fold where they differ little between states (the
-                    // columns that vary only through missing calls): the partials and every
-                    // state's split-branch steps are formed in double-float and each ratio
-                    // to the column's largest is rounded once
-                    // (FP64 arithmetic only once per column: per state it would hold the
-                    // FP64 pipe, 64 cycles a warp instruction)
-                    df *ed = (df *)eb;
-                    df eref =
-                        near ? emit_near_df(ctx, chars, X, (df (*)[2])wscr, (df (*)[2])wscr + n, ed)
-                             : emit_column<df, EM_F64>(ctx, chars, 0, (df (*)[4])wscr,
-                                                       (df (*)[4])wscr + n, ed);
-                    if (penalised) {
-                        // states that break the infinite-sites model times the penalty
-                        // (emit.cpp:847-862); below FP32's range that leaves the ratio 0,
-                        // written as the smallest negative value below, as the FP64 form
-                        // writes it
-                        const df pen(penalty);
-                        df mx;
-                        for (int kb = 0; kb < S; kb += 32) {
-                            const int k = kb + lane;
-                            const bool ok = state_ok(vword, k < S ? snode[k] : 0);
-                            if (k < S) {
-                                if (!ok) ed[k] = ed[k] * pen;
-                                mx = fmax(mx, ed[k]);
-                            }
-                        }
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-                        eref = mx;
-                        __syncwarp();
-                    }
-                    // 1 / (4 e_ref): the FP32 reciprocal and one Newton step in double-float
-                    const df one(1.0f, 0.0f);
-                    const df y0(1.0f / eref.hi, 0.0f);
-                    const df inv1 = y0 + y0 * (one - eref * y0);
-                    for (int k = lane; k < S; k += 32) {
-                        // e_k / e_ref; the largest state's r can round a hair above 1, so its
-                        // complement is clamped at +0 (a negative value would read as a
-                        // ratio, i.e. an emission near zero)
-                        const df r = ed[k] * inv1;
-                        float v = r.hi >= 0.5f ? fmaxf((one - r).hi, 0.0f) : -r.hi;
-                        if (r.hi < 0.5f && v == 0.0f) v = -__int_as_float(1);  // stays a ratio
-                        row[k] = v;
-                    }
-                    if (lane == 0) d.vref[B.vrow0 + vrow] = .25 * (double)eref;
                 } else if (!internal) {
                     // brackets against the column's largest: D form x / plain form y
                     float *fs = (float *)wscr, *fe = (float *)eb;
@@ -2077,20 +1733,6 @@ size_t tables_smem(int n, int S, int S1, int T, bool want32) {
 
 }  // namespace
 
-// CTAs of a persistent kernel: as many as are resident on the GPU at once, at most one per
-// unit of work.
-template <typename K>
-int persistent_grid(K kernel, int threads, size_t smem, int nunits) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 1;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    return imax(1, imin(nunits, per_sm * sms));
-}
-
 void launch_tables(const BatchDev &d, bool want32, cudaStream_t s, int *queue, int chunk) {
     size_t smem = tables_smem(d.maxnodes, d.maxS, d.maxS, d.maxT, want32);
     if (!queue) {
@@ -2155,7 +1797,8 @@ void launch_varemit_t(const BatchDev &d, cudaStream_t s, int *queue, int chunk) 
 }
 
 void launch_varemit(const BatchDev &d, bool fp32, cudaStream_t s, int *queue, int chunk) {
-    if (fp32) launch_varemit_t<true>(d, s, queue, chunk);
+    if (fp32 && d.vardf) launch_varemit_df(d, s, queue, chunk);
+    else if (fp32) launch_varemit_t<true>(d, s, queue, chunk);
     else launch_varemit_t<false>(d, s, queue, chunk);
 }
 
