@@ -5,7 +5,8 @@
 // per instance:
 //   k_traceback_lots  the reference's scan, a CTA drawing or testing many columns at once: FP64,
 //                     and FP32 where the decomposed draw's tables do not fit
-//   k_traceback_split FP32: the draw decomposed by the structure of the transition
+//   k_traceback_split FP32: the draw decomposed by the structure of the transition, by one warp
+//                     with two that bring its tables
 //
 // The scan by one warp splits the states into 32 contiguous chunks (lane t sums chunk t with
 // two accumulators, even and odd states); chunk sums are scanned across lanes and the chunk
@@ -36,6 +37,13 @@ template <> struct TTab<float> {
           rrow(d.recombrow32), crow(d.recoalrow32), fw(d.fw32) {}
     __device__ static float same(float v, float tmab) { return v + tmab; }
 };
+
+// A hint that moves the whole 16-byte granules of [p, p + bytes) from HBM into L2.
+__device__ __forceinline__ void l2_prefetch(const void *p, size_t bytes) {
+    const uintptr_t a = ((uintptr_t)p + 15) & ~(uintptr_t)15, e = ((uintptr_t)p + bytes) & ~(uintptr_t)15;
+    if (e > a)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(e - a)) : "memory");
+}
 
 // Inclusive lane scan.
 template <typename F>
@@ -233,429 +241,555 @@ __device__ void warp_sample_group(int n, const F *const (&cg)[G], const F *trans
 // state carry weight (its gather list plus the recombination and recoalescence sources),
 // so the switch draw runs over those, in state order.
 //
-// Speculation: the warp tests 8 columns at once for the common case, the draw staying at
-// the current state k: lanes 4g .. 4g+3 take column g, each a quarter of the node's states
-// and of the bins, and combine V before k, V at k, V and W by two butterfly steps. The
-// first column whose draw leaves k (if any) is drawn exactly by the whole warp; the
-// columns after it are tested again under the new state.
+// Speculation: the warp tests up to 32 columns at once for the common case, the draw staying at
+// the current state k: four lanes take a column's V and W terms, four columns each, in whatever
+// order suits the loads. All terms are >= 0, so a sum in any order is within 64 roundings of the
+// one that the draw is defined by (quarters of the states and of the bins in order, then a
+// tree), and a column whose pick lies within `margin` of an end of k's interval is decided by
+// that one. The first column that leaves k (about one in a thousand inside an external tree, one
+// in a few hundred of a cut one) is drawn exactly by the whole warp; the columns after it are
+// tested again under the new state.
 //
-// Data movement is TMA bulk copies (cp.async.bulk) completing on mbarriers, issued by one
-// lane: the forward table streams into a ring of NCH chunks of up to 8 consecutive columns
-// of one tree (one copy for the chunk's columns, one for their bins, one for their
-// uniforms), and each tree's tables (tmatrix, stay complements, time-bin CSR, state info,
-// row offsets, switch gather lists and probabilities) into one of two buffers one tree
-// ahead. Every wait is bounded; one that runs out records ERR_WAIT_LIMIT and the kernel
-// returns after its copies have landed.
+// What bounds it: latencies on one warp's path, a tree of some 28 columns (at 100 leaves) after
+// the other, so per tree there is one wait for the forward table: a test reads only the states of
+// k's node, straight from L2, and the switch's sources (a lane each) are loaded with the last
+// test, for the state that the tree will most likely keep. Everything else is in shared memory
+// by then: two producer warps copy it by TMA (cp.async.bulk) completing on mbarriers, one the
+// bins and uniforms of up to 32 columns of a tree at a time into a ring (and hints the table into
+// L2), the other each tree's tables into one of three buffers (two where three do not fit), with
+// its same-branch rows and breakpoint factors where they fit (STAGED; else they are read from
+// global memory).
+// 0.085 us a column at 100 leaves; with whole columns copied in by the drawing warp itself, 8
+// tested at a time, and rows and factors read when needed, 0.210. Every wait is bounded; one that
+// runs out records ERR_WAIT_LIMIT and the kernel returns after its copies have landed.
 
-// Fields of a tree the traceback needs, in registers.
+constexpr float margin = 2e-5f;  // over twice 64 roundings
+
+// Fields of a tree the traceback needs.
 struct TreeRef {
-    int blk, start, len, S, S1;
+    int blk, start, len, S, S1, M;
     long long cell0, state0, prev_state0, t2_0, gptr0;
 };
 __device__ __forceinline__ TreeRef tree_ref(const BatchDev &d, int blk) {
     const BlockDev &B = d.blocks[blk];
-    return TreeRef{blk, B.start, B.len, B.S, B.S1, B.cell0, B.state0, B.prev_state0, B.t2_0, B.gptr0};
+    return TreeRef{blk, B.start, B.len, B.S, B.S1, B.M, B.cell0, B.state0, B.prev_state0, B.t2_0, B.gptr0};
 }
 
-// Layout of one tree buffer (bytes from its start; every part 16-byte aligned).
+// The arrays of a tree buffer, each copied from the 16-byte boundary below its start.
+enum { A_TM, A_RSTAY, A_BPTR, A_SINFO, A_T2OFF, A_PERM, A_GPTR, A_GIDX, A_DP, A_RROW, A_CROW, A_ROWS, ARRAYS };
+// Layout of one tree buffer: array a from word at[a] on.
 struct TreeBufLayout {
-    int tm, rstay, bptr, sinfo, t2off, perm, gptr, gidx, dp, total;
-    __host__ __device__ explicit TreeBufLayout(int maxS) {
-        const int arr = (4 * maxS + 32 + 15) & ~15;  // a 4-byte array copied from its 16-B start
-        tm = 0;
-        rstay = tm + 4 * MAXT * MAXT;
-        bptr = rstay + 4 * MAXT;
-        sinfo = bptr + 160;
-        t2off = sinfo + 16 * maxS;
-        perm = t2off + arr;
-        gptr = perm + arr;
-        gidx = gptr + arr;
-        dp = gidx + arr;
-        total = dp + arr;
+    int at[ARRAYS], total;
+    // maxM: entries of the same-branch rows, 0: neither they nor the breakpoint's factors staged
+    __host__ __device__ TreeBufLayout(int maxS, int maxM) {
+        const int arr = (4 * maxS + 32 + 15) & ~15;
+        const int bytes[ARRAYS] = {4 * MAXT * MAXT, 4 * MAXT, 160, 16 * maxS, arr, arr, arr, arr, arr,
+                                   maxM > 0 ? arr : 0, maxM > 0 ? arr : 0,
+                                   maxM > 0 ? (4 * maxM + 32 + 15) & ~15 : 0};
+        total = 0;
+        for (int a = 0; a < ARRAYS; a++) {
+            at[a] = total / 4;
+            total += bytes[a];
+        }
     }
 };
+// A tree as its buffer holds it.
+struct TreeTables {
+    TreeRef ref;
+    int2 src;         // the breakpoint's states
+    int off[ARRAYS];  // where each array begins, in words of the buffer
+};
 
-constexpr int CW = 8;  // columns per ring chunk (= the speculation group)
+constexpr int CC = 32;  // columns of a chunk and of a test: a tree's, from its last down
+constexpr int NCH = 4;  // chunks of the ring
+constexpr int CHUNK_BYTES = 4 * CC * MAXT + 8 * (CC + 4);  // bins, then uniforms (the column before too)
 
-// Bytes of one ring chunk's table part.
-__host__ __device__ inline int chunk_tab_bytes(int maxS) { return (4 * CW * maxS + 32 + 15) & ~15; }
-
-template <int NCH>
-__global__ void __launch_bounds__(32) k_traceback_split(BatchDev d, int maxS) {
-    constexpr int G = CW;
+template <bool STAGED>
+__global__ void __launch_bounds__(96) k_traceback_split(BatchDev d, int maxS, int nbuf) {
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) unsigned char dyn_b[];
-    const int tab_bytes = chunk_tab_bytes(maxS);
-    unsigned char *rtab = dyn_b;                                     // [NCH] table chunks
-    float *rbins = (float *)(rtab + (size_t)NCH * tab_bytes);        // [NCH][CW][MAXT]
-    double *ru = (double *)(rbins + NCH * CW * MAXT);                // [NCH][CW + 2]
-    unsigned char *tbuf = (unsigned char *)(ru + NCH * (CW + 2));    // [2] tree buffers
-    __shared__ uint64_t cbar[NCH];                                   // chunk barriers
-    __shared__ uint64_t tbar[2];                                     // tree buffer barriers
-    __shared__ int ch_lo[NCH], ch_cnt[NCH], ch_off[NCH], ch_uoff[NCH], ch_S[NCH];
-    __shared__ float t2row[32], tmcol[32];                           // the state's V, W factors
-    const TreeBufLayout TL(maxS);
+    unsigned char *ring = dyn_b;                            // [NCH] chunks
+    unsigned char *tbuf = ring + NCH * CHUNK_BYTES;         // [nbuf] tree buffers
+    __shared__ uint64_t cfull[NCH], cfree[NCH], tfull[3], tfree[3];  // copies landed; buffer read
+    __shared__ int chunks_issued, trees_issued;
+    __shared__ volatile int stop;
+    __shared__ TreeTables trees[3];
+    __shared__ __align__(16) float t2row[32], tmcol[32];    // the state's V, W factors
+    __shared__ float ordw[32];
+    __shared__ int ordj[32];
+    const TreeBufLayout TL(maxS, STAGED ? d.maxM : 0);
     const TTab<float> tab(d);
     const int qi = cta_instance(d);
     const InstDev I = d.inst[qi];
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int NB = I.T - 1;
-    int *path = d.path + I.col0;
-    const double *u = d.uniforms + I.col0;
-    const float *bins = d.bins32 + (size_t)I.col0 * MAXT;
     const int L = I.seqlen;
-    bool failed = false;
+    const double *u = d.uniforms + I.col0;
 
-    if (lane == 0) {
-        for (int q = 0; q < NCH; q++) mbar_init(&cbar[q], 1);
-        mbar_init(&tbar[0], 1);
-        mbar_init(&tbar[1], 1);
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < NCH; q++) {
+            mbar_init(&cfull[q], 1);
+            mbar_init(&cfree[q], 1);
+        }
+        for (int q = 0; q < 3; q++) {
+            mbar_init(&tfull[q], 1);
+            mbar_init(&tfree[q], 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        stop = chunks_issued = trees_issued = 0;
     }
-    __syncwarp();
-
-    // ---- chunk ring: chunk m in slot m % NCH, phase (m / NCH) & 1; chunks hold columns in
-    // descending order of their highest column, never across a tree start
-    int pcol = L - 1, pblk = I.ntrees - 1;
-    TreeRef pc = tree_ref(d, I.block0 + pblk);
-    TreeRef pn = pblk > 0 ? tree_ref(d, I.block0 + pblk - 1) : pc;  // the cursor's next tree
-    int issued = 0, waited = 0, mc = 0;  // chunks issued, complete, oldest in use
-    auto issue = [&]() {
-        if (pcol < 0) return;
-        const int cnt = imin(CW, pcol - pc.start + 1), lo = pcol - cnt + 1;
-        const int slot = issued % NCH;
-        const int Sm = imax(pc.S, 1);
-        __syncwarp();  // the slot's previous chunk is no longer read
-        if (lane == 0) {
-            const Rounded<4> rt(tab.fw + pc.cell0 + (size_t)(lo - pc.start) * Sm, (long long)cnt * Sm);
-            const Rounded<8> ru8(u + lo, cnt);
-            ch_lo[slot] = lo;
-            ch_cnt[slot] = cnt;
-            ch_off[slot] = rt.off;
-            ch_uoff[slot] = ru8.off;
-            ch_S[slot] = Sm;
-            mbar_expect_tx(&cbar[slot], rt.bytes + 4u * MAXT * cnt + ru8.bytes);
-            bulk_g2s(rtab + (size_t)slot * tab_bytes, rt.a16, rt.bytes, &cbar[slot]);
-            bulk_g2s(rbins + slot * CW * MAXT, bins + (size_t)lo * MAXT, 4u * MAXT * cnt, &cbar[slot]);
-            bulk_g2s(ru + slot * (CW + 2), ru8.a16, ru8.bytes, &cbar[slot]);
-        }
-        __syncwarp();
-        issued++;
-        pcol = lo - 1;
-        if (pblk > 0 && pcol < pc.start) {
-            pblk--;
-            pc = pn;
-            if (pblk > 0) pn = tree_ref(d, I.block0 + pblk - 1);
-        }
+    __syncthreads();
+    // a producer's wait for a buffer, given up when the drawing warp has stopped
+    auto wait_free = [&](uint64_t *bar, unsigned parity) -> bool {
+        for (int it = 0; it < WAIT_TRIES && !stop; it++)
+            if (mbar_test(bar, parity)) return true;
+        return false;
     };
-    // chunk index of column c: mc, or mc + 1 when c lies below chunk mc
-    auto chunk_of = [&](int c) { return c >= ch_lo[mc % NCH] ? mc : mc + 1; };
-    auto ensure = [&](int m) -> bool {  // chunks up to m have landed
+    int waited_chunks = 0, waited_trees = 0;  // the drawing warp's
+
+    if (warp == 1) {
+        // ---- chunks: m in slot m % NCH
+        const float *bins = d.bins32 + (size_t)I.col0 * MAXT;
+        int m = 0;
         bool ok = true;
-        while (waited <= m && ok) {
-            ok = mbar_wait(&cbar[waited % NCH], (unsigned)((waited / NCH) & 1));
-            waited++;
-        }
-        return ok;
-    };
-    auto column = [&](int c) -> const float * {
-        const int s = chunk_of(c) % NCH;
-        return (const float *)(rtab + (size_t)s * tab_bytes) + ch_off[s] + (size_t)(c - ch_lo[s]) * ch_S[s];
-    };
-    auto colbins = [&](int c) -> const float * {
-        const int s = chunk_of(c) % NCH;
-        return rbins + (s * CW + (c - ch_lo[s])) * MAXT;
-    };
-    auto uniform = [&](int c) -> double {
-        const int s = chunk_of(c) % NCH;
-        return ru[s * (CW + 2) + ch_uoff[s] + (c - ch_lo[s])];
-    };
-    // columns >= c consumed: release the chunks wholly above c (each landed first, so its
-    // barrier phase is complete before the slot is issued again) and issue new ones
-    auto consumed_to = [&](int c) {
-        while (mc < issued && ch_lo[mc % NCH] >= c) {
-            failed |= !ensure(mc);
-            mc++;
-            issue();
-        }
-    };
-
-    // ---- tree buffers: tree x in buffer x & 1
-    unsigned tphase[2] = {0u, 0u};
-    bool tpend[2] = {false, false};  // staged, not yet waited for
-    __shared__ int o_t2off[2], o_perm[2], o_gptr[2], o_gidx[2], o_dp[2], o_bptr[2];
-    auto stage = [&](const TreeRef &X) {
-        const int b = X.blk & 1;
-        unsigned char *base = tbuf + (size_t)b * TL.total;
-        const int S = X.S, S1 = imax(X.S1, 1);
-        const bool sw = X.start > 0;  // a switch into this tree exists
-        const Rounded<4> rb(d.bt_ptr + (size_t)X.blk * (MAXT + 1), MAXT + 1);
-        const Rounded<4> rt(d.t2off + X.state0, S);
-        const Rounded<4> rp(d.bt_perm + X.state0, S);
-        const Rounded<4> rg(d.gptr + X.gptr0, imax(S, 1) + 1);
-        const Rounded<4> ri(d.gidx + X.prev_state0, S1);
-        const Rounded<4> rq(tab.dprob + X.prev_state0, S1);
-        tpend[b] = true;
-        __syncwarp();
-        if (lane == 0) {
-            o_bptr[b] = rb.off;
-            o_t2off[b] = rt.off;
-            o_perm[b] = rp.off;
-            o_gptr[b] = rg.off;
-            o_gidx[b] = ri.off;
-            o_dp[b] = rq.off;
-            const unsigned tmb = 4u * MAXT * (unsigned)NB;
-            const unsigned tx = (S > 0 ? tmb + 4 * MAXT + rb.bytes + 16u * S + rt.bytes + rp.bytes : 0u) +
-                                (sw ? rg.bytes + ri.bytes + rq.bytes : 0u);
-            mbar_expect_tx(&tbar[b], tx);
-            if (S > 0) {
-                bulk_g2s(base + TL.tm, tab.tm + (size_t)X.blk * MAXT * MAXT, tmb, &tbar[b]);
-                bulk_g2s(base + TL.rstay, tab.rstay + (size_t)X.blk * MAXT, 4 * MAXT, &tbar[b]);
-                bulk_g2s(base + TL.bptr, rb.a16, rb.bytes, &tbar[b]);
-                bulk_g2s(base + TL.sinfo, d.sinfo + X.state0, 16u * S, &tbar[b]);
-                bulk_g2s(base + TL.t2off, rt.a16, rt.bytes, &tbar[b]);
-                bulk_g2s(base + TL.perm, rp.a16, rp.bytes, &tbar[b]);
+        TreeRef t = tree_ref(d, I.block0 + I.ntrees - 1);
+        for (int bi = I.ntrees - 1; bi >= 0 && ok; bi--) {
+            TreeRef next = t;
+            if (bi > 0) next = tree_ref(d, t.blk - 1);
+            for (int hi = t.start + t.len - 1; hi >= t.start; hi -= CC, m++) {
+                const int lo = imax(t.start, hi - CC + 1), slot = m % NCH;
+                if (m >= NCH && !wait_free(&cfree[slot], (unsigned)(((m / NCH) & 1) ^ 1))) {
+                    ok = false;
+                    break;
+                }
+                if (lane == 0) {
+                    // the chunk's part of the table into L2, and the column before it
+                    const size_t Sm = (size_t)imax(t.S, 1), S1 = (size_t)imax(t.S1, 1);
+                    const float *col = tab.fw + t.cell0 + (size_t)(lo - t.start) * Sm;
+                    l2_prefetch(col, sizeof(float) * Sm * (hi - lo + 1));
+                    if (lo == t.start && lo > 0) l2_prefetch(col - S1, sizeof(float) * S1);
+                    unsigned char *at = ring + slot * CHUNK_BYTES;
+                    const int ulo = imax(lo - 1, 0);
+                    const Rounded<8> ru(u + ulo, hi - ulo + 1);
+                    const unsigned bb = 4u * MAXT * (unsigned)(hi - lo + 1);
+                    mbar_expect_tx(&cfull[slot], bb + ru.bytes);
+                    bulk_g2s(at, bins + (size_t)lo * MAXT, bb, &cfull[slot]);
+                    bulk_g2s(at + 4 * CC * MAXT, ru.a16, ru.bytes, &cfull[slot]);
+                }
+                __syncwarp();
             }
-            if (sw) {
-                bulk_g2s(base + TL.gptr, rg.a16, rg.bytes, &tbar[b]);
-                bulk_g2s(base + TL.gidx, ri.a16, ri.bytes, &tbar[b]);
-                bulk_g2s(base + TL.dp, rq.a16, rq.bytes, &tbar[b]);
+            t = next;
+        }
+        if (lane == 0) chunks_issued = m;
+    } else if (warp == 2) {
+        // ---- tree tables: the x-th tree from the last in buffer x % nbuf, an array a lane
+        TreeRef X = tree_ref(d, I.block0 + I.ntrees - 1);
+        int2 src = d.srcs[X.blk];
+        int x = 0, b = 0;
+        unsigned phase = 0;
+        for (; x < I.ntrees; x++) {
+            const bool sw = X.start > 0;  // a switch into this tree exists
+            const int S = X.S, S1 = imax(X.S1, 1);
+            const void *at = nullptr;
+            int words = 0;
+            switch (lane) {
+                case A_TM: at = tab.tm + (size_t)X.blk * MAXT * MAXT; words = MAXT * NB; break;
+                case A_RSTAY: at = tab.rstay + (size_t)X.blk * MAXT; words = MAXT; break;
+                case A_BPTR: at = d.bt_ptr + (size_t)X.blk * (MAXT + 1); words = MAXT + 1; break;
+                case A_SINFO: at = d.sinfo + X.state0; words = 4 * S; break;
+                case A_T2OFF: at = d.t2off + X.state0; words = S; break;
+                case A_PERM: at = d.bt_perm + X.state0; words = S; break;
+                case A_ROWS: at = tab.rows + X.t2_0; words = STAGED ? X.M : 0; break;
+                case A_GPTR: at = d.gptr + X.gptr0; words = imax(S, 1) + 1; break;
+                case A_GIDX: at = d.gidx + X.prev_state0; words = S1; break;
+                case A_DP: at = tab.dprob + X.prev_state0; words = S1; break;
+                case A_RROW: at = tab.rrow + X.state0; words = STAGED ? imax(S, 1) : 0; break;
+                case A_CROW: at = tab.crow + X.state0; words = STAGED ? imax(S, 1) : 0; break;
+            }
+            const bool of_switch = lane >= A_GPTR && lane <= A_CROW;
+            if (of_switch ? !sw : S == 0) words = 0;
+            const Rounded<4> r(at, words);
+            if (x >= nbuf) {
+                if (words > 0) l2_prefetch(r.a16, r.bytes);
+                if (!wait_free(&tfree[b], phase ^ 1)) break;
+            }
+            const unsigned tx = __reduce_add_sync(FULL, r.bytes);
+            if (lane == 0) {
+                trees[b].ref = X;
+                trees[b].src = src;
+            }
+            if (lane < ARRAYS) trees[b].off[lane] = TL.at[lane] + r.off;
+            __syncwarp();
+            if (lane == 0) mbar_expect_tx(&tfull[b], tx);
+            __syncwarp();
+            if (words > 0)
+                bulk_g2s(tbuf + (size_t)b * TL.total + 4 * TL.at[lane], r.a16, r.bytes, &tfull[b]);
+            if (x + 1 < I.ntrees) {
+                X = tree_ref(d, X.blk - 1);
+                src = d.srcs[X.blk];
+            }
+            if (++b == nbuf) {
+                b = 0;
+                phase ^= 1;
             }
         }
-        __syncwarp();
-    };
-    auto wait_tree = [&](int blk) -> bool {
-        const int b = blk & 1;
-        const bool ok = mbar_wait(&tbar[b], tphase[b]);
-        tphase[b] ^= 1u;
-        tpend[b] = false;
-        return ok;
-    };
-
-    for (int q = 0; q < NCH; q++) issue();
-    TreeRef cur = tree_ref(d, I.block0 + I.ntrees - 1);
-    TreeRef nx1 = I.ntrees > 1 ? tree_ref(d, I.block0 + I.ntrees - 2) : cur;
-    stage(cur);
-
-    int state;
-    {
-        const int col = L - 1;
-        failed |= !ensure(chunk_of(col));
-        __syncwarp();
-        const float *c = column(col);
-        const int x = warp_sample<float>(imax(cur.S, 1), uniform(col), [&](int j) { return c[j]; });
-        if (lane == 0) path[col] = x;
-        state = x;
-        __syncwarp();
-        consumed_to(col);
-    }
-    const int g = lane >> 2, sub = lane & 3;  // fast path: column g of a group, quarter sub
-    for (int bi = I.ntrees - 1; bi >= 0 && !failed; bi--) {
-        const TreeRef B = cur;
-        const int b = B.blk & 1;
-        const unsigned char *base = tbuf + (size_t)b * TL.total;
-        failed |= !wait_tree(B.blk);
-        __syncwarp();
-        // tables of the next tree, while this one is sampled
-        TreeRef nx2 = nx1;
-        if (bi > 0) {
-            stage(nx1);
-            if (bi > 1) nx2 = tree_ref(d, I.block0 + bi - 2);
+        if (lane == 0) trees_issued = x;
+    } else {
+        int *path = d.path + I.col0;
+        bool failed = false;
+        int state = 0, m = 0;                     // m: chunks taken
+        const int g = lane >> 2, sub = lane & 3;  // a test's columns g + 8 j, by four lanes
+        {
+            // the last column of all (sample_thread.cpp:534-539)
+            const BlockDev &B = d.blocks[I.block0 + I.ntrees - 1];
+            const float *c = tab.fw + B.cell0 + (size_t)(B.len - 1) * imax(B.S, 1);
+            state = warp_sample<float>(imax(B.S, 1), u[L - 1], [&](int j) { return c[j]; });
+            if (lane == 0) path[L - 1] = state;
         }
-        const float *tmS = (const float *)(base + TL.tm);
-        const float *rst = (const float *)(base + TL.rstay);
-        const int *bptr = (const int *)(base + TL.bptr) + o_bptr[b];
-        const StateInfo *sinfo = (const StateInfo *)(base + TL.sinfo);
-        const int *t2off = (const int *)(base + TL.t2off) + o_t2off[b];
-        const int *perm = (const int *)(base + TL.perm) + o_perm[b];
-        const int S = B.S;
-        int c0 = B.start + B.len - 2;
-        if (S == 0) {
-            // fully specified tree: its single state carries over
-            for (; c0 >= B.start; c0--)
-                if (lane == 0) path[c0] = 0;
-            if (B.len > 1) consumed_to(B.start);
-        } else {
+        int b = 0;
+        unsigned tphase = 0;
+        for (int bi = I.ntrees - 1; bi >= 0 && !failed; bi--) {
+            failed |= !mbar_wait(&tfull[b], tphase);
+            waited_trees++;
+            failed = __any_sync(FULL, failed);
+            if (failed) break;
+            const TreeTables &X = trees[b];
+            const int S = X.ref.S, start = X.ref.start;
+            const float *const fw = tab.fw + X.ref.cell0;  // the tree's table
+            const int *const base = (const int *)(tbuf + (size_t)b * TL.total);
+            auto floats = [&](int a) { return (const float *)base + X.off[a]; };
+            const float *tmS = floats(A_TM), *rst = floats(A_RSTAY);
+            const int *bptr = base + X.off[A_BPTR], *t2off = base + X.off[A_T2OFF], *perm = base + X.off[A_PERM];
+            const StateInfo *sinfo = (const StateInfo *)(base + X.off[A_SINFO]);
+
+            // The drawn state: its node's states, its V and W factors and a lane's share of them.
             int kj1 = 0, km = 0, ys = 0;
-            float t2r[8], tmr[8];
+            float t2r[8];
+            float4 tmr[2];
             auto set_state = [&](int k) {
                 const StateInfo sk = sinfo[k];
                 kj1 = sk.j1;
                 km = sk.m;
                 ys = k - sk.j1;
-                const long long row = B.t2_0 + t2off[k];
+                const int row = t2off[k];
                 const float stay = 1.0f - rst[sk.time];
+                const float *r = STAGED ? floats(A_ROWS) + row : tab.rows + X.ref.t2_0 + row;
                 __syncwarp();
-                t2row[lane] = lane < km ? tab.rows[row + (long long)lane * km] + (lane == ys ? stay : 0.0f) : 0.0f;
+                t2row[lane] = lane < km ? r[(long long)lane * km] + (lane == ys ? stay : 0.0f) : 0.0f;
                 tmcol[lane] = lane < NB ? tmS[lane * MAXT + sk.time] : 0.0f;
                 __syncwarp();
 #pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    t2r[q] = t2row[8 * sub + q];
-                    tmr[q] = tmcol[8 * sub + q];
+                for (int i = 0; i < 8; i++) t2r[i] = t2row[sub + 4 * i];
+#pragma unroll
+                for (int q = 0; q < 2; q++) tmr[q] = ((const float4 *)tmcol)[2 * sub + ((q + g) & 1)];
+            };
+            // The switch into this tree (sample_hmm_posterior_step) from state k: the gather list
+            // merged with the recombination and recoalescence sources, in state order; a lane's
+            // source, its factor and its value of the column before. More than 30: by one lane.
+            int p0 = 0, ng2 = 0, e0 = -1, e1 = -1, src_j = -1;
+            float w0 = 0.0f, w1 = 0.0f, src_w = 0.0f, src_c = 0.0f;
+            const float *const before = fw - imax(X.ref.S1, 1);
+            const int *gi = base + X.off[A_GIDX], *gp = base + X.off[A_GPTR];
+            const float *dp = floats(A_DP);
+            auto sources = [&](int k) {
+                p0 = gp[k];
+                ng2 = gp[k + 1] - p0;
+                const float rr = STAGED ? floats(A_RROW)[k] : tab.rrow[X.ref.state0 + k];
+                const float cr = STAGED ? floats(A_CROW)[k] : tab.crow[X.ref.state0 + k];
+                const int2 src = X.src;
+                // the two extra sources in state order (get(): recoalescence wins a tie)
+                e0 = e1 = -1;
+                w0 = w1 = 0.0f;
+                if (src.x >= 0 && src.x != src.y) { e0 = src.x; w0 = rr; }
+                if (src.y >= 0) {
+                    if (e0 < 0) { e0 = src.y; w0 = cr; }
+                    else if (src.y < e0) { e1 = e0; w1 = w0; e0 = src.y; w0 = cr; }
+                    else { e1 = src.y; w1 = cr; }
+                }
+                src_j = -1;
+                if (ng2 <= 30) {
+                    if (lane < ng2) { src_j = gi[p0 + lane]; src_w = dp[src_j]; }
+                    if (lane == 30 && e0 >= 0) { src_j = e0; src_w = w0; }
+                    if (lane == 31 && e1 >= 0) { src_j = e1; src_w = w1; }
+                    src_c = src_j >= 0 ? before[src_j] : 0.0f;
                 }
             };
-            set_state(state);
-            while (c0 >= B.start && !failed) {
-                const int ng = imin(G, c0 - B.start + 1);
-                const int cg = c0 - imin(g, ng - 1);
-                failed |= !ensure(chunk_of(c0 - ng + 1));
-                __syncwarp();
-                if (failed) break;
-                // fast path: does column g's draw stay at the current state?
-                const float *cp = column(cg);
-                const float *bp = colbins(cg);
-                float sb = 0.0f, ss = 0.0f, sa = 0.0f, sw = 0.0f;
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    const int y = 8 * sub + q;
-                    const float v = y < km ? cp[kj1 + y] * t2r[q] : 0.0f;
-                    sa += v;
-                    sb += y < ys ? v : 0.0f;
-                    ss += y == ys ? v : 0.0f;
-                    sw += y < NB ? bp[y] * tmr[q] : 0.0f;
+            if (S > 0) set_state(state);
+            bool ready = false;  // the switch's sources are loaded
+            int lo = start;
+            const double *uc = nullptr;  // the chunk's uniforms, by column - lo
+            int slot = 0;
+            for (int hi = start + X.ref.len - 1; hi >= start; hi = lo - 1) {
+                lo = imax(start, hi - CC + 1);
+                slot = m % NCH;
+                const unsigned phase = (unsigned)((m / NCH) & 1);
+                m++;
+                if (lo == start && bi > 0) {
+                    sources(state);
+                    ready = true;
                 }
-#pragma unroll
-                for (int o = 1; o < 4; o <<= 1) {
-                    sb += __shfl_xor_sync(FULL, sb, o);
-                    ss += __shfl_xor_sync(FULL, ss, o);
-                    sa += __shfl_xor_sync(FULL, sa, o);
-                    sw += __shfl_xor_sync(FULL, sw, o);
+                // the tree's last column is drawn already
+                int c0 = hi == start + X.ref.len - 1 ? hi - 1 : hi;
+                bool landed = false;
+                const float *bins = (const float *)(ring + slot * CHUNK_BYTES);
+                auto land = [&]() {
+                    if (landed) return;
+                    failed |= !mbar_wait(&cfull[slot], phase);
+                    failed = __any_sync(FULL, failed);
+                    waited_chunks++;
+                    landed = true;
+                    const int ulo = imax(lo - 1, 0);
+                    uc = (const double *)(ring + slot * CHUNK_BYTES + 4 * CC * MAXT) +
+                         ((uintptr_t)(u + ulo) & 15) / 8 + (lo - ulo);
+                };
+                if (S == 0) {
+                    // fully specified tree: its single state carries over
+                    if (lane <= c0 - lo) path[c0 - lane] = 0;
+                    c0 = lo - 1;
                 }
-                const float t = (float)uniform(cg) * (sa + sw);
-                const bool stay = (ys == 0 || sb < t) && t <= sb + ss;
-                const unsigned leave = __ballot_sync(FULL, sub == 0 && g < ng && !stay);
-                const int nstay = leave ? (__ffs(leave) - 1) >> 2 : ng;
-                if (sub == 0 && g < nstay) path[c0 - g] = state;
-                int x = state;
-                if (leave) {
-                    // exact draw of the first column that leaves, by the whole warp
+                while (c0 >= lo) {
+                    const int ng = c0 - lo + 1;
+                    // does a column's draw stay at the current state? The lane's part of V is on
+                    // its way while W is summed; no branches, so that the four columns overlap
+                    // (past the last one they repeat it)
+                    float v[4][8], sb[4], ss[4], sr[4], uf[4];
+                    const float *cp[4];
+                    int col[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        col[j] = c0 - imin(g + 8 * j, ng - 1);
+                        cp[j] = fw + (size_t)(col[j] - start) * S + kj1 + sub;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        if (4 * i >= km) break;
+#pragma unroll
+                        for (int j = 0; j < 4; j++) v[j][i] = sub + 4 * i < km ? cp[j][4 * i] : 0.0f;
+                    }
+                    land();
+                    if (failed) break;
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        uf[j] = (float)uc[col[j] - lo];
+                        const float4 *bp = (const float4 *)(bins + (col[j] - lo) * MAXT);
+                        float w[2];
+#pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            const int y = 4 * (2 * sub + ((q + g) & 1));  // no bank twice
+                            const float4 bv = bp[y >> 2];
+                            w[q] = ((y < NB ? bv.x * tmr[q].x : 0.0f) + (y + 1 < NB ? bv.y * tmr[q].y : 0.0f)) +
+                                   ((y + 2 < NB ? bv.z * tmr[q].z : 0.0f) + (y + 3 < NB ? bv.w * tmr[q].w : 0.0f));
+                        }
+                        sr[j] = w[0] + w[1];
+                        sb[j] = ss[j] = 0.0f;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        if (4 * i >= km) break;
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const float w = v[j][i] * t2r[i];
+                            sb[j] += sub + 4 * i < ys ? w : 0.0f;
+                            ss[j] += sub + 4 * i == ys ? w : 0.0f;
+                            sr[j] += sub + 4 * i > ys ? w : 0.0f;
+                        }
+                    }
+#pragma unroll
+                    for (int o = 1; o < 4; o <<= 1) {
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            sb[j] += __shfl_xor_sync(FULL, sb[j], o);
+                            ss[j] += __shfl_xor_sync(FULL, ss[j], o);
+                            sr[j] += __shfl_xor_sync(FULL, sr[j], o);
+                        }
+                    }
+                    unsigned open = 0;  // a bit per column
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const float t = uf[j] * (sb[j] + ss[j] + sr[j]);
+                        const bool sure = (ys == 0 || sb[j] * (1.0f + margin) < t * (1.0f - margin)) &&
+                                          t * (1.0f + margin) <= (sb[j] + ss[j]) * (1.0f - margin) && t > 1e-30f;
+                        open |= g + 8 * j < ng && !sure ? 1u << (g + 8 * j) : 0u;
+                    }
+                    open = __reduce_or_sync(FULL, open);
+                    int nstay = open ? __ffs(open) - 1 : ng;
+                    bool leaves = false;
                     const int cs = c0 - nstay;
-                    const float *cq = column(cs);
-                    const float *bq = colbins(cs);
-                    const float v = lane < km ? cq[kj1 + lane] * t2row[lane] : 0.0f;
-                    const float w = lane < NB ? bq[lane] * tmcol[lane] : 0.0f;
-                    const float vin = lane_scan(v, lane), win = lane_scan(w, lane);
-                    const float vt = __shfl_sync(FULL, vin, 31), wt = __shfl_sync(FULL, win, 31);
-                    const float tt = (float)uniform(cs) * (vt + wt);
-                    if (tt <= vt) {
-                        const unsigned hit = __ballot_sync(FULL, lane < km && vin >= tt);
-                        x = kj1 + (hit ? __ffs(hit) - 1 : km - 1);
-                    } else {
-                        const float t2 = tt - vt;
-                        const unsigned hit = __ballot_sync(FULL, lane < NB && win >= t2);
-                        const unsigned pos = __ballot_sync(FULL, w > 0.0f);
-                        const int a = hit ? __ffs(hit) - 1 : (pos ? 31 - __clz(pos) : 0);
-                        const float excl = __shfl_sync(FULL, win - w, a);
-                        const float r = (t2 - excl) / tmcol[a];  // threshold on the fw scale
-                        const int p0 = bptr[a], p1 = bptr[a + 1];
-                        float carry = 0.0f;
-                        int res = -1, last = p0;
-                        for (int pb = p0; pb < p1; pb += 32) {
-                            const int pp = pb + lane;
-                            const float f = pp < p1 ? cq[perm[pp]] : 0.0f;
-                            const float fin = lane_scan(f, lane);
-                            const unsigned got = __ballot_sync(FULL, pp < p1 && carry + fin >= r);
-                            const unsigned nz = __ballot_sync(FULL, pp < p1 && f > 0.0f);
-                            if (nz) last = pb + 31 - __clz(nz);
-                            if (got) {
-                                res = pb + __ffs(got) - 1;
-                                break;
-                            }
-                            carry += __shfl_sync(FULL, fin, 31);
+                    const float *cq = fw + (size_t)(cs - start) * S, *bq = bins + (cs - lo) * MAXT;
+                    if (nstay < ng) {
+                        // the same for one column as the draw is defined
+                        float db = 0.0f, ds = 0.0f, da = 0.0f, dw = 0.0f;
+#pragma unroll
+                        for (int q = 0; q < 8; q++) {
+                            const int y = 8 * sub + q;
+                            const float w = y < km ? cq[kj1 + y] * t2row[y] : 0.0f;
+                            da += w;
+                            db += y < ys ? w : 0.0f;
+                            ds += y == ys ? w : 0.0f;
+                            dw += y < NB ? bq[y] * tmcol[y] : 0.0f;
                         }
-                        // past the bin's sum by rounding: its last state of positive weight
-                        x = res >= 0 ? perm[res] : (p1 > p0 ? perm[last] : state);
+#pragma unroll
+                        for (int o = 1; o < 4; o <<= 1) {
+                            db += __shfl_xor_sync(FULL, db, o);
+                            ds += __shfl_xor_sync(FULL, ds, o);
+                            da += __shfl_xor_sync(FULL, da, o);
+                            dw += __shfl_xor_sync(FULL, dw, o);
+                        }
+                        const float t = (float)uc[cs - lo] * (da + dw);
+                        leaves = !((ys == 0 || db < t) && t <= db + ds);
+                        if (!leaves) nstay++;
                     }
-                    if (lane == 0) path[cs] = x;
+                    if (lane < nstay) path[c0 - lane] = state;
+                    int x = state;
+                    if (leaves) {
+                        // exact draw of the first column that leaves, by the whole warp
+                        const float w_v = lane < km ? cq[kj1 + lane] * t2row[lane] : 0.0f;
+                        const float w = lane < NB ? bq[lane] * tmcol[lane] : 0.0f;
+                        const float vin = lane_scan(w_v, lane), win = lane_scan(w, lane);
+                        const float vt = __shfl_sync(FULL, vin, 31), wt = __shfl_sync(FULL, win, 31);
+                        const float tt = (float)uc[cs - lo] * (vt + wt);
+                        if (tt <= vt) {
+                            const unsigned hit = __ballot_sync(FULL, lane < km && vin >= tt);
+                            x = kj1 + (hit ? __ffs(hit) - 1 : km - 1);
+                        } else {
+                            const float t2 = tt - vt;
+                            const unsigned hit = __ballot_sync(FULL, lane < NB && win >= t2);
+                            const unsigned pos = __ballot_sync(FULL, w > 0.0f);
+                            const int a = hit ? __ffs(hit) - 1 : (pos ? 31 - __clz(pos) : 0);
+                            const float excl = __shfl_sync(FULL, win - w, a);
+                            const float rem = (t2 - excl) / tmcol[a];  // threshold on the fw scale
+                            const int q0 = bptr[a], q1 = bptr[a + 1];
+                            float carry = 0.0f;
+                            int res = -1, last = q0;
+                            for (int pb = q0; pb < q1; pb += 32) {
+                                const int pp = pb + lane;
+                                const float f = pp < q1 ? cq[perm[pp]] : 0.0f;
+                                const float fin = lane_scan(f, lane);
+                                const unsigned got = __ballot_sync(FULL, pp < q1 && carry + fin >= rem);
+                                const unsigned nz = __ballot_sync(FULL, pp < q1 && f > 0.0f);
+                                if (nz) last = pb + 31 - __clz(nz);
+                                if (got) {
+                                    res = pb + __ffs(got) - 1;
+                                    break;
+                                }
+                                carry += __shfl_sync(FULL, fin, 31);
+                            }
+                            // past the bin's sum by rounding: its last state of positive weight
+                            x = res >= 0 ? perm[res] : (q1 > q0 ? perm[last] : state);
+                        }
+                        if (lane == 0) path[cs] = x;
+                    }
+                    c0 -= leaves ? nstay + 1 : nstay;
+                    if (x != state) {
+                        state = x;
+                        set_state(state);
+                        ready = false;
+                    }
                 }
-                __syncwarp();
-                const int r = leave ? nstay + 1 : nstay;
-                c0 -= r;
-                consumed_to(c0 + 1);
-                if (x != state) {
-                    state = x;
-                    set_state(state);
+                land();
+                if (failed) break;
+                if (lo > start) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&cfree[slot]);
                 }
             }
-        }
-        if (bi > 0 && !failed) {
-            // switch into this tree (sample_hmm_posterior_step): sources in state order,
-            // the gather list of the drawn state merged with the recombination and
-            // recoalescence sources
-            const int col = B.start - 1;
-            const int k = state;
-            const int2 src = d.srcs[B.blk];
-            const int *gp = (const int *)(base + TL.gptr) + o_gptr[b];
-            const int *gi = (const int *)(base + TL.gidx) + o_gidx[b];
-            const float *dp = (const float *)(base + TL.dp) + o_dp[b];
-            const float rr = tab.rrow[B.state0 + k], cr = tab.crow[B.state0 + k];
-            failed |= !ensure(chunk_of(col));
-            __syncwarp();
-            if (!failed) {
-                const float *c = column(col);
-                const int p0 = gp[k], ng2 = gp[k + 1] - p0;
+            if (failed) break;
+            if (bi > 0) {
+                if (!ready) sources(state);
+                const double ub = uc[-1];
                 int x = 0;
-                if (lane == 0) {
-                    // the two extra sources in state order (get(): recoalescence wins a tie)
-                    int e0 = -1, e1 = -1;
-                    float w0 = 0.0f, w1 = 0.0f;
-                    if (src.x >= 0 && src.x != src.y) { e0 = src.x; w0 = rr; }
-                    if (src.y >= 0) {
-                        if (e0 < 0) { e0 = src.y; w0 = cr; }
-                        else if (src.y < e0) { e1 = e0; w1 = w0; e0 = src.y; w0 = cr; }
-                        else { e1 = src.y; w1 = cr; }
+                if (ng2 <= 30) {
+                    // put in state order; the sums run in that order
+                    int rank = lane + (e0 >= 0 && e0 < src_j) + (e1 >= 0 && e1 < src_j);
+                    const int n0 = __popc(__ballot_sync(FULL, lane < ng2 && src_j <= e0));
+                    const int n1 = __popc(__ballot_sync(FULL, lane < ng2 && src_j <= e1));
+                    if (lane == 30) rank = n0;
+                    if (lane == 31) rank = n1 + 1;
+                    if (src_j >= 0) {
+                        ordw[rank] = src_c * src_w;
+                        ordj[rank] = src_j;
                     }
-                    // merged walk of the gather list and the extras: pass 0 sums, pass 1 draws
-                    float tot = 0.0f, run = 0.0f, pick = 0.0f;
-                    int last = -1;
-                    x = -1;
-                    for (int pass = 0; pass < 2 && x < 0; pass++) {
-                        int p = 0, q = 0;
-                        while ((p < ng2 || q < 2) && x < 0) {
-                            const int eq = q == 0 ? e0 : (q == 1 ? e1 : -1);
-                            if (eq < 0 && q < 2) { q++; continue; }
-                            int j;
-                            float wv;
-                            if (q < 2 && (p >= ng2 || eq < gi[p0 + p])) {
-                                j = eq;
-                                wv = c[j] * (q == 0 ? w0 : w1);
-                                q++;
-                            } else {
-                                j = gi[p0 + p];
-                                wv = c[j] * dp[j];
-                                p++;
-                            }
-                            if (pass == 0) {
-                                tot += wv;
-                            } else {
-                                run += wv;
-                                if (wv > 0.0f) last = j;
-                                if (run >= pick) x = j;
-                            }
+                    __syncwarp();
+                    const int cnt = ng2 + (e0 >= 0) + (e1 >= 0);
+                    const float wv = lane < cnt ? ordw[lane] : 0.0f;
+                    const int j = lane < cnt ? ordj[lane] : -1;
+                    float tot = 0.0f, run = 0.0f;
+                    for (int q = 0; q < cnt; q += 4) {  // (past the last: + 0)
+                        float w[4];
+#pragma unroll
+                        for (int y = 0; y < 4; y++) w[y] = __shfl_sync(FULL, wv, (q + y) & 31);
+#pragma unroll
+                        for (int y = 0; y < 4; y++) {
+                            tot += w[y];
+                            if (lane == q + y) run = tot;
                         }
-                        if (pass == 0) pick = (float)uniform(col) * tot;
                     }
-                    if (x < 0) x = last >= 0 ? last : 0;
+                    const float pick = (float)ub * tot;
+                    const unsigned hit = __ballot_sync(FULL, lane < cnt && run >= pick);
+                    const unsigned pos = __ballot_sync(FULL, lane < cnt && wv > 0.0f);
+                    const int sel = hit ? __ffs(hit) - 1 : pos ? 31 - __clz(pos) : -1;
+                    x = sel >= 0 ? __shfl_sync(FULL, j, sel) : 0;
+                } else {
+                    if (lane == 0) {
+                        // merged walk of the gather list and the extras: pass 0 sums, pass 1 draws
+                        float tot = 0.0f, run = 0.0f, pick = 0.0f;
+                        int last = -1;
+                        x = -1;
+                        for (int pass = 0; pass < 2 && x < 0; pass++) {
+                            int p = 0, q = 0;
+                            while ((p < ng2 || q < 2) && x < 0) {
+                                const int eq = q == 0 ? e0 : (q == 1 ? e1 : -1);
+                                if (eq < 0 && q < 2) { q++; continue; }
+                                int j;
+                                float wv;
+                                if (q < 2 && (p >= ng2 || eq < gi[p0 + p])) {
+                                    j = eq;
+                                    wv = before[j] * (q == 0 ? w0 : w1);
+                                    q++;
+                                } else {
+                                    j = gi[p0 + p];
+                                    wv = before[j] * dp[j];
+                                    p++;
+                                }
+                                if (pass == 0) {
+                                    tot += wv;
+                                } else {
+                                    run += wv;
+                                    if (wv > 0.0f) last = j;
+                                    if (run >= pick) x = j;
+                                }
+                            }
+                            if (pass == 0) pick = (float)ub * tot;
+                        }
+                        if (x < 0) x = last >= 0 ? last : 0;
+                    }
+                    x = __shfl_sync(FULL, x, 0);
                 }
-                x = __shfl_sync(FULL, x, 0);
-                if (lane == 0) path[col] = x;
+                if (lane == 0) path[start - 1] = x;
                 state = x;
-                __syncwarp();
-                consumed_to(col);
+            }
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&cfree[slot]);
+                mbar_arrive(&tfree[b]);
+            }
+            if (++b == nbuf) {
+                b = 0;
+                tphase ^= 1;
             }
         }
-        cur = nx1;
-        nx1 = nx2;
+        if (failed && lane == 0) {
+            stop = 1;
+            report_error(d.err, ERR_WAIT_LIMIT, qi, -1, -1);
+        }
     }
-    if (failed && lane == 0) report_error(d.err, ERR_WAIT_LIMIT, qi, -1, -1);
+    __syncthreads();
     // every copy issued has landed before the CTA's shared memory is released
-    if (lane == 0) {
-        for (int m = waited; m < issued; m++) mbar_wait(&cbar[m % NCH], (unsigned)((m / NCH) & 1));
-        for (int q = 0; q < 2; q++)
-            if (tpend[q]) mbar_wait(&tbar[q], tphase[q]);
+    if (threadIdx.x == 0) {
+        for (int m = waited_chunks; m < chunks_issued; m++) mbar_wait(&cfull[m % NCH], (unsigned)((m / NCH) & 1));
+        for (int m = waited_trees; m < trees_issued; m++) mbar_wait(&tfull[m % nbuf], (unsigned)((m / nbuf) & 1));
     }
-    __syncwarp();
+    __syncthreads();
 }
 
 // ---------------------------------------------------------------------------------------
@@ -996,17 +1130,27 @@ void launch_lots(const BatchDev &d, cudaStream_t s) {
     note_launch();
 }
 
-template <int NCH>
-bool launch_split(const BatchDev &d, cudaStream_t s, size_t budget) {
+template <bool STAGED>
+bool launch_split(const BatchDev &d, cudaStream_t s) {
     const int maxS = imax(d.maxS, 1);
-    const size_t smem = (size_t)NCH * chunk_tab_bytes(maxS) + (size_t)NCH * CW * MAXT * sizeof(float) +
-                        (size_t)NCH * (CW + 2) * sizeof(double) + 2 * (size_t)TreeBufLayout(maxS).total;
-    if (smem > budget) return false;
-    prefer_shared(k_traceback_split<NCH>);
-    if (!raise_dynamic_smem(k_traceback_split<NCH>, smem)) return true;  // the launch reports it
-    k_traceback_split<NCH><<<d.ninst, 32, smem, s>>>(d, maxS);
+    const size_t tree = TreeBufLayout(maxS, STAGED ? imax(d.maxM, 1) : 0).total;
+    const int nbuf = NCH * CHUNK_BYTES + 3 * tree <= 224 * 1024 ? 3 : 2;
+    const size_t smem = NCH * CHUNK_BYTES + nbuf * tree;
+    if (smem > 224 * 1024) return false;
+    prefer_shared(k_traceback_split<STAGED>);
+    if (!raise_dynamic_smem(k_traceback_split<STAGED>, smem)) return true;  // the launch reports it
+    k_traceback_split<STAGED><<<d.ninst, 96, smem, s>>>(d, maxS, nbuf);
     note_launch();
     return true;
+}
+
+// Batches drawn by the decomposed draw. It maps a uniform to another state than the scan does, so
+// this line is part of the results: some 1,290 states, which two tree buffers and three times
+// eight columns in 224 KB came to.
+bool split_draws(const BatchDev &d) {
+    const int maxS = imax(d.maxS, 1);
+    const size_t columns = (4 * 8 * (size_t)maxS + 32 + 15) & ~(size_t)15;
+    return d.bins32 && 3 * (columns + 4 * 8 * MAXT + 8 * (8 + 2)) + 2 * (size_t)TreeBufLayout(maxS, 0).total <= 224 * 1024;
 }
 
 }  // namespace
@@ -1016,10 +1160,7 @@ void launch_traceback(const BatchDev &d, bool fp32, cudaStream_t s) {
         launch_lots<double>(d, s);
         return;
     }
-    // the decomposed draw with the deepest ring that leaves room for two CTAs per SM, else one
-    if (d.bins32 && (launch_split<4>(d, s, 112 * 1024) || launch_split<3>(d, s, 112 * 1024) ||
-                     launch_split<4>(d, s, 224 * 1024) || launch_split<3>(d, s, 224 * 1024)))
-        return;
+    if (split_draws(d) && (launch_split<true>(d, s) || launch_split<false>(d, s))) return;
     launch_lots<float>(d, s);
 }
 
