@@ -427,10 +427,11 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                 mostq[q] = TAIL ? uniform(m[q]) : 0;
                 most = imax(most, m[q]);
             }
-            constexpr int B1 = KPT > 1 ? 1 : 0;  // the second state of a pair, if there is one
+            // pair u: states 2 u and pair2(u), the same one where there is no second
+            auto pair2 = [](int u) { return 2 * u + 1 < KPT ? 2 * u + 1 : 2 * u; };
 #pragma unroll
             for (int u = 0; u < NP; u++) {
-                const int q0 = 2 * u, q1 = 2 * u + B1;
+                const int q0 = 2 * u, q1 = pair2(u);
                 rs[u] = pk(rsv[tq[q0]], rsv[tq[q1]]);
                 iv[u] = pk(inv[ks[q0]], inv[ks[q1]]);
                 xh[u] = xl[u] = pk(0.0f, 0.0f);
@@ -544,8 +545,8 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                 }
 #pragma unroll
                 for (int u = 0; u < NP; u++) {
-                    xh[u] = pk(a[2 * u].hi, a[2 * u + B1].hi);
-                    xl[u] = pk(a[2 * u].lo, a[2 * u + B1].lo);
+                    xh[u] = pk(a[2 * u].hi, a[pair2(u)].hi);
+                    xl[u] = pk(a[2 * u].lo, a[pair2(u)].lo);
                 }
             }
             // the variant rows: the next one to fetch (column EDEPTH + 1 on)
@@ -649,7 +650,7 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                     float least = 0.0f;
 #pragma unroll
                     for (int u = 0; u < NP; u++) {
-                        e[u] = pk(slot_e[ks[2 * u]], slot_e[ks[2 * u + B1]]);
+                        e[u] = pk(slot_e[ks[2 * u]], slot_e[ks[pair2(u)]]);
                         least = fminf(least, fminf(lo(e[u]), hi(e[u])));
                     }
                     ratios = __any_sync(FULL, least < 0.0f);
@@ -666,9 +667,9 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
 #pragma unroll
                 for (int u = 0; u < NP; u++) {
                     // plus the inflow
-                    const float4 t0 = *(const float4 *)tfp[tq[2 * u]], t1 = *(const float4 *)tfp[tq[2 * u + B1]];
+                    const float4 t0 = *(const float4 *)tfp[tq[2 * u]], t1 = *(const float4 *)tfp[tq[pair2(u)]];
                     const V2 tf = pk(((t0.x + t0.y) + t0.z) + t0.w, ((t1.x + t1.y) + t1.z) + t1.w);
-                    x[u] = p2_add(x[u], tf + pk(dot[2 * u], dot[2 * u + B1]));
+                    x[u] = p2_add(x[u], tf + pk(dot[2 * u], dot[pair2(u)]));
                 }
                 const float norm = ((n4.x + n4.y) + n4.z) + n4.w;
                 const float inv_norm = __frcp_rn(norm);
@@ -849,11 +850,12 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
 // a thread; the wide form for batches with larger trees has 20 warps at 96.
 constexpr int OWNERS = 384, WIDE_OWNERS = 512;
 
-// States per owner thread (1, 2, 4 or 8) for an instance's largest tree; at least `least`. One
+// States per owner thread (1, 2, 3, 4 or 8) for an instance's largest tree; at least `least`. One
 // while the owners suffice: a thread's shared loads are issued one after another, so a column
-// takes 0.47 us at 99 states and 0.67 at 351 with one, 0.64 and 0.78 with two.
+// takes 0.47 us at 99 states and 0.67 at 351 with one, 0.64 and 0.78 with two; 1.24 at 789 and
+// 1.30 at 930 with three, 1.48 at 930 with four.
 __host__ __device__ inline int states_per_thread(int maxS, int least, int owners) {
-    const int k = maxS <= owners ? 1 : maxS <= 2 * owners ? 2 : maxS <= 4 * owners ? 4 : 8;
+    const int k = maxS <= owners ? 1 : maxS <= 2 * owners ? 2 : maxS <= 3 * owners ? 3 : maxS <= 4 * owners ? 4 : 8;
     return imax(k, least);
 }
 __host__ __device__ inline int owner_threads(int maxS, int kpt) {
@@ -862,11 +864,15 @@ __host__ __device__ inline int owner_threads(int maxS, int kpt) {
 
 // One CTA per instance, each by its own largest tree: a batch's small instances run as fast as
 // alone. Warps that an instance has no use for leave at once. LONG: more than 21 time points.
-template <bool LONG, bool WIDE>
-__global__ void __launch_bounds__(32 * NRW + (WIDE ? WIDE_OWNERS : OWNERS)) k_forward32(BatchDev d, int maxM, int smem, int least, float nzero) {
+// FEW: batches up to 768 states, without the form of three states a thread (in the same kernel it
+// cost the smaller trees' forms 1.5%, by the registers that all of them are given: 0.91 and 0.90 us
+// a column at 704 states); WIDE: more owner warps at fewer registers each.
+enum Forms { FEW, MANY, WIDE };
+template <bool LONG, Forms FORMS>
+__global__ void __launch_bounds__(32 * NRW + (FORMS == WIDE ? WIDE_OWNERS : OWNERS)) k_forward32(BatchDev d, int maxM, int smem, int least, float nzero) {
     const int qi = cta_instance(d);
     const InstDev I = d.inst[qi];
-    const int kpt = states_per_thread(I.maxS, least, WIDE ? WIDE_OWNERS : OWNERS);
+    const int kpt = states_per_thread(I.maxS, least, FORMS == WIDE ? WIDE_OWNERS : OWNERS);
     const int ntc = 32 * NRW + owner_threads(I.maxS, kpt);
     if ((int)threadIdx.x >= ntc) return;
     const V2 nz = pk(nzero, nzero);
@@ -874,34 +880,43 @@ __global__ void __launch_bounds__(32 * NRW + (WIDE ? WIDE_OWNERS : OWNERS)) k_fo
     // rows longer than the registers hold (a node spans at most T - 1 times): the tables staged
     // a tree ahead with two buffers of rows; where they do not fit, only the rows in shared
     // memory; else neither
-    constexpr int R4 = WIDE ? 4 : 8;
+    constexpr int R4 = FORMS == WIDE ? 4 : 8;
     if (kpt == 1) {
         forward32<1, LONG ? 32 : 20, false, true>(d, I, qi, maxM, 1, ntc, nz);
     } else if (kpt == 2) {
         if (!LONG) forward32<2, 20, false, true>(d, I, qi, maxM, 1, ntc, nz);
         else if (fits(2, true)) forward32<2, 16, true, true>(d, I, qi, maxM, 2, ntc, nz);
         else forward32<4, R4, true, false>(d, I, qi, maxM, fits(1, false), ntc, nz);
+    } else if (FORMS != FEW && kpt == 3) {
+        if (fits(2, true)) forward32<3, 8, true, true>(d, I, qi, maxM, 2, ntc, nz);
+        else forward32<3, 8, true, false>(d, I, qi, maxM, fits(1, false), ntc, nz);
     } else if (kpt == 4) {
-        if (!WIDE && fits(2, true)) forward32<4, R4, true, true>(d, I, qi, maxM, 2, ntc, nz);
+        if (FORMS != WIDE && fits(2, true)) forward32<4, R4, true, true>(d, I, qi, maxM, 2, ntc, nz);
         else forward32<4, R4, true, false>(d, I, qi, maxM, fits(1, false), ntc, nz);
     } else {
         forward32<8, 4, true, false>(d, I, qi, maxM, fits(1, false), ntc, nz);
     }
 }
 
-template <bool LONG, bool WIDE>
+template <bool LONG, Forms FORMS>
 void launch(const BatchDev &d, cudaStream_t s, int least) {
     const int maxS = imax(d.maxS, 1), maxM = imax(d.maxM, 1);
     // shared memory for the most demanding form that fits
     constexpr int LIMIT = 222 * 1024;  // beside the static part
     int smem = SmemPlan(maxS, maxM, d.maxnodes, 2, true).total;
     if (smem > LIMIT) smem = LIMIT;
-    if (!raise_dynamic_smem(k_forward32<LONG, WIDE>, smem)) return;  // the launch reports it
+    if (!raise_dynamic_smem(k_forward32<LONG, FORMS>, smem)) return;  // the launch reports it
     // an instance with one state a thread may need every warp
-    const int owners = WIDE ? WIDE_OWNERS : OWNERS;
+    const int owners = FORMS == WIDE ? WIDE_OWNERS : OWNERS;
     const int nt = 32 * NRW + (maxS <= owners && least <= 1 ? owner_threads(maxS, 1) : owners);
-    k_forward32<LONG, WIDE><<<d.ninst, nt, smem, s>>>(d, maxM, smem, least, -0.0f);
+    k_forward32<LONG, FORMS><<<d.ninst, nt, smem, s>>>(d, maxM, smem, least, -0.0f);
     note_launch();
+}
+
+template <Forms FORMS>
+void launch(const BatchDev &d, cudaStream_t s, int least) {
+    if (d.maxT <= 21) launch<false, FORMS>(d, s, least);
+    else launch<true, FORMS>(d, s, least);
 }
 
 }  // namespace
@@ -916,8 +931,9 @@ bool launch_forward32(const BatchDev &d, cudaStream_t s, int want_kpt) {
     }();
     auto known = [](int k) { return k == 1 || k == 2 || k == 4 || k == 8; };
     const int least = known(want_kpt) ? want_kpt : known(env) ? env : 1;
-    if (d.maxS <= 4 * OWNERS) d.maxT <= 21 ? launch<false, false>(d, s, least) : launch<true, false>(d, s, least);
-    else d.maxT <= 21 ? launch<false, true>(d, s, least) : launch<true, true>(d, s, least);
+    if (d.maxS <= 2 * OWNERS) launch<FEW>(d, s, least);
+    else if (d.maxS <= 4 * OWNERS) launch<MANY>(d, s, least);
+    else launch<WIDE>(d, s, least);
     return true;
 }
 
