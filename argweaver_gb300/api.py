@@ -78,7 +78,8 @@ def run_batch(problems: Sequence[Problem], *, precision: str = "fp64",
     outs = (capi.AwgOutputs * n)()
     results, keep = [], []
     ncells = np.zeros(n, dtype=np.int64)
-    if lib.awg_problems_cells(probs, n, ncells.ctypes.data) != 0:
+    # (the run checks the problems too: a table's size is what is needed here)
+    if (want_forward or want_posterior) and lib.awg_problems_cells(probs, n, ncells.ctypes.data) != 0:
         raise ValueError(capi.last_error())
     for q, b in enumerate(bound):
         r = Result()
@@ -108,7 +109,10 @@ def run_batch(problems: Sequence[Problem], *, precision: str = "fp64",
         results.append((r, ll))
     rc = lib.awg_run_batch(probs, outs, n, capi.AWG_FP32 if fp32 else capi.AWG_FP64)
     if rc != 0:
-        raise GpuError(f"awg_run_batch failed ({rc}): {capi.last_error()}")
+        failure = GpuError(f"awg_run_batch failed ({rc}): {capi.last_error()}")
+        if lib.awg_problems_cells(probs, n, ncells.ctypes.data) != 0:
+            raise ValueError(capi.last_error())
+        raise failure
     out = []
     for r, ll in results:
         r.loglik = float(ll[0])

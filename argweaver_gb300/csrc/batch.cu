@@ -269,7 +269,7 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         h = dry_stage.data();
         if (!plan_fill(probs, n, plan, PlanDst{(int *)(h + o_nodes), (int *)(h + o_map),
                                                (uint8_t *)(h + o_seq), (uint8_t *)(h + o_cls),
-                                               (int *)(h + o_cvar)},
+                                               (int *)(h + o_cvar), nullptr},
                        &err))
             return -1;
     } else {
@@ -285,14 +285,16 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         // ---------------- stage inputs
         h = C.host;
         // per-node, per-column and sequence arrays straight into the staging buffer
+        std::vector<const double *> uniforms(n);
+        for (int q = 0; q < n && want_path; q++) uniforms[q] = outs[q].uniforms;
         if (!plan_fill(probs, n, plan, PlanDst{(int *)(h + o_nodes), (int *)(h + o_map),
                                                (uint8_t *)(h + o_seq), (uint8_t *)(h + o_cls),
-                                               (int *)(h + o_cvar)},
-                       &err))
+                                               (int *)(h + o_cvar), (double *)(h + o_u)},
+                       &err, want_path ? uniforms.data() : nullptr))
             return -1;
-        memcpy(h + o_inst, plan.inst.data(), sizeof(InstDev) * plan.ninst);
-        memcpy(h + o_blocks, plan.blocks.data(), sizeof(BlockDev) * plan.nblocks);
-        memcpy(h + o_model, plan.model.data(), sizeof(double) * plan.model.size());
+        parallel_copy({{h + o_inst, plan.inst.data(), sizeof(InstDev) * plan.ninst},
+                       {h + o_blocks, plan.blocks.data(), sizeof(BlockDev) * plan.nblocks},
+                       {h + o_model, plan.model.data(), sizeof(double) * plan.model.size()}});
     }
 
     Layout w;  // work region follows the inputs
@@ -386,12 +388,9 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         double *u = (double *)(h + o_u);
         for (int q = 0; q < n; q++) {
             const InstDev &I = plan.inst[q];
-            if (outs[q].uniforms) {
-                memcpy(u + I.col0, outs[q].uniforms, sizeof(double) * I.seqlen);
-            } else {
-                // the reference's draws: rand()/RAND_MAX, last column first (common.h:103-110)
-                for (int c = I.seqlen - 1; c >= 0; c--) u[I.col0 + c] = rand() / double(RAND_MAX);
-            }
+            if (outs[q].uniforms) continue;  // copied with the columns
+            // the reference's draws: rand()/RAND_MAX, last column first (common.h:103-110)
+            for (int c = I.seqlen - 1; c >= 0; c--) u[I.col0 + c] = rand() / double(RAND_MAX);
         }
     }
 
@@ -709,6 +708,10 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         size_t bytes;
     };
     std::vector<Pending> pend;
+    // several problems' paths and log-likelihoods lie side by side on the device: two copies to
+    // page-locked staging, handed over by ctx_complete (a copy to pageable memory each took 20 ms
+    // for 256 problems of 58,000 columns). A path of 256 MB and more goes as it is.
+    const bool packed = !async && n > 1 && sizeof(int) * COLS <= ((size_t)256 << 20);
     for (int q = 0; q < n; q++) {
         const InstDev &I = plan.inst[q];
         const long long cells = (q + 1 < n ? plan.inst[q + 1].cell0 : plan.total_cells) - I.cell0;
@@ -718,11 +721,22 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         if (o.posterior) pend.push_back({o.posterior, d.post + I.cell0, sizeof(double) * cells});
         if (opt.backward && opt.backward[q])
             pend.push_back({opt.backward[q], (double *)(D + o_bw) + I.cell0, sizeof(double) * cells});
+        if (packed) continue;
         if (o.path) pend.push_back({o.path, d.path + I.col0, sizeof(int) * I.seqlen});
         if (o.loglik) pend.push_back({o.loglik, d.lnl + q, sizeof(double)});
     }
     if (async) {
         for (const Pending &pd : pend) C.copies.push_back({pd.dst, out_slot(pd.bytes), pd.bytes});
+    }
+    size_t lnl_at = 0, path_at = 0;
+    if (packed) {
+        lnl_at = out_slot(sizeof(double) * n);
+        path_at = out_slot(want_path ? sizeof(int) * COLS : 0);
+        for (int q = 0; q < n; q++) {
+            const InstDev &I = plan.inst[q];
+            if (outs[q].loglik) C.copies.push_back({outs[q].loglik, lnl_at + sizeof(double) * q, sizeof(double)});
+            if (outs[q].path) C.copies.push_back({outs[q].path, path_at + sizeof(int) * I.col0, sizeof(int) * I.seqlen});
+        }
     }
     C.err_off = out_slot(4 * sizeof(int));
     if (hout_bytes > C.hout_cap) {
@@ -736,6 +750,11 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
     for (size_t i = 0; i < pend.size(); i++)
         CK(cudaMemcpyAsync(async ? (void *)(C.hout + C.copies[i].off) : pend[i].dst, pend[i].src,
                            pend[i].bytes, cudaMemcpyDeviceToHost, s));
+    if (packed) {
+        CK(cudaMemcpyAsync(C.hout + lnl_at, d.lnl, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+        if (want_path)
+            CK(cudaMemcpyAsync(C.hout + path_at, d.path, sizeof(int) * COLS, cudaMemcpyDeviceToHost, s));
+    }
     CK(cudaMemcpyAsync(C.hout + C.err_off, d.err, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
     if (T) CK(cudaEventRecord(C.ev[7], s));
     CK(cudaEventRecord(C.done, s));
@@ -777,7 +796,9 @@ int ctx_complete(Ctx &C, std::string &err) {
         C.copies.clear();
         return -4;
     }
-    for (const Ctx::Copy &c : C.copies) memcpy(c.dst, C.hout + c.off, c.bytes);
+    std::vector<HostCopy> copies;
+    for (const Ctx::Copy &c : C.copies) copies.push_back({c.dst, C.hout + c.off, c.bytes});
+    parallel_copy(copies);
     C.copies.clear();
     return 0;
 }

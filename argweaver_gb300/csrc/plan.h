@@ -1,6 +1,7 @@
 // Host-side plan of a batch: validated inputs packed into the flat arrays the kernels read.
 #pragma once
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -37,6 +38,7 @@ struct PlanDst {
     uint8_t *seqT;       // [total_seq]
     uint8_t *colclass;   // [total_cols]
     int *colvar;         // [total_cols]
+    double *u;           // [total_cols] or NULL: the traceback's uniforms
 };
 
 // Passes 1-2: validates the problems (sequence bytes too when check_seqs; plan_fill checks
@@ -46,8 +48,9 @@ bool plan_layout(const awg_problem *probs, int n, HostPlan &plan, std::string &e
                  bool check_seqs);
 // Pass 3: fills the arrays into dst, the trees' roots and the variant-emission offsets,
 // and checks every sequence byte (A, C, G, T or N); false with *err set on a bad byte.
+// uniforms (or NULL): per problem its uniforms, or NULL, copied to dst.u.
 bool plan_fill(const awg_problem *probs, int n, HostPlan &plan, const PlanDst &dst,
-               std::string *err);
+               std::string *err, const double *const *uniforms = nullptr);
 // Both, into the plan's own vectors; returns false with a message on bad input.
 bool build_plan(const awg_problem *probs, int n, HostPlan &plan, std::string &err);
 
@@ -58,6 +61,14 @@ void model_arrays(const double *times, const double *popsizes, int T, double rho
 // Threads the calling thread's planning may use (0: all hardware threads); callers that
 // plan several batches at once share the cores this way.
 void set_plan_threads(int n);
+// Runs f(k) for k < n on as many threads as `ns` nanoseconds of work are worth.
+void parallel_tasks(int n, double ns, const std::function<void(int)> &f);
+struct HostCopy {
+    void *dst;
+    const void *src;
+    size_t bytes;
+};
+void parallel_copy(const std::vector<HostCopy> &copies);
 
 // Number of states of a local tree given by parent/age arrays (states.cpp:53-199).
 int count_states(const int *parent, const int *age, int n, int T, bool internal, int minage,
