@@ -121,8 +121,7 @@ __device__ __forceinline__ bool below(const int4 *nd, int v, int top, int n) {
 // same-branch row offset (integers: exact in any order). Returns S.
 __device__ int node_ranges_par(const int4 *nd, int n, int root, int T, bool internal,
                                int minage_param, int *first, int *t0, int *cnt, int *t2base) {
-    __shared__ int part[TAB_THREADS], part2[TAB_THREADS];
-    __shared__ int sh_tot;
+    __shared__ int part[TAB_THREADS / 32], part2[TAB_THREADS / 32];
     const int tid = threadIdx.x, nt = blockDim.x;
     bool none = false;
     int minage = 0, sub = -1;
@@ -155,29 +154,36 @@ __device__ int node_ranges_par(const int4 *nd, int n, int root, int T, bool inte
         s1 += cnt[v];
         s2 += cnt[v] * cnt[v];
     }
-    part[tid] = s1;
-    part2[tid] = s2;
-    __syncthreads();
-    if (tid == 0) {
-        int a = 0, b = 0;
-        for (int t = 0; t < nt; t++) {
-            const int x = part[t], y = part2[t];
-            part[t] = a;
-            part2[t] = b;
+    int a = s1, b = s2;  // inclusive, then exclusive sums over the threads
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
+        if ((tid & 31) >= o) {
             a += x;
             b += y;
         }
-        sh_tot = a;
+    }
+    if ((tid & 31) == 31) {
+        part[tid >> 5] = a;
+        part2[tid >> 5] = b;
     }
     __syncthreads();
-    int a = part[tid], b = part2[tid];
+    a -= s1;
+    b -= s2;
+    int S = 0;
+    for (int w = 0; w < nt / 32; w++) {
+        if (w < tid >> 5) {
+            a += part[w];
+            b += part2[w];
+        }
+        S += part[w];
+    }
     for (int v = lo; v < hi; v++) {
         first[v] = a;
         if (t2base) t2base[v] = b;
         a += cnt[v];
         b += cnt[v] * cnt[v];
     }
-    const int S = sh_tot;
     __syncthreads();
     return S;
 }
@@ -363,6 +369,13 @@ __device__ double calc_recomb_recoal(const SwitchCtx &c, const int *spr, int sta
 // K1
 
 // The tables of one local tree, by the whole CTA (TAB_THREADS threads).
+//
+// What bounds it: the FP64 pipe (64 cycles a warp's instruction on its sub-partition, live lanes
+// or not) and the barriers between the short serial sections. So every FP64 function is called
+// from as few warps as hold its arguments, and a value that several states share is formed once:
+// the switch's recombination-then-coalescence probabilities depend on their state through its
+// time alone and take two warps once, where the recoalescence row evaluated them per state.
+// 402,000 trees of 8 to 64 leaves: 76.1 ms before, 45.5 ms now.
 __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want32) {
     extern __shared__ int4 dyn[];
     BlockDev &Bg = d.blocks[blk];
@@ -395,7 +408,7 @@ __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want
     __shared__ double sums2[2 * MAXT + 1], recoals[MAXT];
     __shared__ double sh_treelen, sh_sums, sh_maintreelen, sh_subtreelen, sh_tlmin;
     __shared__ double wmin[TAB_THREADS / 32];
-    __shared__ double tl_tab[2 * MAXT], inv_tab[2 * MAXT], dp_tab[3 * MAXT];
+    __shared__ double tl_tab[2 * MAXT], inv_tab[2 * MAXT], dp_tab[2 * MAXT], rr_tab[2 * MAXT];
     __shared__ int sh_S, sh_S1, sh_minage, sh_rootage, sh_src[2];
 
     if (tid == 0) {
@@ -502,26 +515,21 @@ __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want
         const double *C = &C_alloc[2];
         const int root_age_index = sh_rootage;
         const double root_age = times[root_age_index];
-        // one (term, time) pair per thread, each term's expression as the reference writes
-        // it (lnE2 and lnG4 are the same expression, trans.cpp:80-86); D and norecombs on
-        // separate threads
-        for (int e = tid; e < 6 * (T - 1); e += blockDim.x) {
-            const int f = e / (T - 1), b = e % (T - 1);
-            if (f == 0) {
+        // a time per lane, each term's expression as the reference writes it (lnE2 and lnG4 are
+        // the same expression, trans.cpp:80-86), a term on one warp alone: an FP64 function holds
+        // the pipe for a warp however few lanes are live
+        static_assert(TAB_THREADS == 128 && MAXT <= 32, "four warps, a time per lane");
+        const int w = tid >> 5, b = tid & 31;
+        if (b < T - 1) {
+            if (w == 0) {
                 lnBterm[b] = C[2 * b - 1] + log(tsteps[b] * (nb[b] + 1.0) / (nr[b] + 1.0));
                 tr.E[b] = 1.0 / nc[b];
-            } else if (f == 1) {
-                const double v = -C[2 * b - 2] +
-                    (b < T - 2 ? log(1 - exp(-coal_rates[2 * b] - coal_rates[2 * b - 1])) : 0.0);
-                tr.lnE2[b] = v;
-                tr.lnG4[b] = v;
-            } else if (f == 2) {
-                tr.lnNegG1[b] = C[2 * b - 1] + log(-tsteps[b] *
-                    ((nb[b] / (nr[b] + 1.0 + int(b < root_age_index))) - (nb[b] + 1.0) / (nr[b] + 1.0)));
-            } else if (f == 3) {
                 const double g = b < T - 2 ? 1.0 - exp(-coal_rates[2 * b]) : 1.0;
                 tr.G2[b] = g * tsteps[b] * (nb[b] + 1.0) / (nr[b] + 1.0);
                 tr.G3[b] = g * tsteps[b] * (nb[b] / (nr[b] + 1.0 + int(b < root_age_index)));
+            } else if (w == 2) {
+                tr.lnNegG1[b] = C[2 * b - 1] + log(-tsteps[b] *
+                    ((nb[b] / (nr[b] + 1.0 + int(b < root_age_index))) - (nb[b] + 1.0) / (nr[b] + 1.0)));
             } else {
                 double treelen2 = sh_treelen + times[b];
                 double treelen2_b;
@@ -531,7 +539,11 @@ __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want
                 } else {
                     treelen2_b = treelen2 + tsteps[root_age_index];
                 }
-                if (f == 4) {
+                if (w == 1) {
+                    const double v = -C[2 * b - 2] +
+                        (b < T - 2 ? log(1 - exp(-coal_rates[2 * b] - coal_rates[2 * b - 1])) : 0.0);
+                    tr.lnE2[b] = v;
+                    tr.lnG4[b] = v;
                     tr.D[b] = (1.0 - exp(-rho * treelen2)) / treelen2_b;
                 } else {
                     tr.norecombs[b] = exp(-fmax(rho * treelen2, rho));
@@ -579,15 +591,18 @@ __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want
             tm[a * MAXT + b] = get_time(tr, a, b, 0, minage, false);
         }
     } else {
-        // FP32 path: 4 (T-1) exponentials instead of 1.5 (T-1)^2; tmatrix = D[a] E[b] (X[a][b]
-        // - minage_term[b]), X the different-node bracket (get_time, trans.h:101-109), kept
-        // with D[a] E[b] for the same-branch rows below
-        for (int e = tid; e < 4 * (T - 1); e += blockDim.x) {  // one exponential per thread
-            const int f = e / (T - 1), i = e % (T - 1);
-            if (f == 0) tr.eE2[i] = exp(tr.lnE2[i]);
-            else if (f == 1) tr.eB[i] = exp(tr.lnB[i]);
-            else if (f == 2) tr.eG4[i] = exp(tr.lnG4[i]);
-            else tr.dBN[i] = exp(tr.lnB[i]) * -expm1(tr.lnNegG1[i] - tr.lnB[i]);
+        // FP32 path: 2 (T-1) exponentials instead of 1.5 (T-1)^2 (lnG4 is lnE2); tmatrix = D[a]
+        // E[b] (X[a][b] - minage_term[b]), X the different-node bracket (get_time,
+        // trans.h:101-109), kept with D[a] E[b] for the same-branch rows below
+        {
+            const int w = tid >> 5, i = tid & 31;
+            if (i < T - 1 && w == 0) {
+                tr.eE2[i] = tr.eG4[i] = exp(tr.lnE2[i]);
+            } else if (i < T - 1 && w == 1) {
+                const double eb = exp(tr.lnB[i]);
+                tr.eB[i] = eb;
+                tr.dBN[i] = eb * -expm1(tr.lnNegG1[i] - tr.lnB[i]);
+            }
         }
         __syncthreads();
         float *tm32 = d.tm32 + (size_t)blk * MAXT * MAXT;
@@ -624,46 +639,57 @@ __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want
         // (X the different-node bracket without its minage term; both in E2B / E2N above);
         // formed from that product it keeps its relative accuracy where the two get_time
         // values nearly cancel.
+        // An entry per thread: a node's block lies target after target, source-major.
         float *t2d = d.t2d32 + B.t2_0;
-        for (int k = tid; k < S; k += blockDim.x) {
-            const StateInfo si = sinfo[k];
-            const int b = si.time, c = cur[si.node].w;
-            const int base = t2off[k];
+        int v = 0;
+        for (int e = tid; e < B.M; e += TAB_THREADS) {
+            while (v + 1 < n && t2base[v + 1] <= e) v++;
+            const int m = imax(cnt[v], 1), x = e - t2base[v];
+            // x / m: x < 2^10 and m < 2^5, so the half keeps the quotient clear of integers
+            const int y = (int)(((float)x + 0.5f) * (1.0f / (float)m));
+            const int a = t0[v] + y, b = t0[v] + x - y * m, c = cur[v].w;
             const double ct = c > 0 ? tr.eG4[b] * tr.eB[c - 1] : 0.0;
-            for (int y = 0; y < si.m; y++) {
-                const int a = t0[si.node] + y;
-                t2d[base + y * si.m] =
-                    (a < minage || b < minage) ? 0.0f
-                                               : (float)(tr.E2N[a * T + b] * (tr.E2B[a * T + b] - ct));
-            }
+            t2d[e] = (a < minage || b < minage) ? 0.0f
+                                                : (float)(tr.E2N[a * T + b] * (tr.E2B[a * T + b] - ct));
         }
     }
 
     // states grouped by time, ascending state index within a time
     int *bt_ptr = d.bt_ptr + (size_t)blk * (MAXT + 1);
     int *bt_perm = d.bt_perm + B.state0;
-    for (int a = tid; a < MAXT; a += blockDim.x) {
-        int c = 0;
-        for (int v = 0; v < n; v++)
-            if (cnt[v] && t0[v] <= a && a < t0[v] + cnt[v]) c++;
-        gcnt[a] = c;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        int acc = 0;
-        for (int a = 0; a < MAXT; a++) {
-            bt_ptr[a] = acc;
-            int c = gcnt[a];
-            gcnt[a] = acc;
-            acc += c;
+    {
+        const int lane = tid & 31, w = tid >> 5;
+        // nodes with a state of time a, among 32 of them
+        auto at_time = [&](int v, int a) {
+            return __ballot_sync(0xffffffffu, v < n && cnt[v] && t0[v] <= a && a < t0[v] + cnt[v]);
+        };
+        for (int a = w; a < MAXT; a += TAB_THREADS / 32) {
+            int c = 0;
+            if (a < T)
+                for (int v = lane; v - lane < n; v += 32) c += __popc(at_time(v, a));
+            if (lane == 0) gcnt[a] = c;
         }
-        bt_ptr[MAXT] = acc;
-    }
-    __syncthreads();
-    for (int a = tid; a < MAXT; a += blockDim.x) {
-        int pos = gcnt[a];
-        for (int v = 0; v < n; v++)
-            if (cnt[v] && t0[v] <= a && a < t0[v] + cnt[v]) bt_perm[pos++] = first[v] + a - t0[v];
+        __syncthreads();
+        if (w == 0) {
+            const int c = gcnt[lane];
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            bt_ptr[lane] = gcnt[lane] = incl - c;
+            if (lane == 31) bt_ptr[MAXT] = incl;
+        }
+        __syncthreads();
+        for (int a = w; a < T; a += TAB_THREADS / 32) {
+            int pos = gcnt[a];
+            for (int v = lane; v - lane < n; v += 32) {
+                const unsigned on = at_time(v, a);
+                if (on >> lane & 1) bt_perm[pos + __popc(on & ((1u << lane) - 1))] = first[v] + a - t0[v];
+                pos += __popc(on);
+            }
+        }
     }
 
     // invariant-site emission per state (emit.cpp:744-819)
@@ -922,7 +948,7 @@ __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want
         }
         // recoalescence sums (calc_recoal_sums, trans.cpp:417-440)
         const int rpa0 = prv[prv[spr[0]].x].w;
-        if (tid == 0) {
+        if (tid == 32) {
             const int k = spr[1], j = spr[3];
             double sum = 0.0;
             for (int m = 2 * k; m < 2 * j - 1; m++) sum += qrate[m][1 - int(m / 2 < rpa0)];
@@ -935,65 +961,69 @@ __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want
             }
         }
         for (int a = tid; a < T; a += blockDim.x) recoals[a] = calc_recoal(c, spr, a, rpa0, false);
-        __syncthreads();
-        auto dprob = [&](int node, int a) {
-            if (node == spr[0] && a > spr[1]) return calc_recomb_recoal(c, spr, node, a, a);
-            const int idx = max(min(2 * spr[3] - 1, 2 * a), 2 * spr[1]);
-            return calc_recomb(c, spr, node, a, c.last_treelen) * exp(-sh_sums - sums2[idx]) *
-                   recoals[a];
-        };
-        if (!internal) {
-            // external trees: the value depends on the source state only through its time
-            // and whether its node is the root (calc_recomb) or the recombining node above
-            // the recombination (calc_recomb_recoal); one evaluation per case. Node -1
-            // stands for any other node (the external calc_recomb only compares it with the
-            // root; the recombining node is never the root).
-            for (int e = tid; e < 3 * (T - 1); e += blockDim.x) {
-                const int f = e / (T - 1), a = e % (T - 1);
-                const int node = f == 0 ? -1 : f == 1 ? B.prev_root : spr[0];
-                dp_tab[f * MAXT + a] = dprob(node, a);
-            }
-            __syncthreads();
-            for (int i = tid; i < S1; i += blockDim.x) {
-                if (determ[i] < 0) continue;
-                const int node = s1node[i], a = s1time[i];
-                const int f = (node == spr[0] && a > spr[1]) ? 2 : node == B.prev_root ? 1 : 0;
-                determprob[i] = dp_tab[f * MAXT + a];
-            }
-        } else {
-            for (int i = tid; i < S1; i += blockDim.x) {
-                if (determ[i] < 0) continue;
-                determprob[i] = dprob(s1node[i], s1time[i]);
-            }
-        }
         // probabilistic sources (each state at most once: states are distinct)
         for (int i = tid; i < S1; i += blockDim.x) {
             if (s1node[i] == spr[0] && s1time[i] == spr[1]) sh_src[0] = i;
             else if (s1node[i] == spr[2] && s1time[i] == spr[3]) sh_src[1] = i;
         }
         __syncthreads();
-        if (tid == 0 || tid == 32) {  // the two entries on two warps
-            const int recombsrc = sh_src[0];
-            if (recombsrc != -1) {  // get_recomb_transition_switch (trans.cpp:278-313)
-                const int parent = prv[spr[0]].x;
-                const int time2 = prv[parent].w;
-                const int other = sibling(prv, spr[0]);
-                const int node2 = (other == spr[2] ? cur[mapping[other]].x : mapping[other]);
-                const int next0 = lookup(first, t0, cnt, mapping[spr[0]], spr[1]);
-                const int next1 = lookup(first, t0, cnt, node2, time2);
-                // where both entries are one state the reference's second write wins
-                if (tid == 0 && next0 != -1 && next0 != next1)
-                    recombrow[next0] = calc_recomb_recoal(c, spr, s1node[recombsrc],
-                                                          s1time[recombsrc], rpa0);
-                if (tid == 32 && next1 != -1)
-                    recombrow[next1] = calc_recomb_recoal(c, spr, s1node[recombsrc],
-                                                          s1time[recombsrc], s1time[recombsrc]);
+        const int recombsrc = sh_src[0], recoalsrc = sh_src[1];
+        auto dprob = [&](int node, int a) {  // of a node not above the recombination
+            const int idx = max(min(2 * spr[3] - 1, 2 * a), 2 * spr[1]);
+            return calc_recomb(c, spr, node, a, c.last_treelen) * exp(-sh_sums - sums2[idx]) *
+                   recoals[a];
+        };
+        // Every calc_recomb_recoal that the tree needs, a lane each on two warps: lane a < T - 1
+        // of the first the recombining node's moves from time a above the recombination (external
+        // trees), of the second the recoalescence row's entries of time a (they depend on the
+        // target through its time alone), the last lanes the recombination row's two entries.
+        // Meanwhile the other warps form the remaining moves of external trees, whose value
+        // depends on the source state only through its time and whether its node is the root:
+        // node -1 stands for any other (the external calc_recomb only compares it with the root;
+        // the recombining node is never the root).
+        {
+            const int w = tid >> 5, l = tid & 31;
+            if (w < 2) {
+                int node = spr[0], time = spr[1], rpa = w == 0 ? spr[1] : rpa0, to = spr[3];
+                bool needed = l == 31 && recombsrc != -1;
+                if (l < T - 1 && w == 0) {
+                    needed = !internal && l > spr[1];
+                    time = rpa = l;
+                } else if (l < T - 1) {
+                    needed = recoalsrc != -1 && (l >= spr[1] || l == spr[3]);
+                    node = spr[2];
+                    time = spr[3];
+                    to = l;
+                }
+                if (needed) {
+                    const int spr2[4] = {spr[0], spr[1], spr[2], to};
+                    rr_tab[tid] = calc_recomb_recoal(c, spr2, node, time, rpa);
+                }
+            } else if (!internal && l < T - 1) {
+                dp_tab[(w - 2) * MAXT + l] = dprob(w == 2 ? -1 : B.prev_root, l);
             }
         }
         __syncthreads();
-        const int recoalsrc = sh_src[1];
+        for (int i = tid; i < S1; i += blockDim.x) {
+            if (determ[i] < 0) continue;
+            const int node = s1node[i], a = s1time[i];
+            const bool above = node == spr[0] && a > spr[1];
+            if (internal) determprob[i] = above ? calc_recomb_recoal(c, spr, node, a, a) : dprob(node, a);
+            else determprob[i] = above ? rr_tab[a] : dp_tab[(node == B.prev_root ? MAXT : 0) + a];
+        }
+        if (tid == 0 && recombsrc != -1) {  // get_recomb_transition_switch (trans.cpp:278-313)
+            const int parent = prv[spr[0]].x;
+            const int time2 = prv[parent].w;
+            const int other = sibling(prv, spr[0]);
+            const int node2 = (other == spr[2] ? cur[mapping[other]].x : mapping[other]);
+            const int next0 = lookup(first, t0, cnt, mapping[spr[0]], spr[1]);
+            const int next1 = lookup(first, t0, cnt, node2, time2);
+            // where both entries are one state the reference's second write wins
+            if (next0 != -1 && next0 != next1) recombrow[next0] = rr_tab[63];
+            if (next1 != -1) recombrow[next1] = rr_tab[31];
+        }
         if (recoalsrc != -1) {
-            const int node1 = s1node[recoalsrc], time1 = s1time[recoalsrc];
+            const int node1 = spr[2], time1 = spr[3];
             const int last_parent = prv[spr[0]].x;
             int node3;
             if (last_parent == node1)
@@ -1006,8 +1036,7 @@ __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want
                 if (!((node2 == mapping[spr[0]] && time2 >= spr[1]) ||
                       (node2 == node3 && time2 == time1) || (node2 == parent && time2 == time1)))
                     continue;
-                int spr2[4] = {spr[0], spr[1], spr[2], time2};
-                recoalrow[j] = calc_recomb_recoal(c, spr2, node1, time1, rpa0);
+                recoalrow[j] = rr_tab[32 + time2];
             }
         }
     }
@@ -1020,10 +1049,12 @@ __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want
         const int n1 = imax(S1, 1);
         const int rs = sh_src[0], cs = sh_src[1];
         if (tid == 0) d.srcs[blk] = make_int2(rs, cs);
+        int *const target = s1time;  // (the sources' times are taken)
         for (int k = tid; k <= Sm; k += blockDim.x) gcnt[k] = 0;
+        for (int j = tid; j < n1; j += blockDim.x) target[j] = determ[j];
         __syncthreads();
         for (int j = tid; j < n1; j += blockDim.x) {
-            const int k = determ[j];
+            const int k = target[j];
             if (j != rs && j != cs && k >= 0) atomicAdd(&gcnt[k + 1], 1);
         }
         __syncthreads();
@@ -1048,7 +1079,7 @@ __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want
             __syncwarp();
             for (int jb = 0; jb < n1; jb += 32) {
                 const int j = jb + lane;
-                const int k = j < n1 ? determ[j] : -1;
+                const int k = j < n1 ? target[j] : -1;
                 const bool ok = j < n1 && j != rs && j != cs && k >= 0;
                 const unsigned peers = __match_any_sync(0xffffffffu, ok ? k : -1 - lane);
                 if (ok) gidx[gcnt[k] + __popc(peers & ((1u << lane) - 1))] = j;
