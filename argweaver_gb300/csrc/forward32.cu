@@ -196,11 +196,13 @@ struct Int {
     static constexpr int value = N;
 };
 
-// One instance. KPT states per owner thread; their same-branch rows' first ROWS entries in
-// registers. TAIL: rows may be longer (ROWS < T - 1); the rest is read from shared memory, or
-// from global memory where the rows do not fit. STAGED: per-state tables staged a tree ahead
+// One instance. KPT states per owner thread; of their same-branch rows the first ROWS0 entries
+// (a thread's first state) and ROWS (its others) in registers. TAIL: rows may be longer than
+// that; the rest is read from shared memory, or from global memory where the rows do not fit.
+// SORT: the owners take the states in descending order of their node's, so that a warp's dots
+// are of like length, and past a thread's first state mostly short. STAGED: per-state tables staged a tree ahead
 // (else read from global memory). NTC: the threads at work, reducers and owners.
-template <int KPT, int ROWS, bool TAIL, bool STAGED>
+template <int KPT, int ROWS0, int ROWS, bool TAIL, bool STAGED, bool SORT>
 __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, int qi, int maxM, int t2_bufs, int NTC, V2 nz) {
     extern __shared__ __align__(16) unsigned char dyn_b[];
     constexpr int NP = (KPT + 1) / 2;      // packed pairs of states
@@ -225,6 +227,7 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
     float2 *const last = (float2 *)(dyn_b + P.last);  // a tree's last column, high and low parts
     __shared__ __align__(16) float tfp[32][NRW];   // [a][reducer] shares of tf; [31]: of the norm
     __shared__ uint64_t full;                      // the staged tree has landed
+    __shared__ int by_m[MAXT];                     // states by their node's, then where they begin
     __shared__ double lnl0;
 
     if (tid == 0) {
@@ -304,17 +307,16 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
         cw0 = class_at(lane);
         cw1 = class_at(32 + lane);
     }
-    // emission row r of a tree's variant columns into a ring slot
-    auto fetch = [&](float *slot, const float *row, int S) {
-#pragma unroll
-        for (int q = 0; q < KPT; q++)
-            if (st + q * NTS < S) cp_async4(slot + st + q * NTS, row + q * NTS);
-    };
     // the emission rows of a tree's first columns (classes in cw0): column i <= EDEPTH, slot i
     auto first_rows = [&](long long var0, int S, int len) {
-        const float *row = d.var32 + var0 + st;
+        const float *row = d.var32 + var0;
         unsigned todo = __ballot_sync(FULL, cw0 == COL_VARIANT && lane <= EDEPTH && lane < len);
-        for (; todo; todo &= todo - 1, row += S) fetch(ring + (__ffs(todo) - 1) * ringstride, row, S);
+        for (; todo; todo &= todo - 1, row += S) {
+            float *slot = ring + (__ffs(todo) - 1) * ringstride;
+#pragma unroll
+            for (int q = 0; q < KPT; q++)
+                if (st + q * NTS < S) cp_async4(slot + st + q * NTS, row + st + q * NTS);
+        }
 #pragma unroll
         for (int i = 0; i < EDEPTH; i++) cp_commit();  // all in the first group
     };
@@ -413,18 +415,39 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
             bool ok[KPT];
             int ks[KPT], nbo[KPT], pos[KPT], m[KPT], roff[KPT], tq[KPT], slot[KPT], most = 0, mostq[KPT];
             V2 rs[NP], iv[NP], xh[NP], xl[NP];
-            V2 row[KPT][ROWS / 2];  // entries y and y + 1 packed
+            V2 row0[ROWS0 / 2], row[KPT > 1 ? KPT - 1 : 1][ROWS / 2];  // entries y and y + 1 packed
+            const bool sorted = SORT && len > 3;
+            int *const order = (int *)col;  // until column 0 is stored
+            if (sorted) {
+                if (st < MAXT) by_m[st] = 0;
+                named_sync(5, NTS);
+                for (int k = st; k < S; k += NTS) atomicAdd(&by_m[MAXT - sinfo[k].m], 1);
+                named_sync(5, NTS);
+                if (st < 32) {
+                    const int c = by_m[lane];
+                    int incl = c;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int v = __shfl_up_sync(FULL, incl, o);
+                        if (lane >= o) incl += v;
+                    }
+                    by_m[lane] = incl - c;
+                }
+                named_sync(5, NTS);
+                for (int k = st; k < S; k += NTS) order[atomicAdd(&by_m[MAXT - sinfo[k].m], 1)] = k;
+                named_sync(5, NTS);
+            }
 #pragma unroll
             for (int q = 0; q < KPT; q++) {
                 ok[q] = st + q * NTS < S;
-                ks[q] = ok[q] ? st + q * NTS : 0;
+                ks[q] = !ok[q] ? 0 : sorted ? order[st + q * NTS] : st + q * NTS;
                 const StateInfo si = sinfo[ks[q]];
                 tq[q] = si.time;
                 nbo[q] = (si.j1 + 3 * si.node) & ~3;
                 pos[q] = ok[q] ? nbo[q] + ks[q] - si.j1 : colstride - 1;
                 m[q] = ok[q] ? si.m : 0;
                 roff[q] = t2off[ks[q]];
-                mostq[q] = TAIL ? uniform(m[q]) : 0;
+                mostq[q] = SORT || TAIL ? uniform(m[q]) : 0;
                 most = imax(most, m[q]);
             }
             // pair u: states 2 u and pair2(u), the same one where there is no second
@@ -437,28 +460,45 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                 xh[u] = xl[u] = pk(0.0f, 0.0f);
             }
             most = uniform(most);
-            // rows: 4, 8, 12, 20 or ROWS entries by the warp's longest, zeros past a node's states
-            auto load = [&](auto n) {
+            // rows: 4, 8, 12, 20 or all entries by the warp's longest, zeros past a node's states
+            auto by_length = [&](auto all, int longest, auto &&fn) {
+                constexpr int R = decltype(all)::value;
+                if (R <= 4 || longest <= 4) fn(Int<4>{});
+                else if (R <= 8 || longest <= 8) fn(Int<(R < 8 ? R : 8)>{});
+                else if (R <= 12 || longest <= 12) fn(Int<(R < 12 ? R : 12)>{});
+                else if (R > 20 && longest <= 20) fn(Int<(R < 20 ? R : 20)>{});
+                else fn(Int<R>{});
+            };
+            // fn(q, its row registers, the entries to take) for each of the thread's states
+            static_assert(SORT || KPT == 1 || ROWS0 == ROWS, "states in order: one length for all");
+            auto each_row = [&](auto &&fn) {
+                by_length(Int<ROWS0>{}, SORT ? mostq[0] : most, [&](auto n) {
+                    fn(0, row0, n);
+                    if constexpr (!SORT) {
 #pragma unroll
-                for (int q = 0; q < KPT; q++) {
-                    const float *r = rows + roff[q];
-#pragma unroll
-                    for (int y = 0; y < decltype(n)::value; y += 2) {
-                        const float v0 = y < m[q] ? r[0] : 0.0f, v1 = y + 1 < m[q] ? r[m[q]] : 0.0f;
-                        r += 2 * m[q];
-                        row[q][y / 2] = pk(v0, v1);
+                        for (int q = 1; q < KPT; q++) fn(q, row[q - 1], n);
                     }
+                });
+                if constexpr (SORT) {
+#pragma unroll
+                    for (int q = 1; q < KPT; q++)
+                        by_length(Int<ROWS>{}, mostq[q], [&](auto n) { fn(q, row[q - 1], n); });
                 }
             };
-            auto by_length = [&](auto &&fn) {
-                if (ROWS <= 4 || most <= 4) fn(Int<4>{});
-                else if (ROWS <= 8 || most <= 8) fn(Int<(ROWS < 8 ? ROWS : 8)>{});
-                else if (ROWS <= 12 || most <= 12) fn(Int<(ROWS < 12 ? ROWS : 12)>{});
-                else if (ROWS > 20 && most <= 20) fn(Int<(ROWS < 20 ? ROWS : 20)>{});
-                else fn(Int<ROWS>{});
-            };
+            // where a thread's states lie in an array of all, from `own` on
+            const int own = SORT ? 0 : st;
+            auto at = [&](int q) { return SORT ? ks[q] : q * NTS; };
             const float *tails = STAGED || !t2_bufs ? rows : t2buf;
-            by_length(load);
+            each_row([&](int q, auto &into, auto n) {
+                const float *r = rows + roff[q];
+#pragma unroll
+                for (int y = 0; y < decltype(n)::value; y += 2) {
+                    const float v0 = y < m[q] ? r[0] : 0.0f, v1 = y + 1 < m[q] ? r[m[q]] : 0.0f;
+                    r += 2 * m[q];
+                    into[y / 2] = pk(v0, v1);
+                }
+            });
+            cp_wait<EDEPTH - 1>();  // the first emission rows, which other threads read
             named_sync(3, NTC);  // positions stored, slots cleared
 #pragma unroll
             for (int q = 0; q < KPT; q++) {
@@ -498,7 +538,6 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                 const float *rr = table(d.recombrow32 + s0, SL.rrow);
                 const float *cr = table(d.recoalrow32 + s0, SL.crow);
                 const int2 src = *table(d.srcs + blk, SL.src);
-                cp_wait<EDEPTH - 1>();
                 // pairs: the previous column's values with their low parts, each deterministic
                 // move by its FP64 probability (kept as a complement near 1), the
                 // recombination rows (a small inflow) plain, then the emission
@@ -550,8 +589,7 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                 }
             }
             // the variant rows: the next one to fetch (column EDEPTH + 1 on)
-            const float *vrow = d.var32 + Bs->var0 + st +
-                                (size_t)__popcll(vm & ((2ull << EDEPTH) - 1)) * S;
+            const float *vrow = d.var32 + Bs->var0 + own + (size_t)__popcll(vm & ((2ull << EDEPTH) - 1)) * S;
             named_sync(4, NTC);  // T2 (barrier A of column 1): column 0 complete, the tables taken
             // the next tree's first classes and where its emission rows are
             int nS = 0, nlen = 0;
@@ -569,7 +607,7 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
             float *const ring_end = ring + EDEPTH * ringstride;
 
             // ---- columns; iteration i also finalises column i-1
-            float *outp = fw + st;
+            float *outp = fw + own;
             bool wr[KPT];  // the instance's column 0 keeps the unnormalised prior
 #pragma unroll
             for (int q = 0; q < KPT; q++) wr[q] = ok[q] && bi > 0;
@@ -579,7 +617,7 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                 if (ndone) {
 #pragma unroll
                     for (int q = 0; q < KPT; q++)
-                        if (wr[q]) outp[q * NTS] = q & 1 ? hi(done[q >> 1]) : lo(done[q >> 1]);
+                        if (wr[q]) outp[at(q)] = q & 1 ? hi(done[q >> 1]) : lo(done[q >> 1]);
 #pragma unroll
                     for (int q = 0; q < KPT; q++) wr[q] = ok[q];
                     outp += S;
@@ -597,34 +635,28 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                 // same-branch dots: sum_y t2[y][k] col[j1 + y], even and odd terms in the two
                 // halves of a packed sum
                 V2 dot2[KPT];
-                auto dots = [&](auto n) {
+                each_row([&](int q, const auto &from, auto n) {
+                    const float *nb = col + cur + nbo[q];
+                    V2 sum = pk(0.0f, 0.0f);
+#pragma unroll
+                    for (int y = 0; y < decltype(n)::value; y += 4) {
+                        const float4 v = *(const float4 *)(nb + y);
+                        sum = fma2(from[y / 2], pk(v.x, v.y), sum);
+                        sum = fma2(from[y / 2 + 1], pk(v.z, v.w), sum);
+                    }
+                    dot2[q] = sum;
+                });
+                if (TAIL && most > (ROWS < ROWS0 ? ROWS : ROWS0)) {
 #pragma unroll
                     for (int q = 0; q < KPT; q++) {
-                        const float *nb = col + cur + nbo[q];
-                        V2 sum = pk(0.0f, 0.0f);
+                        for (int y = q ? ROWS : ROWS0; y < mostq[q]; y += 4) {
+                            const float *r = tails + roff[q] + y * m[q];
+                            float v[4];
 #pragma unroll
-                        for (int y = 0; y < decltype(n)::value; y += 4) {
-                            const float4 v = *(const float4 *)(nb + y);
-                            sum = fma2(row[q][y / 2], pk(v.x, v.y), sum);
-                            sum = fma2(row[q][y / 2 + 1], pk(v.z, v.w), sum);
-                        }
-                        dot2[q] = sum;
-                    }
-                };
-                by_length(dots);
-                if (TAIL && most > ROWS) {
-                    for (int y = ROWS; y < most; y += 4) {
-#pragma unroll
-                        for (int q = 0; q < KPT; q++) {
-                            if (y < mostq[q]) {
-                                const float *r = tails + roff[q] + y * m[q];
-                                float v[4];
-#pragma unroll
-                                for (int u = 0; u < 4; u++) v[u] = y + u < m[q] ? r[u * m[q]] : 0.0f;
-                                const float4 n = *(const float4 *)(col + cur + nbo[q] + y);
-                                dot2[q] = fma2(pk(v[0], v[1]), pk(n.x, n.y), dot2[q]);
-                                dot2[q] = fma2(pk(v[2], v[3]), pk(n.z, n.w), dot2[q]);
-                            }
+                            for (int u = 0; u < 4; u++) v[u] = y + u < m[q] ? r[u * m[q]] : 0.0f;
+                            const float4 n = *(const float4 *)(col + cur + nbo[q] + y);
+                            dot2[q] = fma2(pk(v[0], v[1]), pk(n.x, n.y), dot2[q]);
+                            dot2[q] = fma2(pk(v[2], v[3]), pk(n.z, n.w), dot2[q]);
                         }
                     }
                 }
@@ -636,7 +668,12 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                     // column i - 1 + EDEPTH's row into the slot before column i - 1's (column
                     // i - 2 is done); this column's class masks are one shifted on
                     if (vm >> (EDEPTH - 1) & 1) {
-                        if (i - 1 + EDEPTH < len) fetch(slot_e == ring ? ring_end : slot_e - ringstride, vrow, S);
+                        if (i - 1 + EDEPTH < len) {
+                            float *slot = (slot_e == ring ? ring_end : slot_e - ringstride) + own;
+#pragma unroll
+                            for (int q = 0; q < KPT; q++)
+                                if (ok[q]) cp_async4(slot + at(q), vrow + at(q));
+                        }
                         vrow += S;
                     }
                     cp_commit();
@@ -716,7 +753,7 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                 const F2 x = f2_mul(q & 1 ? F2{hi(xh[q >> 1]), hi(xl[q >> 1])} : F2{lo(xh[q >> 1]), lo(xl[q >> 1])},
                                     inv_norm);
                 if (ok[q]) last[ks[q]] = make_float2(x.hi, x.lo);
-                if (wr[q]) outp[q * NTS] = x.hi;
+                if (wr[q]) outp[at(q)] = x.hi;
             }
         } else {
             // ================= reducers
@@ -880,21 +917,25 @@ __global__ void __launch_bounds__(32 * NRW + (FORMS == WIDE ? WIDE_OWNERS : OWNE
     // rows longer than the registers hold (a node spans at most T - 1 times): the tables staged
     // a tree ahead with two buffers of rows; where they do not fit, only the rows in shared
     // memory; else neither
+    // States are sorted by their node's for more than 21 time points alone: 1.69 us a column
+    // unsorted and 1.40 sorted at 1138 states of 32, 0.90 and 0.90 at 704 of 20, 1.30 and 1.32 at
+    // 930 (the sort and the scattered stores cost what the shorter dots give).
     constexpr int R4 = FORMS == WIDE ? 4 : 8;
+    constexpr int R3 = LONG ? 20 : 8, R40 = LONG ? R4 + 8 : R4;
     if (kpt == 1) {
-        forward32<1, LONG ? 32 : 20, false, true>(d, I, qi, maxM, 1, ntc, nz);
+        forward32<1, LONG ? 32 : 20, 2, false, true, false>(d, I, qi, maxM, 1, ntc, nz);
     } else if (kpt == 2) {
-        if (!LONG) forward32<2, 20, false, true>(d, I, qi, maxM, 1, ntc, nz);
-        else if (fits(2, true)) forward32<2, 16, true, true>(d, I, qi, maxM, 2, ntc, nz);
-        else forward32<4, R4, true, false>(d, I, qi, maxM, fits(1, false), ntc, nz);
+        if (!LONG) forward32<2, 20, 20, false, true, false>(d, I, qi, maxM, 1, ntc, nz);
+        else if (fits(2, true)) forward32<2, 20, 12, true, true, true>(d, I, qi, maxM, 2, ntc, nz);
+        else forward32<4, R40, R4, true, false, LONG>(d, I, qi, maxM, fits(1, false), ntc, nz);
     } else if (FORMS != FEW && kpt == 3) {
-        if (fits(2, true)) forward32<3, 8, true, true>(d, I, qi, maxM, 2, ntc, nz);
-        else forward32<3, 8, true, false>(d, I, qi, maxM, fits(1, false), ntc, nz);
+        if (fits(2, true)) forward32<3, R3, 8, true, true, LONG>(d, I, qi, maxM, 2, ntc, nz);
+        else forward32<3, R3, 8, true, false, LONG>(d, I, qi, maxM, fits(1, false), ntc, nz);
     } else if (kpt == 4) {
-        if (FORMS != WIDE && fits(2, true)) forward32<4, R4, true, true>(d, I, qi, maxM, 2, ntc, nz);
-        else forward32<4, R4, true, false>(d, I, qi, maxM, fits(1, false), ntc, nz);
+        if (FORMS != WIDE && fits(2, true)) forward32<4, R40, R4, true, true, LONG>(d, I, qi, maxM, 2, ntc, nz);
+        else forward32<4, R40, R4, true, false, LONG>(d, I, qi, maxM, fits(1, false), ntc, nz);
     } else {
-        forward32<8, 4, true, false>(d, I, qi, maxM, fits(1, false), ntc, nz);
+        forward32<8, 4, 4, true, false, LONG>(d, I, qi, maxM, fits(1, false), ntc, nz);
     }
 }
 
