@@ -303,8 +303,8 @@ void launch(const BatchDev &d, double *bw_out, cudaStream_t s) {
 }  // namespace
 
 void launch_backward(const BatchDev &d, bool fp32, double *bw_out, cudaStream_t s) {
-    if (launch_backward_chain(d, fp32, bw_out, s)) return;
-    if (fp32) launch<float>(d, bw_out, s);
+    if (launch_backward_chain(d, fp32, s)) launch_posterior(d, fp32, bw_out, s);
+    else if (fp32) launch<float>(d, bw_out, s);
     else launch<double>(d, bw_out, s);
 }
 

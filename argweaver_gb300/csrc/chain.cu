@@ -850,13 +850,15 @@ bool launch_forward64(const BatchDev &d, cudaStream_t s, bool table) {
     return true;
 }
 
-bool launch_backward_chain(const BatchDev &d, bool fp32, double *bw_out, cudaStream_t s) {
-    if (!(fp32 ? launch<float, false>(d, s) : launch<double, false>(d, s))) return false;
+bool launch_backward_chain(const BatchDev &d, bool fp32, cudaStream_t s) {
+    return fp32 ? launch<float, false>(d, s) : launch<double, false>(d, s);
+}
+
+void launch_posterior(const BatchDev &d, bool fp32, double *bw_out, cudaStream_t s) {
     const dim3 grid(d.nblocks, column_shares(d));
     if (fp32) k_posterior<float><<<grid, 128, 0, s>>>(d, bw_out);
     else k_posterior<double><<<grid, 128, 0, s>>>(d, bw_out);
     note_launch();
-    return true;
 }
 
 }  // namespace awg

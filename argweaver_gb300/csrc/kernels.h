@@ -47,10 +47,14 @@ bool forward_writes_bins(int maxS);
 // launched).
 bool launch_forward32(const BatchDev &d, cudaStream_t s, int kpt);
 bool launch_forward64(const BatchDev &d, cudaStream_t s, bool table);
-bool launch_backward_chain(const BatchDev &d, bool fp32, double *bw_out, cudaStream_t s);
+// K5's first half: the backward table into d.post. It reads nothing that K3 writes, so the two
+// passes may run side by side.
+bool launch_backward_chain(const BatchDev &d, bool fp32, cudaStream_t s);
+// K5's second half: the marginals from both tables.
+void launch_posterior(const BatchDev &d, bool fp32, double *bw_out, cudaStream_t s);
 // K4: stochastic traceback, one warp per instance; FP32 with bins32 set: the decomposed draw.
 void launch_traceback(const BatchDev &d, bool fp32, cudaStream_t s);
-// K5: backward pass fused with the posterior marginals, one CTA per instance.
+// K5: backward pass and posterior marginals, behind K3 on one stream.
 void launch_backward(const BatchDev &d, bool fp32, double *bw_out, cudaStream_t s);
 
 // Kernel attributes, set once per kernel and safe to call from several host threads (the
