@@ -19,7 +19,7 @@
 //     and parallel kernels normalise it where it is wanted. The log-likelihood telescopes to
 //     log(sum of the last column) plus ln 2 times the exponents.
 //   - the power is chosen a column ahead, so a column's factor is ready before its inflow and
-//     ends it with one fused product: 1.22 us a column at 99 states and 2.81 at 483, 1.27 and
+//     ends it with one fused product: 1.22 us a column at 99 states and 2.81 at 483 when it came in, 1.27 and
 //     2.90 with the power of the column's own bins (1.99 and 4.46 with a division a column).
 //   - bins by a segmented scan over lanes (log2 of a bin's lanes dependent adds); the product
 //     with tm split over all lanes of the four reduction warps, so the owners add one value
@@ -28,6 +28,10 @@
 //     have dots of like length, and up to OWNERS / 2 states two lanes take one state's even
 //     and odd terms. A dot is always (even terms) + (odd terms): results do not depend on the
 //     form, the block size or the batch.
+//   - a tree's set-up (13,000 cycles at 99 states, 20,000 at 483, where a tree has some 30
+//     columns) waits for memory as few times as it can: rows are copied as they lie and turned
+//     into moving parts by the owner of their dot, a switch's sources come two at a time.
+//     10,000 columns in 221 trees at 99 states: 13.2 ms with rows gathered by state, 12.9 so.
 // FP32 (backward): the stay and the emission, which carry almost all of a state's mass, on
 // pairs (f2.cuh), the inflow plain.
 
@@ -357,7 +361,21 @@ __device__ __forceinline__ void run_chain(const BatchDev &d, const InstDev &I, i
             hist[a] = 0;
         }
         for (int p = tid; p < S; p += NTC) rank[d.bt_perm[s0 + p]] = p;
-        named_sync(4, NTC);  // tm, bins, positions, sums
+        // the rows as they lie: one wait for memory, where a thread that gathered a state's own
+        // entries waited for each
+        if (rows_n) {
+            const F *const rows = tab.rows + B.t2_0;
+            const int M = B.M;
+            for (int e0 = tid; e0 < M; e0 += 8 * NTC) {
+                F v[8];
+#pragma unroll
+                for (int x = 0; x < 8; x++) v[x] = e0 + x * NTC < M ? rows[e0 + x * NTC] : F(0);
+#pragma unroll
+                for (int x = 0; x < 8; x++)
+                    if (e0 + x * NTC < M) rowsS[e0 + x * NTC] = v[x];
+            }
+        }
+        named_sync(4, NTC);  // tm, bins, positions, rows, sums
         if (tid == 0) {
             if (FWD) {
                 sumk -= ek;
@@ -377,17 +395,9 @@ __device__ __forceinline__ void run_chain(const BatchDev &d, const InstDev &I, i
             sbS[r + 1] = sbS[r] + 32 * ckS[r];
         }
         for (int x = tid; x < sbS[NRW]; x += NTC) head[x] = own[x] = F(0);
-        // rows, and owners' order: descending by the node's states
-        for (int k = tid; k < S; k += NTC) {
-            const StateInfo si = d.sinfo[s0 + k];
-            if (SORT) atomicAdd(&hist[MAXT - si.m], 1);
-            if (rows_n) {
-                const int off = d.t2off[s0 + k], a0 = si.time - (k - si.j1);
-                for (int y = 0; y < si.m; y++)
-                    rowsS[off + y * si.m] = Tab<F>::t2(tab.rows[B.t2_0 + off + y * si.m], tmS[(a0 + y) * MAXT + si.time]);
-            }
-        }
         if (SORT) {
+            // owners' order: descending by the node's states
+            for (int k = tid; k < S; k += NTC) atomicAdd(&hist[MAXT - d.sinfo[s0 + k].m], 1);
             named_sync(4, NTC);  // counts
             if (rw == 0) {
                 const int n = hist[lane];
@@ -403,7 +413,7 @@ __device__ __forceinline__ void run_chain(const BatchDev &d, const InstDev &I, i
             named_sync(4, NTC);  // starts
             for (int k = tid; k < S; k += NTC) order[atomicAdd(&hist[MAXT - d.sinfo[s0 + k].m], 1)] = k;
         }
-        named_sync(4, NTC);  // rows, order, slots cleared
+        named_sync(4, NTC);  // order, slots cleared
 
         if (!reducer) {
             // ================= owners
@@ -411,6 +421,8 @@ __device__ __forceinline__ void run_chain(const BatchDev &d, const InstDev &I, i
             bool ok[KPT];   // publishes its state
             F iv[KPT], rs[KPT], e_next[KPT];
             F2 g[KPT];      // FP32: the owned states' published pairs
+            int g0[KPT], gn[KPT], gmost = 0;  // forward: the switch's gather list
+            F rr[KPT], cr[KPT];               // and breakpoint factors, loaded with the rest
             const int half = SPLIT == 2 ? st & 1 : 0;
 #pragma unroll
             for (int q = 0; q < KPT; q++) {
@@ -432,6 +444,16 @@ __device__ __forceinline__ void run_chain(const BatchDev &d, const InstDev &I, i
                 e_next[q] = F(0);
                 g[q] = F2{0.0f, 0.0f};
                 most = imax(most, cnt[q]);
+                g0[q] = gn[q] = 0;
+                rr[q] = cr[q] = F(0);
+                if (FWD && !first) {
+                    const int *gp = d.gptr + B.gptr0 + k;
+                    g0[q] = gp[0];
+                    gn[q] = ok[q] ? gp[1] - g0[q] : 0;
+                    rr[q] = tab.rrow[s0 + k];
+                    cr[q] = tab.crow[s0 + k];
+                    gmost = imax(gmost, gn[q]);
+                }
                 // its slot: in the first piece of a chunk, or in the bin's own piece
                 const int p = rank[k], b = si.time, bs = bptr[b];
                 int r = 0;
@@ -451,6 +473,23 @@ __device__ __forceinline__ void run_chain(const BatchDev &d, const InstDev &I, i
                 slot[q] = clo >= bs ? P.head + sb + 32 * (p - clo) + l : P.own + sb + 32 * (p - bs) + (b - bl);
             }
             most = uniform(most);
+            gmost = uniform(gmost);
+            // the rows' moving parts (FP32: they are that already): an entry belongs to one dot, so
+            // its owner forms them, a warp's lanes having rows of like length
+            if (rows_n && !pairs) {
+#pragma unroll
+                for (int q = 0; q < KPT; q++) {
+                    const int t0 = tq[q] - (ks[q] - (nb[q] - half)) + half;
+                    F *r = rowsS + ro[q];
+                    const F *tm = tmS + (FWD ? t0 * MAXT + tq[q] : tq[q] * MAXT + t0);
+#pragma unroll 4
+                    for (int y = 0; y < cnt[q]; y++) {
+                        *r = Tab<F>::t2(*r, *tm);
+                        r += SPLIT * rst[q];
+                        tm += FWD ? SPLIT * MAXT : SPLIT;
+                    }
+                }
+            }
             const F *var = tab.var + B.var0;
             int vr = FWD ? 0 : uniform(B.nvar);  // FWD: the next variant row; else one past it
             auto load_next = [&](int abs) {      // the emissions of column abs, if variant
@@ -503,19 +542,38 @@ __device__ __forceinline__ void run_chain(const BatchDev &d, const InstDev &I, i
                 for (int q = 0; q < KPT; q++)
                     if (ok[q]) cur[ks[q]] = base_f[slot[q]] = x_own[q] = outf[ks[q]];  // priors (K1)
             } else {
+                F sums[KPT];
+                if constexpr (FWD) {
+                    const int *gi = d.gidx + B.prev_state0;
+                    const F *dp = tab.dprob + B.prev_state0;
+#pragma unroll
+                    for (int q = 0; q < KPT; q++) sums[q] = F(0);
+                    for (int t = 0; t < gmost; t += 2) {  // two sources of each state at a time
+                        int j[KPT][2];
+                        F p[KPT][2];
+#pragma unroll
+                        for (int q = 0; q < KPT; q++)
+#pragma unroll
+                            for (int x = 0; x < 2; x++) j[q][x] = t + x < gn[q] ? gi[g0[q] + t + x] : 0;
+#pragma unroll
+                        for (int q = 0; q < KPT; q++)
+#pragma unroll
+                            for (int x = 0; x < 2; x++) p[q][x] = t + x < gn[q] ? dp[j[q][x]] : F(0);
+#pragma unroll
+                        for (int q = 0; q < KPT; q++)
+#pragma unroll
+                            for (int x = 0; x < 2; x++)
+                                if (t + x < gn[q]) sums[q] = fma(prev[j[q][x]], p[q][x], sums[q]);
+                    }
+                }
 #pragma unroll
                 for (int q = 0; q < KPT; q++) {
                     if (!ok[q]) continue;
                     const int k = ks[q];
                     if constexpr (FWD) {
-                        const int *gp = d.gptr + B.gptr0;
-                        const int *gi = d.gidx + B.prev_state0;
-                        const F *dp = tab.dprob + B.prev_state0;
-                        F s = F(0);
-                        for (int p = gp[k]; p < gp[k + 1]; p++) s = fma(prev[gi[p]], dp[gi[p]], s);
-                        const F rr = tab.rrow[s0 + k], cr = tab.crow[s0 + k];
-                        if (src.x != -1 && rr > F(0)) s += prev[src.x] * rr;
-                        if (src.y != -1 && cr > F(0)) s += prev[src.y] * cr;
+                        F s = sums[q];
+                        if (src.x != -1 && rr[q] > F(0)) s += prev[src.x] * rr[q];
+                        if (src.y != -1 && cr[q] > F(0)) s += prev[src.y] * cr[q];
                         s *= factor(abs, q, ek);
                         outf[k] = s;
                         cur[k] = base_f[slot[q]] = x_own[q] = s;
