@@ -40,7 +40,7 @@ def nvcc_flags(src: str):
         return [f if f != "--fmad=false" else "--fmad=true" for f in NVCC_FLAGS]
     return NVCC_FLAGS
 
-CUDA_SOURCES = ["host_plan.cpp", "tables.cu", "forward.cu", "forward32.cu", "chain.cu", "emit_df.cu", "traceback.cu",
+CUDA_SOURCES = ["host_plan.cpp", "tables.cu", "forward.cu", "forward32.cu", "chain.cu", "emit_groups.cu", "traceback.cu",
                 "backward.cu", "batch.cu", "static_run.cu", "dense_hmm.cu", "dense_tables.cu",
                 "arg_prob.cu", "recomb.cu", "capi.cpp", "server.cpp", "formats.cpp",
                 "arg_surgery.cpp"]

@@ -1,4 +1,5 @@
-// K5: backward pass fused with the posterior marginals, one CTA per instance.
+// K5 for trees of more than 3,072 states (the others: chain.cu): backward pass fused with the
+// posterior marginals, one CTA per instance.
 //
 // The reference has no backward pass for the threading HMM. This one uses the forward
 // pass's transition semantics (TransMatrix::get, trans.h:64-83; TransMatrixSwitch::get,

@@ -3,7 +3,8 @@
 // Device memory is one grow-only arena per process (no allocation per call once warm);
 // inputs travel in one pinned staging buffer and one host-to-device copy. The kernel
 // sequence is K1 tables -> K2 variant emissions -> K3 forward -> K4 traceback (when a path
-// is wanted) -> K5 backward+posterior (when posteriors are wanted), all on one stream.
+// is wanted); K5's backward pass (when posteriors are wanted) runs beside K3, the marginals
+// behind both.
 
 #include <cuda_runtime.h>
 

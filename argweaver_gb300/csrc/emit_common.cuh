@@ -1,4 +1,4 @@
-// Shared by the emission kernels (tables.cu, emit_df.cu): a tree's level schedules, the
+// Shared by the emission kernels (tables.cu, emit_groups.cu): a tree's level schedules, the
 // infinite-sites test, the log-likelihood's references and the persistent kernels' work queue.
 #pragma once
 

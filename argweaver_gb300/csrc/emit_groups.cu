@@ -1,10 +1,11 @@
-// K2 of the FP32 path in double-float: emissions of a tree's variant columns (calc_emissions'
-// non-invariant branch, emit.cpp:822-844), each as its ratio to the column's largest, rounded
-// once.
+// K2: emissions of a tree's variant columns (calc_emissions' non-invariant branch,
+// emit.cpp:822-844), in FP64 as the reference forms them, or for the FP32 path in double-float,
+// each as its ratio to the column's largest, rounded once.
 //
 // Per column: inner partials up the tree (likelihood_site_node_inner, emit.cpp:151-196), outer
 // partials down it (likelihood_site_outer, emit.cpp:273-296), then calc_emit (emit.cpp:620-645)
-// for the states; JC69 steps as P x = mut * sum(x) + (nomut - mut) * x.
+// for the states; JC69 steps in the reference's order (FP64) or as P x = mut * sum(x) +
+// (nomut - mut) * x.
 //
 // What bounds it: instructions at the states (about 200 each a column) and, in the tree passes,
 // the chain of levels (some 15 up and 15 down at 64 leaves, few nodes on most of them) with the
@@ -18,9 +19,12 @@
 //     warp), so 3 or 4 CTAs fit an SM where 1 or 2 did.
 // 402,000 trees of 8 to 64 leaves, 37 columns each with 11 variant: 70.6 ms with a warp a column
 // and factors by state, 47.7 ms so; 840 trees of 150 to 200 leaves at 32 time points: 6.28 and
-// 1.26 ms.
+// 1.26 ms. FP64 (the FP64 pipe, one SM a tree): 99 trees of 21 leaves 0.45 and 0.26 ms, 202 of 64
+// leaves 1.55 and 1.38 ms.
 
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "df.cuh"
 #include "emit_common.cuh"
@@ -35,20 +39,43 @@ constexpr int WINDOW = 1024;  // columns whose variant ones are listed at a time
 constexpr int GMAX = 8;       // columns a warp carries through the tree at once, at most
 constexpr unsigned FULL = 0xffffffffu;
 
-// JC69 factors of a branch: mut and nomut - mut
-struct Factor {
+// JC69 factors of a branch: mut, and nomut - mut (double-float) or nomut (FP64)
+template <typename R>
+struct Factor;
+template <>
+struct Factor<df> {
     df m, d;
-    __device__ Factor() {}
     __device__ Factor(df mut, df nomut) : m(mut), d(nomut - mut) {}
+    __device__ explicit Factor(const float4 *t) {
+        const float4 v = *t;
+        m = df(v.x, v.y);
+        d = df(v.z, v.w);
+    }
+    __device__ void store(float4 *t) const { *t = make_float4(m.hi, m.lo, d.hi, d.lo); }
 };
-__device__ __forceinline__ Factor factor_at(const float4 *t) {
-    const float4 v = *t;
-    Factor f;
-    f.m = df(v.x, v.y);
-    f.d = df(v.z, v.w);
-    return f;
+template <>
+struct Factor<double> {
+    double m, d;
+    __device__ Factor(double mut, double nomut) : m(mut), d(nomut) {}
+    __device__ explicit Factor(const float4 *t) {
+        const double2 v = *(const double2 *)t;
+        m = v.x;
+        d = v.y;
+    }
+    __device__ void store(float4 *t) const { *(double2 *)t = make_double2(m, d); }
+};
+__device__ __forceinline__ void load2(const float4 *p, df &a, df &b) {
+    const float4 v = *p;
+    a = df(v.x, v.y);
+    b = df(v.z, v.w);
 }
-__device__ __forceinline__ float4 pack(df a, df b) { return make_float4(a.hi, a.lo, b.hi, b.lo); }
+__device__ __forceinline__ void load2(const float4 *p, double &a, double &b) {
+    const double2 v = *(const double2 *)p;
+    a = v.x;
+    b = v.y;
+}
+__device__ __forceinline__ void store2(float4 *p, df a, df b) { *p = make_float4(a.hi, a.lo, b.hi, b.lo); }
+__device__ __forceinline__ void store2(float4 *p, double a, double b) { *(double2 *)p = make_double2(a, b); }
 
 // An instance's branch factors by time points i <= j (entry tri(i) + j): every branch is a
 // difference of two time points floored at mintime. Node branches and split branches round
@@ -60,41 +87,41 @@ __host__ __device__ inline int tri_size(int T) { return T * (T + 1) / 2; }
 // X, 2 (X and any other: the leaves' are (1, 0) or, missing, (1, 1), and JC69 treats the other
 // three alike; about 26% of all columns at 0.5% missing calls, 87% of the variant ones). Half h
 // of the partials is an array of its own, so lanes on neighbouring pairs read without conflicts.
-template <int NC>
+template <typename R, int NC>
 struct Part {
-    df x[NC];
+    R x[NC];
     __device__ __forceinline__ void load(const float4 *p, int stride) {
 #pragma unroll
-        for (int h = 0; h < NC / 2; h++) {
-            const float4 v = p[h * stride];
-            x[2 * h] = df(v.x, v.y);
-            x[2 * h + 1] = df(v.z, v.w);
-        }
+        for (int h = 0; h < NC / 2; h++) load2(p + h * stride, x[2 * h], x[2 * h + 1]);
     }
     __device__ __forceinline__ void store(float4 *p, int stride) const {
 #pragma unroll
-        for (int h = 0; h < NC / 2; h++) p[h * stride] = pack(x[2 * h], x[2 * h + 1]);
+        for (int h = 0; h < NC / 2; h++) store2(p + h * stride, x[2 * h], x[2 * h + 1]);
     }
     __device__ __forceinline__ void leaf(uint8_t ch) {
         if constexpr (NC == 2) {
             x[0] = df(1.0f, 0.0f);
             x[1] = ch == 'N' ? df(1.0f, 0.0f) : df();
         } else {
-            leaf_partial<df>(ch, x);
+            leaf_partial<R>(ch, x);
         }
     }
     __device__ __forceinline__ void ones() {
 #pragma unroll
-        for (int a = 0; a < NC; a++) x[a] = df(1.0f, 0.0f);
+        for (int a = 0; a < NC; a++) x[a] = R(1);
     }
-    __device__ __forceinline__ Part step(const Factor &f) const {
+    __device__ __forceinline__ Part step(const Factor<R> &f) const {
         Part y;
-        df sum;
-        if constexpr (NC == 2) sum = df_addp(x[0], df(3.0f, 0.0f) * x[1]);
-        else sum = (x[0] + x[1]) + (x[2] + x[3]);
-        const df ms = f.m * sum;
+        if constexpr (std::is_same<R, double>::value) {
+            jc_apply<false>(x, f.m, f.d, y.x);  // the reference's order
+        } else {
+            df sum;
+            if constexpr (NC == 2) sum = df_addp(x[0], df(3.0f, 0.0f) * x[1]);
+            else sum = (x[0] + x[1]) + (x[2] + x[3]);
+            const df ms = f.m * sum;
 #pragma unroll
-        for (int a = 0; a < NC; a++) y.x[a] = df_addp(f.d * x[a], ms);
+            for (int a = 0; a < NC; a++) y.x[a] = df_addp(f.d * x[a], ms);
+        }
         return y;
     }
     __device__ __forceinline__ Part operator*(const Part &o) const {
@@ -127,7 +154,7 @@ __host__ __device__ inline int tree_bytes(int n, int S) {
 }
 
 // G columns (window positions list[0 .. G)) of a tree by one warp.
-template <int NC>
+template <typename R, int NC>
 __device__ void emit_group(const BatchDev &d, const BlockDev &B, const InstDev &I, const Tree &t,
                            char *area, const uint16_t *list, int w0, int G, unsigned vword, double penalty) {
     const int lane = threadIdx.x & 31;
@@ -142,7 +169,7 @@ __device__ void emit_group(const BatchDev &d, const BlockDev &B, const InstDev &
 
     for (int e = lane; e < t.inp[1] * G; e += 32) {
         const int x = e * inv >> 16, g = e - x * G, j = t.inl[x];
-        Part<NC> p;
+        Part<R, NC> p;
         p.leaf(seq[(size_t)(start + list[g]) * ns + j]);
         p.store(in + j * G + g, half);
     }
@@ -152,15 +179,15 @@ __device__ void emit_group(const BatchDev &d, const BlockDev &B, const InstDev &
         for (int e = lane; e < m; e += 32) {
             const int x = e * inv >> 16, g = e - x * G, j = t.inl[x0 + x];
             const int c1 = nd[j].y, c2 = nd[j].z;
-            Part<NC> a, b;
+            Part<R, NC> a, b;
             a.load(in + c1 * G + g, half);
             b.load(in + c2 * G + g, half);
-            (a.step(factor_at(t.nf + c1)) * b.step(factor_at(t.nf + c2))).store(in + j * G + g, half);
+            (a.step(Factor<R>(t.nf + c1)) * b.step(Factor<R>(t.nf + c2))).store(in + j * G + g, half);
         }
         __syncwarp();
     }
     if (lane < G) {
-        Part<NC> p;
+        Part<R, NC> p;
         p.ones();
         p.store(out + t.mainr * G + lane, half);
     }
@@ -172,13 +199,13 @@ __device__ void emit_group(const BatchDev &d, const BlockDev &B, const InstDev &
             const int p = nd[j].x;
             const int4 np = nd[p];
             const int sib = np.y == j ? np.z : np.y;
-            Part<NC> a;
+            Part<R, NC> a;
             a.load(in + sib * G + g, half);
-            a = a.step(factor_at(t.nf + sib));
+            a = a.step(Factor<R>(t.nf + sib));
             if (p != t.mainr) {
-                Part<NC> b;
+                Part<R, NC> b;
                 b.load(out + p * G + g, half);
-                a = a * b.step(factor_at(t.nf + p));
+                a = a * b.step(Factor<R>(t.nf + p));
             }
             a.store(out + j * G + g, half);
         }
@@ -189,35 +216,54 @@ __device__ void emit_group(const BatchDev &d, const BlockDev &B, const InstDev &
         const int col = start + list[g];
         // the threaded leaf's (or cut subtree's) factor by the state's time
         if (lane < t.T) {
-            Part<NC> p;
+            Part<R, NC> p;
             if (t.internal) p.load(in + t.node1 * G + g, half);
             else p.leaf(seq[(size_t)col * ns + t.nleaves]);
-            p.step(factor_at(t.internal ? t.st + tri(t.T, t.age1) + imax(lane, t.age1) : t.e0 + lane))
+            p.step(Factor<R>(t.internal ? t.st + tri(t.T, t.age1) + imax(lane, t.age1) : t.e0 + lane))
                 .store(p1s + lane, t.T);
         }
         __syncwarp();
-        auto state_v = [&](int k) -> df {
+        auto state_v = [&](int k) -> R {
             const int2 sk = t.states[k];
             const int node2 = sk.x & 0xffff;
-            Part<NC> p1, p2, p3;
+            Part<R, NC> p1, p2, p3;
             p1.load(p1s + (sk.x >> 16), t.T);
             p2.load(in + node2 * G + g, half);
-            p2 = p2.step(factor_at(t.st + (sk.y & 0xffff)));
+            p2 = p2.step(Factor<R>(t.st + (sk.y & 0xffff)));
             if constexpr (NC == 2) {
                 if (node2 != t.mainr) {
                     p3.load(out + node2 * G + g, half);
-                    p2 = p2 * p3.step(factor_at(t.st + (sk.y >> 16)));
+                    p2 = p2 * p3.step(Factor<R>(t.st + (sk.y >> 16)));
                 }
                 return df_addp(p1.x[0] * p2.x[0], df(3.0f, 0.0f) * (p1.x[1] * p2.x[1]));
             } else {
                 p1 = p1 * p2;
                 if (node2 != t.mainr) {
                     p3.load(out + node2 * G + g, half);
-                    p1 = p1 * p3.step(factor_at(t.st + (sk.y >> 16)));
+                    p1 = p1 * p3.step(Factor<R>(t.st + (sk.y >> 16)));
                 }
-                return ((p1.x[0] + p1.x[1]) + p1.x[2]) + p1.x[3];
+                if constexpr (std::is_same<R, double>::value) {
+                    double v = 0;
+#pragma unroll
+                    for (int a = 0; a < 4; a++) v += p1.x[a] * .25;
+                    return v;
+                } else {
+                    return ((p1.x[0] + p1.x[1]) + p1.x[2]) + p1.x[3];
+                }
             }
         };
+        const int vrow = d.colvar[I.col0 + col];
+        if constexpr (std::is_same<R, double>::value) {
+            // FP64: as they are; the states that break the infinite-sites model times the penalty
+            double *row = d.varemit + B.var0 + (size_t)vrow * t.S;
+            for (int kb = 0; kb < t.S; kb += 32) {
+                const int k = imin(kb + lane, t.S - 1);
+                double v = state_v(k);
+                if (penalty < 1.0 && !state_ok(vword, t.states[k].x & 0xffff)) v *= penalty;
+                if (kb + lane < t.S) row[k] = v;
+            }
+            __syncwarp();
+        } else {
         // two states per lane at a time: independent chains the scheduler can interleave (the
         // second one repeats the first where it would run past S)
         df ref = df();
@@ -249,7 +295,6 @@ __device__ void emit_group(const BatchDev &d, const BlockDev &B, const InstDev &
         const df one(1.0f, 0.0f);
         const df y0(1.0f / ref.hi, 0.0f);
         const df inv1 = y0 + y0 * (one - ref * y0);
-        const int vrow = d.colvar[I.col0 + col];
         float *row = d.var32 + B.var0 + (size_t)vrow * t.S;
         for (int k = lane; k < t.S; k += 32) {
             // e_k / e_ref; the largest state's r can round a hair above 1, so its complement
@@ -262,10 +307,12 @@ __device__ void emit_group(const BatchDev &d, const BlockDev &B, const InstDev &
         }
         if (lane == 0) d.vref[B.vrow0 + vrow] = .25 * (double)ref;
         __syncwarp();
+        }
     }
 }
 
 // The variant columns of one tree, by the whole CTA.
+template <typename R>
 __device__ __forceinline__ void emit_tree(const BatchDev &d, int blk, int maxS, int smem_bytes, int &cached) {
     extern __shared__ int4 dyn[];
     __shared__ double times[MAXT];
@@ -274,8 +321,9 @@ __device__ __forceinline__ void emit_tree(const BatchDev &d, int blk, int maxS, 
     const BlockDev B = d.blocks[blk];
     const InstDev I = d.inst[B.inst];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthreads = blockDim.x, nwarps = nthreads >> 5;
+    constexpr bool FP32 = std::is_same<R, df>::value;  // else the plain FP64 path
     if (B.nvar == 0 || B.S == 0) {
-        if (warp == 0) block_log_offset(d, B, I, blk, lane);
+        if (FP32 && warp == 0) block_log_offset(d, B, I, blk, lane);
         return;
     }
     const int T = I.T, n = I.nnodes, S = B.S;
@@ -326,21 +374,22 @@ __device__ __forceinline__ void emit_tree(const BatchDev &d, int blk, int maxS, 
         return;
     }
     if (refill) {
-        const df quarter(0.25f, 0.0f), one(1.0f, 0.0f), three(3.0f, 0.0f);
-        auto split = [&](double e) {  // branch_mut / branch_nomut in double-float
-            const df ex(e);
-            const Factor f(quarter * (one - ex), quarter * (one + three * ex));
-            return pack(f.m, f.d);
+        auto split = [&](double e, float4 *at) {  // a split branch's factors
+            if constexpr (FP32) {  // branch_mut / branch_nomut in double-float
+                const df quarter(0.25f, 0.0f), one(1.0f, 0.0f), three(3.0f, 0.0f), ex(e);
+                Factor<df>(quarter * (one - ex), quarter * (one + three * ex)).store(at);
+            } else {
+                Factor<double>(branch_mut(e), branch_nomut(e)).store(at);
+            }
         };
         for (int e = tid; e < T * T; e += nthreads) {
             const int i = e / T, j = e - i * T;
             if (j < i) continue;
             const double x = branch_exp(fmax(times[j] - times[i], mintime), mu);
-            st[tri(T, i) + j] = split(x);
-            const Factor f(df(branch_mut(x)), df(branch_nomut(x)));
-            nt[tri(T, i) + j] = pack(f.m, f.d);
+            split(x, st + tri(T, i) + j);
+            Factor<R>(R(branch_mut(x)), R(branch_nomut(x))).store(nt + tri(T, i) + j);
         }
-        for (int j = tid; j < T; j += nthreads) e0[j] = split(branch_exp(fmax(times[j] - 0.0, mintime), mu));
+        for (int j = tid; j < T; j += nthreads) split(branch_exp(fmax(times[j] - 0.0, mintime), mu), e0 + j);
         if (tid == 0) cached = B.inst;
     }
     // a branch's entry; ages beyond the time grid (which no branch of a valid tree has) are
@@ -406,6 +455,10 @@ __device__ __forceinline__ void emit_tree(const BatchDev &d, int blk, int maxS, 
                     continue;
                 }
                 const uint8_t *chars = d.seqT + I.seq0 + (size_t)(B.start + w0 + c) * ns;
+                if (!FP32) {
+                    if (lane == 0) list[WINDOW - 1 - atomicAdd(&nother, 1)] = (uint16_t)c;
+                    continue;
+                }
                 unsigned have = 0;  // bases seen: bits of the upper-case letters' low five bits
                 for (int j = lane; j < ns; j += 32) {
                     const uint8_t ch = chars[j];
@@ -442,36 +495,40 @@ __device__ __forceinline__ void emit_tree(const BatchDev &d, int blk, int maxS, 
                 vword = infsites_nodes(t, d.seqT + I.seq0 + (size_t)(B.start + w0 + ls[0]) * ns, (uint8_t *)area,
                                        (uint8_t *)area + n);
             __syncwarp();
-            if (near) emit_group<2>(d, B, I, t, area, ls, w0, G, vword, penalty);
-            else emit_group<4>(d, B, I, t, area, ls, w0, G, vword, penalty);
+            if constexpr (FP32) {
+                if (near) emit_group<df, 2>(d, B, I, t, area, ls, w0, G, vword, penalty);
+                else emit_group<df, 4>(d, B, I, t, area, ls, w0, G, vword, penalty);
+            } else {
+                emit_group<double, 4>(d, B, I, t, area, ls, w0, G, vword, penalty);
+            }
         }
         __syncthreads();
         if (tid == 0) nnear = nother = taken = 0;
         __syncthreads();
     }
-    if (warp == 0) block_log_offset(d, B, I, blk, lane);
+    if (FP32 && warp == 0) block_log_offset(d, B, I, blk, lane);
 }
 
-__global__ void __launch_bounds__(256, 2) k_varemit_df(BatchDev d, int maxS, int smem_bytes, WorkQueue q) {
+template <typename R>
+__global__ void __launch_bounds__(256, 2) k_varemit_groups(BatchDev d, int maxS, int smem_bytes, WorkQueue q) {
     __shared__ int cached;  // instance whose factor tables are in place
     if (threadIdx.x == 0) cached = -1;
     __syncthreads();
     if (!q.counter) {
-        emit_tree(d, cta_block(d), maxS, smem_bytes, cached);
+        emit_tree<R>(d, cta_block(d), maxS, smem_bytes, cached);
         return;
     }
     for (int u = next_unit(q); u >= 0; u = next_unit(q)) {
         const int t1 = imin((u + 1) * q.chunk, d.nblocks);
         for (int t = u * q.chunk; t < t1; t++) {
-            emit_tree(d, d.blkmap ? d.blkmap[t] : t, maxS, smem_bytes, cached);
+            emit_tree<R>(d, d.blkmap ? d.blkmap[t] : t, maxS, smem_bytes, cached);
             __syncthreads();
         }
     }
 }
 
-}  // namespace
-
-void launch_varemit_df(const BatchDev &d, cudaStream_t s, int *queue, int chunk) {
+template <typename R>
+void launch(const BatchDev &d, cudaStream_t s, int *queue, int chunk) {
     const int n = imax(d.maxnodes, 1), S = imax(d.maxS, 1), T = d.maxT;
     constexpr int SM_BYTES = 227 * 1024, STATIC = 4 * 1024;
     auto need = [&](int w) { return tables_bytes(T) + tree_bytes(n, S) + w * (warp_need(n, S, T, 1) + 16); };
@@ -486,20 +543,27 @@ void launch_varemit_df(const BatchDev &d, cudaStream_t s, int *queue, int chunk)
         while (warps > 1 && need(warps) > smem) warps--;
     }
     smem &= ~15;
-    prefer_shared(k_varemit_df);
-    if (!raise_dynamic_smem(k_varemit_df, smem)) return;
+    prefer_shared(k_varemit_groups<R>);
+    if (!raise_dynamic_smem(k_varemit_groups<R>, smem)) return;
     WorkQueue q{queue, d.nblocks, 1};
     int grid = d.nblocks;
     if (queue) {
         // a unit's trees are mostly one instance's, whose factor tables are then made once: up
         // to 8 trees, while the queue still holds several units a CTA
-        grid = persistent_grid(k_varemit_df, 32 * warps, smem, d.nblocks);
+        grid = persistent_grid(k_varemit_groups<R>, 32 * warps, smem, d.nblocks);
         q.chunk = imax(imax(chunk, 1), imin(8, d.nblocks / (8 * grid)));
         q.nunits = (d.nblocks + q.chunk - 1) / q.chunk;
         grid = imin(grid, q.nunits);
     }
-    k_varemit_df<<<grid, 32 * warps, smem, s>>>(d, S, smem, q);
+    k_varemit_groups<R><<<grid, 32 * warps, smem, s>>>(d, S, smem, q);
     note_launch();
+}
+
+}  // namespace
+
+void launch_varemit_groups(const BatchDev &d, bool fp32, cudaStream_t s, int *queue, int chunk) {
+    if (fp32) launch<df>(d, s, queue, chunk);
+    else launch<double>(d, s, queue, chunk);
 }
 
 }  // namespace awg

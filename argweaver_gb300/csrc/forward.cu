@@ -1,4 +1,6 @@
-// K3: the forward pass of the threading HMM, one CTA per instance, column in shared memory.
+// K3: the forward pass of the threading HMM, one CTA per instance, column in shared memory: the
+// dispatch, the dense test step, and the general kernel, for trees of more states (3,072) than
+// the owner threads of forward32.cu (FP32) and chain.cu (FP64) hold.
 //
 // Per column (arghmm_forward_block, sample_thread.cpp:252-295):
 //   fgroups[a] = sum of col1 over states of time a

@@ -18,8 +18,8 @@ void launch_tables(const BatchDev &d, bool want32, cudaStream_t s, int *queue = 
 // K2: emissions of variant columns (Felsenstein pruning); as K1.
 void launch_varemit(const BatchDev &d, bool want32, cudaStream_t s, int *queue = nullptr,
                     int chunk = 1);
-// K2 for an FP32 batch whose variant columns are formed in double-float (BatchDev::vardf).
-void launch_varemit_df(const BatchDev &d, cudaStream_t s, int *queue, int chunk);
+// K2 by groups of columns: FP64, or (fp32) double-float for the FP32 path (BatchDev::vardf).
+void launch_varemit_groups(const BatchDev &d, bool fp32, cudaStream_t s, int *queue, int chunk);
 // Whether K2's carve with FP64 per-state factors and 8-byte scratch fits this largest tree: an
 // FP32 batch then forms its variant columns in double-float.
 bool varemit_full_carve_fits(int maxnodes, int maxS);
@@ -52,7 +52,7 @@ bool launch_forward64(const BatchDev &d, cudaStream_t s, bool table);
 bool launch_backward_chain(const BatchDev &d, bool fp32, cudaStream_t s);
 // K5's second half: the marginals from both tables.
 void launch_posterior(const BatchDev &d, bool fp32, double *bw_out, cudaStream_t s);
-// K4: stochastic traceback, one warp per instance; FP32 with bins32 set: the decomposed draw.
+// K4: stochastic traceback, one CTA per instance; FP32 with bins32 set: the decomposed draw.
 void launch_traceback(const BatchDev &d, bool fp32, cudaStream_t s);
 // K5: backward pass and posterior marginals, behind K3 on one stream.
 void launch_backward(const BatchDev &d, bool fp32, double *bw_out, cudaStream_t s);

@@ -1122,9 +1122,10 @@ __global__ void __launch_bounds__(TAB_THREADS) k_tables_ws(BatchDev d, int want3
 
 // ---------------------------------------------------------------------------------------
 // K2: emissions of variant columns (calc_emissions' non-invariant branch, emit.cpp:822-844)
-// of the FP64 path, and of FP32 batches whose largest tree leaves no room for double-float
-// (about 1,800 states at 259 nodes; the others take emit_df.cu's kernel: 6.28 ms here and
-// 1.26 ms there for 840 trees of 150 to 200 leaves).
+// where the largest tree leaves no room for FP64 or double-float factors by state in 200 KB
+// (about 1,800 states at 259 nodes). That line decides between double-float and FP32 forms, and
+// what the FP64 path takes, so it stays where it was; below it emit_groups.cu's kernel takes
+// all: 6.28 ms here and 1.26 ms there for 840 trees of 150 to 200 leaves.
 //
 // One CTA per local tree. Once per tree: the branch mutation probabilities, the per-state
 // factors of the three split branches (prob_branch, emit.cpp:787-805, FP64), and two level
@@ -1828,7 +1829,7 @@ void launch_varemit_t(const BatchDev &d, cudaStream_t s, int *queue, int chunk) 
 }
 
 void launch_varemit(const BatchDev &d, bool fp32, cudaStream_t s, int *queue, int chunk) {
-    if (fp32 && d.vardf) launch_varemit_df(d, s, queue, chunk);
+    if (fp32 ? d.vardf != 0 : varemit_full_carve_fits(d.maxnodes, d.maxS)) launch_varemit_groups(d, fp32, s, queue, chunk);
     else if (fp32) launch_varemit_t<true>(d, s, queue, chunk);
     else launch_varemit_t<false>(d, s, queue, chunk);
 }

@@ -1,4 +1,4 @@
-"""The FP32 path's variant columns in double-float, at the edges of the groups that a warp carries
+"""Variant columns in FP64 and, on the FP32 path, in double-float, at the edges of the groups that a warp carries
 through a tree at once, against the FP64 path's forward table of the same problem.
 
 Tolerance: the FP32 path's bar is 1e-5 relative to FP64 (columns sum to 1, so the table's 2-norm
@@ -55,3 +55,16 @@ def test_persistent_queue_equals_one_cta_a_tree():
     for p, r in zip(probs, api.run_batch(probs, precision="fp32")):
         one = api.run_batch([p], precision="fp32")[0]
         assert np.array_equal(r.forward, one.forward) and r.loglik == one.loglik
+
+
+@pytest.mark.parametrize("case", [0, 2, 3, 4, 5, 8, 9, 10])
+def test_fp64_columns_in_groups(case):
+    """Against the oracle: FP64 sums in another order over some thousand columns."""
+    import pyoracle
+
+    from argweaver_gb300 import api
+
+    p = _problem(seed=6100 + case, **CASES[case])
+    fw, _ = pyoracle.forward(p)
+    r = api.run_batch([p], precision="fp64")[0]
+    assert np.max(np.abs(r.forward - fw)) <= 1e-10 * np.max(np.abs(fw))
