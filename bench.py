@@ -683,7 +683,7 @@ def main():
                      # (--one-instance 64,100000), 7.26 B per state-cell, scaled to this
                      # step's cells (profiles/forward_traffic_k64_1e5.md)
                      "traffic": FWD_DRAM_BYTES_PER_CELL * cells, "peak_source": src,
-                     "kernel": "forward (k_forward_reg), 4 B of FP32 table written per cell, "
+                     "kernel": "forward (k_forward32), 4 B of FP32 table written per cell, "
                                "timed alone (phases run one after another)"},
         "cpu_baseline": {"value": cpu_v, "unit": UNIT, "cores": os.cpu_count(), "kind": "port",
                          "cpu_model": cpu_model(),
