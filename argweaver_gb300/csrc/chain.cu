@@ -641,14 +641,16 @@ __device__ __forceinline__ void run_chain(const BatchDev &d, const InstDev &I, i
                             }
                         }
                     } else {
-                        // rows in global memory
+                        // rows in global memory: the same terms in the same order (a lane of
+                        // a pair takes every second one)
                         const int a0 = tq[q] - (ks[q] - nb[q]);
                         const F *r = tab.rows + B.t2_0 + ro[q];
                         for (int y = 0; y < cnt[q]; y++) {
-                            const F tmab = FWD ? tmS[(a0 + y) * MAXT + tq[q]] : tmS[tq[q] * MAXT + a0 + y];
-                            const F v = Tab<F>::t2(r[(size_t)y * rst[q]], tmab);
-                            if (y & 1) dd[q] = fma(v, x[y], dd[q]);
-                            else de[q] = fma(v, x[y], de[q]);
+                            const int z = SPLIT * y;
+                            const F tmab = FWD ? tmS[(a0 + z) * MAXT + tq[q]] : tmS[tq[q] * MAXT + a0 + z];
+                            const F v = Tab<F>::t2(r[(size_t)z * rst[q]], tmab);
+                            if (SPLIT == 1 && (y & 1)) dd[q] = fma(v, x[z], dd[q]);
+                            else de[q] = fma(v, x[z], de[q]);
                         }
                     }
                 }
