@@ -39,6 +39,7 @@ struct InstDev {
     int T, internal, minage, nleaves, nnodes, nseqs, seqlen, ntrees;
     int block0;           // first block of this instance in the batch
     int maxS;             // states of its largest local tree (at least 1)
+    int maxM, pad;        // same-branch row entries of its largest local tree (at least 1)
     long long cell0;      // forward-table offset of column 0
     long long col0;       // offset into per-column arrays
     long long seq0;       // offset of the column-major sequences [seqlen][nseqs]

@@ -43,15 +43,16 @@
 
 #include "async_copy.cuh"
 #include "f2.cuh"
+#include "forward32_plan.h"
 #include "kernels.h"
 
 namespace awg {
 
 namespace {
 
-constexpr int NRW = 4;                             // reduction warps
+using namespace fwd32;
+
 constexpr int RBINS = (MAXT - 1 + NRW - 1) / NRW;  // time bins per reduction warp (<= 8)
-constexpr int EDEPTH = 4;                          // columns an emission row is loaded ahead
 constexpr unsigned FULL = 0xffffffffu;
 
 __device__ __forceinline__ void named_sync(int id, int threads) {
@@ -147,49 +148,6 @@ struct LogProd {
     __device__ double value() const { return log(prod) + (double)e * 0.69314718055994530942; }
 };
 
-// The staging buffer of one tree (byte offsets; every part starts on 16 bytes and is copied
-// from the 16-byte boundary below its source). The parts from sinfo on are per state.
-struct StageLayout {
-    int desc, tm, rstay, bptr, sinfo, t2off, perm, inv, gptr, gidx, move, rrow, crow, src, total;
-    __host__ __device__ explicit StageLayout(int maxS) {
-        const int arr = (4 * maxS + 32 + 15) & ~15;
-        desc = 0;  // three descriptors: this tree's, the next one's, the one's after
-        tm = desc + 3 * (int)sizeof(BlockDev);
-        rstay = tm + 4 * MAXT * MAXT;
-        bptr = rstay + 4 * MAXT;
-        sinfo = bptr + 160;
-        t2off = sinfo + 16 * maxS;
-        perm = t2off + arr;
-        inv = perm + arr;
-        gptr = inv + arr;
-        gidx = gptr + arr;
-        move = gidx + arr;
-        rrow = move + ((8 * maxS + 32 + 15) & ~15);
-        crow = rrow + arr;
-        src = crow + arr;
-        total = src + 16;
-    }
-};
-static_assert(sizeof(BlockDev) % 16 == 0, "descriptors are bulk-copied");
-
-// Shared memory of one CTA (byte offsets).
-struct SmemPlan {
-    int stage, t2, t2_bytes, col, red, ring, last, total;
-    __host__ __device__ SmemPlan(int maxS, int maxM, int maxnodes, int t2_bufs, bool staged) {
-        auto up = [](int v) { return (v + 15) & ~15; };
-        stage = 0;
-        t2 = stage + (staged ? StageLayout(maxS).total : StageLayout(maxS).sinfo);
-        t2_bytes = up(4 * maxM + 32);
-        col = t2 + t2_bufs * t2_bytes;
-        // nodes on 16 bytes (up to 3 more slots each); rows end up to MAXT past a node's last
-        red = col + 2 * up(4 * (maxS + 3 * maxnodes + MAXT + 8));
-        // the lanes' positions in groups of up to 8, and a slot for threads without a state
-        ring = red + 8 * (maxS + 32 * 9 * NRW) + 16;
-        last = ring + (EDEPTH + 1) * up(4 * maxS);
-        total = last + up(8 * maxS);
-    }
-};
-
 // a number as a type, for lambdas over unrolled lengths
 template <int N>
 struct Int {
@@ -203,7 +161,7 @@ struct Int {
 // are of like length, and past a thread's first state mostly short. STAGED: per-state tables staged a tree ahead
 // (else read from global memory). NTC: the threads at work, reducers and owners.
 template <int KPT, int ROWS0, int ROWS, bool TAIL, bool STAGED, bool SORT>
-__device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, int qi, int maxM, int t2_bufs, int NTC, V2 nz) {
+__device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, int qi, int t2_bufs, int NTC, V2 nz) {
     extern __shared__ __align__(16) unsigned char dyn_b[];
     constexpr int NP = (KPT + 1) / 2;      // packed pairs of states
     const int maxS = I.maxS;
@@ -213,7 +171,7 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
     const int st = tid - 32 * NRW;
     const bool reducer = tid < 32 * NRW, owner = !reducer, producer = tid == 32 * (NRW - 1);
     const StageLayout SL(maxS);
-    const SmemPlan P(maxS, maxM, d.maxnodes, t2_bufs, STAGED);
+    const SmemPlan P(Sizes{maxS, I.maxM, I.nnodes}, t2_bufs, STAGED);
     unsigned char *const stage = dyn_b + P.stage;
     float *const t2buf = (float *)(dyn_b + P.t2);
     const int colstride = (P.red - P.col) / 8;
@@ -883,22 +841,6 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
     }
 }
 
-// Owner threads of a CTA: 16 warps with the reducers, 4 a sub-partition, leave 128 registers
-// a thread; the wide form for batches with larger trees has 20 warps at 96.
-constexpr int OWNERS = 384, WIDE_OWNERS = 512;
-
-// States per owner thread (1, 2, 3, 4 or 8) for an instance's largest tree; at least `least`. One
-// while the owners suffice: a thread's shared loads are issued one after another, so a column
-// takes 0.47 us at 99 states and 0.67 at 351 with one, 0.64 and 0.78 with two; 1.24 at 789 and
-// 1.30 at 930 with three, 1.48 at 930 with four.
-__host__ __device__ inline int states_per_thread(int maxS, int least, int owners) {
-    const int k = maxS <= owners ? 1 : maxS <= 2 * owners ? 2 : maxS <= 3 * owners ? 3 : maxS <= 4 * owners ? 4 : 8;
-    return imax(k, least);
-}
-__host__ __device__ inline int owner_threads(int maxS, int kpt) {
-    return imax(32, ((maxS + kpt - 1) / kpt + 31) / 32 * 32);
-}
-
 // One CTA per instance, each by its own largest tree: a batch's small instances run as fast as
 // alone. Warps that an instance has no use for leave at once. LONG: more than 21 time points.
 // FEW: batches up to 768 states, without the form of three states a thread (in the same kernel it
@@ -906,51 +848,43 @@ __host__ __device__ inline int owner_threads(int maxS, int kpt) {
 // a column at 704 states); WIDE: more owner warps at fewer registers each.
 enum Forms { FEW, MANY, WIDE };
 template <bool LONG, Forms FORMS>
-__global__ void __launch_bounds__(32 * NRW + (FORMS == WIDE ? WIDE_OWNERS : OWNERS)) k_forward32(BatchDev d, int maxM, int smem, int least, float nzero) {
+__global__ void __launch_bounds__(32 * NRW + (FORMS == WIDE ? WIDE_OWNERS : OWNERS)) k_forward32(BatchDev d, int smem, int least, float nzero) {
     const int qi = cta_instance(d);
     const InstDev I = d.inst[qi];
-    const int kpt = states_per_thread(I.maxS, least, FORMS == WIDE ? WIDE_OWNERS : OWNERS);
-    const int ntc = 32 * NRW + owner_threads(I.maxS, kpt);
+    const Form f = form_of(Sizes{I.maxS, I.maxM, I.nnodes}, smem, LONG, FORMS == WIDE, least);
+    const int ntc = 32 * NRW + f.owners;
     if ((int)threadIdx.x >= ntc) return;
     const V2 nz = pk(nzero, nzero);
-    auto fits = [&](int bufs, bool staged) { return SmemPlan(I.maxS, maxM, d.maxnodes, bufs, staged).total <= smem; };
-    // rows longer than the registers hold (a node spans at most T - 1 times): the tables staged
-    // a tree ahead with two buffers of rows; where they do not fit, only the rows in shared
-    // memory; else neither
     // States are sorted by their node's for more than 21 time points alone: 1.69 us a column
     // unsorted and 1.40 sorted at 1138 states of 32, 0.90 and 0.90 at 704 of 20, 1.30 and 1.32 at
     // 930 (the sort and the scattered stores cost what the shorter dots give).
     constexpr int R4 = FORMS == WIDE ? 4 : 8;
     constexpr int R3 = LONG ? 20 : 8, R40 = LONG ? R4 + 8 : R4;
-    if (kpt == 1) {
-        forward32<1, LONG ? 32 : 20, 2, false, true, false>(d, I, qi, maxM, 1, ntc, nz);
-    } else if (kpt == 2) {
-        if (!LONG) forward32<2, 20, 20, false, true, false>(d, I, qi, maxM, 1, ntc, nz);
-        else if (fits(2, true)) forward32<2, 20, 12, true, true, true>(d, I, qi, maxM, 2, ntc, nz);
-        else forward32<4, R40, R4, true, false, LONG>(d, I, qi, maxM, fits(1, false), ntc, nz);
-    } else if (FORMS != FEW && kpt == 3) {
-        if (fits(2, true)) forward32<3, R3, 8, true, true, LONG>(d, I, qi, maxM, 2, ntc, nz);
-        else forward32<3, R3, 8, true, false, LONG>(d, I, qi, maxM, fits(1, false), ntc, nz);
-    } else if (kpt == 4) {
-        if (FORMS != WIDE && fits(2, true)) forward32<4, R40, R4, true, true, LONG>(d, I, qi, maxM, 2, ntc, nz);
-        else forward32<4, R40, R4, true, false, LONG>(d, I, qi, maxM, fits(1, false), ntc, nz);
+    if (f.kpt == 1) {
+        forward32<1, LONG ? 32 : 20, 2, false, true, false>(d, I, qi, 1, ntc, nz);
+    } else if (f.kpt == 2) {
+        if (!LONG) forward32<2, 20, 20, false, true, false>(d, I, qi, 1, ntc, nz);
+        else forward32<2, 20, 12, true, true, true>(d, I, qi, 2, ntc, nz);
+    } else if (FORMS != FEW && f.kpt == 3) {
+        if (f.staged) forward32<3, R3, 8, true, true, LONG>(d, I, qi, 2, ntc, nz);
+        else forward32<3, R3, 8, true, false, LONG>(d, I, qi, f.bufs, ntc, nz);
+    } else if (f.kpt == 4) {
+        if (FORMS != WIDE && f.staged) forward32<4, R40, R4, true, true, LONG>(d, I, qi, 2, ntc, nz);
+        else forward32<4, R40, R4, true, false, LONG>(d, I, qi, f.bufs, ntc, nz);
     } else {
-        forward32<8, 4, 4, true, false, LONG>(d, I, qi, maxM, fits(1, false), ntc, nz);
+        forward32<8, 4, 4, true, false, LONG>(d, I, qi, f.bufs, ntc, nz);
     }
 }
 
 template <bool LONG, Forms FORMS>
 void launch(const BatchDev &d, cudaStream_t s, int least) {
-    const int maxS = imax(d.maxS, 1), maxM = imax(d.maxM, 1);
-    // shared memory for the most demanding form that fits
-    constexpr int LIMIT = 222 * 1024;  // beside the static part
-    int smem = SmemPlan(maxS, maxM, d.maxnodes, 2, true).total;
-    if (smem > LIMIT) smem = LIMIT;
+    const int maxS = imax(d.maxS, 1);
+    const int smem = launch_bytes(Sizes{maxS, imax(d.maxM, 1), d.maxnodes});
     if (!raise_dynamic_smem(k_forward32<LONG, FORMS>, smem)) return;  // the launch reports it
     // an instance with one state a thread may need every warp
     const int owners = FORMS == WIDE ? WIDE_OWNERS : OWNERS;
     const int nt = 32 * NRW + (maxS <= owners && least <= 1 ? owner_threads(maxS, 1) : owners);
-    k_forward32<LONG, FORMS><<<d.ninst, nt, smem, s>>>(d, maxM, smem, least, -0.0f);
+    k_forward32<LONG, FORMS><<<d.ninst, nt, smem, s>>>(d, smem, least, -0.0f);
     note_launch();
 }
 
@@ -962,7 +896,7 @@ void launch(const BatchDev &d, cudaStream_t s, int least) {
 
 }  // namespace
 
-bool forward_writes_bins(int maxS) { return imax(maxS, 1) <= 8 * OWNERS; }
+bool forward_writes_bins(int maxS) { return imax(maxS, 1) <= MOST_STATES; }
 
 bool launch_forward32(const BatchDev &d, cudaStream_t s, int want_kpt) {
     if (!forward_writes_bins(d.maxS)) return false;

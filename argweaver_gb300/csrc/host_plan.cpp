@@ -390,7 +390,7 @@ bool plan_layout(const awg_problem *probs, int n, HostPlan &plan, std::string &e
         InstDev &I = plan.inst[q];
         I.T = p.ntimes; I.internal = p.internal ? 1 : 0; I.minage = p.minage;
         I.nleaves = nleaves; I.nnodes = p.nnodes; I.nseqs = nemit; I.seqlen = p.seqlen;
-        I.ntrees = p.ntrees; I.block0 = (int)trees; I.maxS = 1;
+        I.ntrees = p.ntrees; I.block0 = (int)trees; I.maxS = I.maxM = 1; I.pad = 0;
         I.cell0 = cell; I.col0 = col; I.seq0 = seq; I.model0 = (long long)q * MODEL_STRIDE;
         model_arrays(p.times, p.popsizes, p.ntimes, p.rho, p.mu, p.infsites_penalty,
                      &plan.model[(size_t)q * MODEL_STRIDE]);
@@ -402,10 +402,11 @@ bool plan_layout(const awg_problem *probs, int n, HostPlan &plan, std::string &e
             t2 += tot[k].t2;
             start += tot[k].cols;
             I.maxS = std::max(I.maxS, tot[k].maxS);
-            plan.maxM = std::max(plan.maxM, tot[k].maxM);
+            I.maxM = std::max(I.maxM, tot[k].maxM);
             plan.maxlen = std::max(plan.maxlen, tot[k].maxlen);
         }
         plan.maxS = std::max(plan.maxS, I.maxS);
+        plan.maxM = std::max(plan.maxM, I.maxM);
         plan.maxnodes = std::max(plan.maxnodes, p.nnodes);
         plan.maxT = std::max(plan.maxT, p.ntimes);
         nodes += (long long)p.ntrees * p.nnodes;

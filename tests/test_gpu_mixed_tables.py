@@ -44,3 +44,19 @@ def test_fp64_small_problems_beside_rows_in_global_memory():
         post = pyoracle.posterior(p, fw, pyoracle.backward(p))
         big = post > 1e-200
         assert np.max(np.abs(r.posterior[big] - post[big]) / post[big]) <= 1e-10
+
+
+@pytest.mark.parametrize("ntimes,k,popsize,rows,small", [(32, 57, 1e7, 42000, (4, 14, 16)), (20, 90, 1e8, 30000, (3, 57, 76))])
+def test_fp32_small_problems_beside_rows_too_long_to_stage(ntimes, k, popsize, rows, small):
+    """FP32 tables within 1e-5 of FP64's, an entry each."""
+    from argweaver_gb300 import api
+
+    probs = [_problem(k, 40, 5, popsize, ntimes)] + [_problem(x, 100, 30 + x, ntimes=ntimes) for x in small]
+    S, M = _sizes(probs[0])
+    assert 1536 < S <= 1850 and M > rows  # no form stages these rows twice in 222 KB
+    batch = api.run_batch(probs, precision="fp32")
+    for p, r, w in zip(probs, batch, api.run_batch(probs)):
+        one = api.run_batch([p], precision="fp32")[0]
+        assert np.array_equal(r.forward, one.forward) and r.loglik == one.loglik
+        assert np.max(np.abs(r.forward - w.forward)) <= 1e-5
+        assert abs(r.loglik - w.loglik) <= 1e-6 * abs(w.loglik)
