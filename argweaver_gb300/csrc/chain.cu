@@ -609,7 +609,12 @@ __device__ __forceinline__ void run_chain(const BatchDev &d, const InstDev &I, i
             passed(abs);
             const int step = FWD ? 1 : -1;
             if (len > 1) load_next(abs + step);
-            if (len == 1) publish_last();
+            if (len == 1) {
+                // other owners may still read the later tree's low parts for their first column
+                // (a longer tree has its columns' barriers in between)
+                if (pairs) named_sync(3, NTS);
+                publish_last();
+            }
             Scale<F> sc;
             for (int n = 1; n < len; n++) {
                 abs += step;

@@ -57,3 +57,17 @@ def test_chain_mixed_sizes_equal_alone():
         one = api.run_batch([p], want_posterior=True)[0]
         assert np.array_equal(r.forward, one.forward) and r.loglik == one.loglik
         assert np.array_equal(r.posterior, one.posterior)
+
+
+@pytest.mark.parametrize("k,columns", [(12, 300), (60, 200), (110, 120)])
+def test_fp32_marginals_through_one_column_trees(k, columns):
+    """Trees of one column end where they begin: their low parts replace the later tree's only once
+    every owner has read those. The same marginals on every run, within 1e-5 of FP64's."""
+    from argweaver_gb300 import api
+
+    p = _problem(k, columns, 20, 31 + k, rho=2e-6)
+    assert np.mean(p.blocklens == 1) > 0.5
+    want = api.posterior(p)
+    runs = [api.posterior(p, precision="fp32") for _ in range(5)]
+    assert np.max(np.abs(runs[0] - want)) <= 1e-5
+    assert all(np.array_equal(r, runs[0]) for r in runs[1:])

@@ -60,3 +60,14 @@ def test_fp32_small_problems_beside_rows_too_long_to_stage(ntimes, k, popsize, r
         assert np.array_equal(r.forward, one.forward) and r.loglik == one.loglik
         assert np.max(np.abs(r.forward - w.forward)) <= 1e-5
         assert abs(r.loglik - w.loglik) <= 1e-6 * abs(w.loglik)
+
+
+def test_fp32_marginals_beside_rows_in_global_memory():
+    from argweaver_gb300 import api
+
+    probs = [_problem(57, 40, 5, 1e7)] + [_problem(x, 100, 30 + x) for x in (4, 14, 16)]
+    S, M = _sizes(probs[0])
+    assert 4 * M > 190 * 1024  # beside columns and slots, past the 200 KB of a launch
+    for p, r in zip(probs, api.run_batch(probs, precision="fp32", want_forward=False, want_posterior=True)):
+        assert np.array_equal(r.posterior, api.posterior(p, precision="fp32"))
+        assert np.max(np.abs(r.posterior - api.posterior(p))) <= 1e-5
