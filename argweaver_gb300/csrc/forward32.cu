@@ -185,11 +185,13 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
     float2 *const last = (float2 *)(dyn_b + P.last);  // a tree's last column, high and low parts
     __shared__ __align__(16) float tfp[32][NRW];   // [a][reducer] shares of tf; [31]: of the norm
     __shared__ uint64_t full;                      // the staged tree has landed
+    __shared__ uint64_t rows_full;                 // the tree's rows have (unstaged forms)
     __shared__ int by_m[MAXT];                     // states by their node's, then where they begin
     __shared__ double lnl0;
 
     if (tid == 0) {
         mbar_init(&full, 1);
+        mbar_init(&rows_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     // rows read past a node's states, times 0: finite
@@ -253,8 +255,8 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
     double extra = 0.0;
     float mynorm = 1.0f;
     int ncols = 0;
-    unsigned phase = 0;
-    bool failed = false;
+    unsigned phase = 0, rows_phase = 0;
+    bool failed = false, rows_late = false;
 
     // ---- owners: the coming tree's classes (lane l: columns l and 32 + l), loaded a tree
     // ahead; columns past the instance read as invariant
@@ -289,11 +291,18 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
         const bool landed = mbar_wait(&full, phase);
         phase ^= 1u;
         // T1: the last tree's column is final, the staged tree has landed
-        if (named_or(4, NTC, !landed)) {
+        if (named_or(4, NTC, !landed || rows_late)) {
             failed = true;
             break;
         }
         const BlockDev *Bs = desc_of(bi);
+        if (TAIL && !STAGED && producer && t2_bufs && Bs->S > 0) {
+            // the last tree's rows are read: this one's by bulk copy (loaded and stored by the
+            // owners, 49,000 cycles of a tree with 30,000 entries went there)
+            const Rounded<4> r2(d.t2d32 + Bs->t2_0, Bs->M);
+            mbar_expect_tx(&rows_full, r2.bytes);
+            bulk_g2s(t2buf, r2.a16, r2.bytes, &rows_full);
+        }
         const int S = uniform(Bs->S), len = uniform(Bs->len), start = uniform(Bs->start);
         float *const fw = d.fw32 + Bs->cell0;
 
@@ -359,9 +368,6 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
             const float *rows = d.t2d32 + Bs->t2_0;
             if constexpr (STAGED) {
                 rows = (const float *)(dyn_b + P.t2 + (TAIL ? (bi & 1) * P.t2_bytes : 0)) + ((uintptr_t)rows & 15) / 4;
-            } else if (TAIL && t2_bufs) {
-                const int M = Bs->M;
-                for (int x = st; x < M; x += NTS) t2buf[x] = rows[x];  // tails: read after T2
             }
             // classes: bit j of vm / mm: column i + j is variant / masked (i = 0 here)
             unsigned long long vm = (unsigned long long)__ballot_sync(FULL, cw1 == COL_VARIANT) << 32 |
@@ -446,7 +452,11 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
             // where a thread's states lie in an array of all, from `own` on
             const int own = SORT ? 0 : st;
             auto at = [&](int q) { return SORT ? ks[q] : q * NTS; };
-            const float *tails = STAGED || !t2_bufs ? rows : t2buf;
+            if (TAIL && !STAGED && t2_bufs) {
+                rows_late |= !mbar_wait(&rows_full, rows_phase);
+                rows_phase ^= 1u;
+                rows = t2buf + ((uintptr_t)rows & 15) / 4;
+            }
             each_row([&](int q, auto &into, auto n) {
                 const float *r = rows + roff[q];
 #pragma unroll
@@ -608,7 +618,7 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
 #pragma unroll
                     for (int q = 0; q < KPT; q++) {
                         for (int y = q ? ROWS : ROWS0; y < mostq[q]; y += 4) {
-                            const float *r = tails + roff[q] + y * m[q];
+                            const float *r = rows + roff[q] + y * m[q];
                             float v[4];
 #pragma unroll
                             for (int u = 0; u < 4; u++) v[u] = y + u < m[q] ? r[u * m[q]] : 0.0f;
@@ -825,6 +835,10 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
             }
             if (tid == 32) extra += blkx;
         }
+    }
+    if (rows_late) {
+        report_error(d.err, ERR_WAIT_LIMIT, qi, -1, -1);
+        mbar_wait(&rows_full, rows_phase ^ 1u);  // the copy in flight, before the memory is released
     }
     if (failed && tid == 0) {
         report_error(d.err, ERR_WAIT_LIMIT, qi, -1, -1);
