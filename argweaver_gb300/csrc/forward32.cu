@@ -164,6 +164,12 @@ template <int KPT, int ROWS0, int ROWS, bool TAIL, bool STAGED, bool SORT>
 __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, int qi, int t2_bufs, int NTC, V2 nz) {
     extern __shared__ __align__(16) unsigned char dyn_b[];
     constexpr int NP = (KPT + 1) / 2;      // packed pairs of states
+    // rows' ends, past the registers: stepped through by pointers, two states side by side where
+    // a thread has four or eight, for more than 21 time points (rows of up to 31 entries) and for
+    // eight states a thread (four registers a row). A column of 1,243 states with rows of 29
+    // entries takes 3.7 us so and 4.9 one after another, of 2,520 with 12 5.7 and 9.2; with the
+    // shorter rows of up to 21 points (1,442 states of 7) 2.6 and 2.1.
+    constexpr bool LONG_ENDS = SORT || KPT == 8;
     const int maxS = I.maxS;
     const int NB = I.T - 1;
     const int tid = threadIdx.x, lane = tid & 31, rw = tid >> 5;
@@ -614,7 +620,7 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                     }
                     dot2[q] = sum;
                 });
-                if (TAIL && most > (ROWS < ROWS0 ? ROWS : ROWS0)) {
+                if (TAIL && !LONG_ENDS && most > ROWS) {
 #pragma unroll
                     for (int q = 0; q < KPT; q++) {
                         for (int y = q ? ROWS : ROWS0; y < mostq[q]; y += 4) {
@@ -625,6 +631,42 @@ __device__ __forceinline__ void forward32(const BatchDev &d, const InstDev &I, i
                             const float4 n = *(const float4 *)(col + cur + nbo[q] + y);
                             dot2[q] = fma2(pk(v[0], v[1]), pk(n.x, n.y), dot2[q]);
                             dot2[q] = fma2(pk(v[2], v[3]), pk(n.z, n.w), dot2[q]);
+                        }
+                    }
+                }
+                if (TAIL && LONG_ENDS && most > ROWS) {
+                    // W states side by side
+                    constexpr int W = KPT % 4 == 0 ? 2 : 1;
+#pragma unroll
+                    for (int q0 = 0; q0 < KPT; q0 += W) {
+                        const float *r[W], *nb[W];
+                        int left[W], end = 0;
+#pragma unroll
+                        for (int w = 0; w < W; w++) {
+                            const int q = q0 + w, y = q ? ROWS : ROWS0;
+                            r[w] = rows + roff[q] + y * m[q];
+                            nb[w] = col + cur + nbo[q] + y;
+                            left[w] = m[q] - y;
+                            end = imax(end, mostq[q] - y);
+                        }
+                        for (int y = 0; y < end; y += 4) {
+                            float v[W][4];
+                            float4 n[W];
+#pragma unroll
+                            for (int w = 0; w < W; w++) {
+#pragma unroll
+                                for (int u = 0; u < 4; u++) v[w][u] = u < left[w] ? r[w][u * m[q0 + w]] : 0.0f;
+                                n[w] = *(const float4 *)(left[w] > 0 ? nb[w] : col);
+                                r[w] += 4 * m[q0 + w];
+                                nb[w] += 4;
+                                left[w] -= 4;
+                            }
+#pragma unroll
+                            for (int w = 0; w < W; w++) {
+                                V2 &dq = dot2[q0 + w];
+                                dq = fma2(pk(v[w][0], v[w][1]), pk(n[w].x, n[w].y), dq);
+                                dq = fma2(pk(v[w][2], v[w][3]), pk(n[w].z, n[w].w), dq);
+                            }
                         }
                     }
                 }
@@ -872,8 +914,8 @@ __global__ void __launch_bounds__(32 * NRW + (FORMS == WIDE ? WIDE_OWNERS : OWNE
     // States are sorted by their node's for more than 21 time points alone: 1.69 us a column
     // unsorted and 1.40 sorted at 1138 states of 32, 0.90 and 0.90 at 704 of 20, 1.30 and 1.32 at
     // 930 (the sort and the scattered stores cost what the shorter dots give).
-    constexpr int R4 = FORMS == WIDE ? 4 : 8;
-    constexpr int R3 = LONG ? 20 : 8, R40 = LONG ? R4 + 8 : R4;
+    constexpr int R4 = FORMS == WIDE || LONG ? 4 : 8;
+    constexpr int R3 = LONG ? 20 : 8, R40 = LONG ? 12 : R4;
     if (f.kpt == 1) {
         forward32<1, LONG ? 32 : 20, 2, false, true, false>(d, I, qi, 1, ntc, nz);
     } else if (f.kpt == 2) {

@@ -25,3 +25,19 @@ def test_fp32_rows_not_staged(k, popsize, ntimes):
     a = api.run_batch([p], precision="fp32")[0]
     assert np.max(np.abs(a.forward - fw)) <= 1e-5
     assert abs(a.loglik - lnl) <= 1e-6 * abs(lnl)
+
+
+@pytest.mark.parametrize("k,popsize,ntimes", [(30, 1e6, 32), (40, 1e7, 32), (50, 1e6, 32), (60, 1e6, 24), (160, 1e5, 32),
+                                              (90, 1e7, 20), (160, 1e7, 20)])
+def test_fp32_rows_past_the_registers_in_one_tree(k, popsize, ntimes):
+    import pyoracle
+
+    from argweaver_gb300 import api
+    from argweaver_gb300.sim import simulate
+
+    p = simulate(k - 1, 70, 300 + k, compress=10, ntimes=ntimes, popsize=popsize, missing=0.005, rho=1e-14)
+    assert p.ntrees == 1
+    fw, lnl = pyoracle.forward(p)
+    a = api.run_batch([p], precision="fp32")[0]
+    assert np.max(np.abs(a.forward - fw)) <= 1e-5
+    assert abs(a.loglik - lnl) <= 1e-6 * abs(lnl)
