@@ -75,6 +75,7 @@ struct Ctx {
     // the last batch's device view, for draws from its resident forward tables
     BatchDev d{};
     bool have_d = false, d_fp32 = false;
+    bool normalised = false;             // the FP64 table has been, for the caller
     size_t o_u = 0;
 };
 
@@ -500,6 +501,10 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
             sz = std::min(2 * sz, std::max(cap, sz));
         }
     }
+    // FP64 tables are normalised last, for the caller: paths and marginals come from the columns as
+    // the chain leaves them, whether or not some problem of the batch wants its table
+    const bool normalise = !fp32 && want_fw && !opt.dense;
+    C.normalised = normalise;
     int *qk = cfg.persistent ? queues : nullptr;
     auto qp = [&](int i) { return qk ? qk + i : nullptr; };
     // the device part of the step (no host synchronisation: it is also what is captured)
@@ -549,13 +554,15 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
                 EQ(cudaEventRecord(C.gev[2 * g], s));
                 EQ(cudaStreamWaitEvent(gs, C.gev[2 * g], 0));
                 EQ(fork_backward(dg, gs, g));
-                launch_forward(dg, fp32, gs, cfg.kpt, want_fw);
+                launch_forward(dg, fp32, gs, cfg.kpt);
                 EQ(cudaGetLastError());
                 if (want_path) {
                     launch_traceback(dg, fp32, gs);
                     EQ(cudaGetLastError());
                 }
                 EQ(join_backward(dg, gs, g));
+                if (normalise) launch_normalise(dg, gs);
+                EQ(cudaGetLastError());
                 EQ(cudaEventRecord(C.gev[2 * g + 1], gs));
             }
             for (int g = 0; g < ng; g++) EQ(cudaStreamWaitEvent(s, C.gev[2 * g + 1], 0));
@@ -565,13 +572,15 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
             launch_varemit(d, fp32, s, qp(1), cfg.chunk);
             EQ(cudaGetLastError());
             EQ(fork_backward(d, s, 0));
-            launch_forward(d, fp32, s, cfg.kpt, want_fw);
+            launch_forward(d, fp32, s, cfg.kpt);
             EQ(cudaGetLastError());
             if (want_path) {
                 launch_traceback(d, fp32, s);
                 EQ(cudaGetLastError());
             }
             EQ(join_backward(d, s, 0));
+            if (normalise) launch_normalise(d, s);
+            EQ(cudaGetLastError());
         }
 #undef EQ
         return cudaSuccess;
@@ -701,7 +710,7 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         CKL("emission kernel");
         if (T) CK(cudaEventRecord(C.ev[3], s));
         if (opt.dense) launch_forward_dense(d, s);
-        else launch_forward(d, fp32, s, cfg.kpt, want_fw);
+        else launch_forward(d, fp32, s, cfg.kpt);
         CKL("forward kernel");
         if (T) CK(cudaEventRecord(C.ev[4], s));
         if (want_path) {
@@ -712,6 +721,10 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         if (want_post) {
             launch_backward(d, fp32, want_bw ? (double *)(D + o_bw) : nullptr, s);
             CKL("backward kernel");
+        }
+        if (normalise) {
+            launch_normalise(d, s);
+            CKL("normalisation kernel");
         }
         if (T) CK(cudaEventRecord(C.ev[6], s));
     }
@@ -938,6 +951,11 @@ int ctx_resample(Ctx *C, const double *const *uniforms, int *const *paths, std::
     CK(cudaMemcpyAsync((void *)C->d.uniforms, u, sizeof(double) * std::max(plan.total_cols, 1LL),
                        cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(C->d.err, 0, 4 * sizeof(int), s));
+    if (C->normalised) {  // back to the columns that paths are drawn from, once
+        launch_forward(C->d, C->d_fp32, s);
+        CK(cudaGetLastError());
+        C->normalised = false;
+    }
     launch_traceback(C->d, C->d_fp32, s);
     CK(cudaGetLastError());
     C->copies.clear();

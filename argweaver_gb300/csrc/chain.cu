@@ -906,13 +906,12 @@ bool launch(const BatchDev &d, cudaStream_t s) {
 
 }  // namespace
 
-bool launch_forward64(const BatchDev &d, cudaStream_t s, bool table) {
-    if (!launch<double, true>(d, s)) return false;
-    if (table) {
-        k_normalise<<<dim3(d.nblocks, column_shares(d)), 128, 0, s>>>(d);
-        note_launch();
-    }
-    return true;
+bool launch_forward64(const BatchDev &d, cudaStream_t s) { return launch<double, true>(d, s); }
+
+void launch_normalise(const BatchDev &d, cudaStream_t s) {
+    if (imax(d.maxS, 1) > 8 * OWNERS) return;  // the general kernel's columns are already
+    k_normalise<<<dim3(d.nblocks, column_shares(d)), 128, 0, s>>>(d);
+    note_launch();
 }
 
 bool launch_backward_chain(const BatchDev &d, bool fp32, cudaStream_t s) {

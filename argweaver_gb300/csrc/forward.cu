@@ -535,8 +535,8 @@ void launch_forward_dense(const BatchDev &d, cudaStream_t s) {
     note_launch();
 }
 
-void launch_forward(const BatchDev &d, bool fp32, cudaStream_t s, int kpt, bool table) {
-    if (fp32 ? launch_forward32(d, s, kpt) : launch_forward64(d, s, table)) return;
+void launch_forward(const BatchDev &d, bool fp32, cudaStream_t s, int kpt) {
+    if (fp32 ? launch_forward32(d, s, kpt) : launch_forward64(d, s)) return;
     if (fp32) launch_old<float>(d, d.maxM, s);
     else launch_old<double>(d, d.maxM, s);
 }

@@ -24,10 +24,12 @@ void launch_varemit_groups(const BatchDev &d, bool fp32, cudaStream_t s, int *qu
 // FP32 batch then forms its variant columns in double-float.
 bool varemit_full_carve_fits(int maxnodes, int maxS);
 // K3: forward pass, one CTA per instance; kpt: at least this many states per owner thread of
-// the FP32 kernel (0: chosen by the state count). table: the FP64 table is to be read, so its
-// columns are normalised (else each is left on a power-of-two scale of its own, which the
-// traceback and the posterior do not see).
-void launch_forward(const BatchDev &d, bool fp32, cudaStream_t s, int kpt = 0, bool table = true);
+// the FP32 kernel (0: chosen by the state count). FP64 columns are left on power-of-two scales of
+// their own, which is how the traceback and the posterior read them, whatever else is wanted.
+void launch_forward(const BatchDev &d, bool fp32, cudaStream_t s, int kpt = 0);
+// The FP64 table's columns divided by their sums, as the reference's table has them: behind
+// everything that reads the columns, where the table itself is wanted.
+void launch_normalise(const BatchDev &d, cudaStream_t s);
 // K3 with the reference's dense test step (arghmm_forward_block_slow), FP64.
 void launch_forward_dense(const BatchDev &d, cudaStream_t s);
 
@@ -46,7 +48,7 @@ bool forward_writes_bins(int maxS);
 // The forms of K3 and K5 for trees that a CTA's owner threads hold (else false: nothing
 // launched).
 bool launch_forward32(const BatchDev &d, cudaStream_t s, int kpt);
-bool launch_forward64(const BatchDev &d, cudaStream_t s, bool table);
+bool launch_forward64(const BatchDev &d, cudaStream_t s);
 // K5's first half: the backward table into d.post. It reads nothing that K3 writes, so the two
 // passes may run side by side.
 bool launch_backward_chain(const BatchDev &d, bool fp32, cudaStream_t s);

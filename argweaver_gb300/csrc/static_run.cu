@@ -226,6 +226,8 @@ int run_static(const awg_problem *p, awg_outputs *out, int precision, cudaStream
     SCK(cudaGetLastError());
     launch_forward(d, fp32, s);
     SCK(cudaGetLastError());
+    if (!fp32) launch_normalise(d, s);
+    SCK(cudaGetLastError());
 
     const long long cells = plan.total_cells;
     if (out->forward)
