@@ -101,8 +101,7 @@ struct BatchDev {
     double *inv_lk;              // [total states] invariant-site emission per state
     int *determ;                 // [total states] switch: target of state j of prev tree
     double *determprob;          // [total states]; FP32 path: once a tree's table is built, a
-                                 // slot's first float holds the move as a complement, 1 - p,
-                                 // when p >= 1/2, else -p (sign bit set)
+                                 // slot's first float holds the move (fp32_move)
     int2 *srcs;                  // [nblocks] {recombsrc, recoalsrc}
     double *recombrow, *recoalrow;  // [total states] dense rows over this block's states
     int *gptr;                   // [total states + nblocks] gather CSR pointers
@@ -162,6 +161,14 @@ __device__ inline void report_error(int *err, int code, int inst, int blk, int c
     }
 }
 #endif
+
+// A deterministic switch move of probability p as the FP32 steps read it (f2_move): its complement
+// 1 - p for p >= 1/2, else -p, told apart by the sign bit. A product that rounds above 1 has the
+// complement +0: a negative one would read as a probability near 0.
+AWG_HD inline float fp32_move(double p) {
+    const float c = (float)(1.0 - p);
+    return p >= 0.5 ? (c > 0.0f ? c : 0.0f) : -(float)p;
+}
 
 AWG_HD inline int imax(int a, int b) { return a > b ? a : b; }
 AWG_HD inline int imin(int a, int b) { return a < b ? a : b; }

@@ -1094,8 +1094,7 @@ __device__ __forceinline__ void tables_tree(const BatchDev &d, int blk, int want
         for (int j = tid; j < imax(S1, 1); j += blockDim.x) {
             const double pj = determprob[j];
             d.determprob32[B.prev_state0 + j] = (float)pj;
-            // the slot then holds the move as the FP32 steps apply it (BatchDev::determprob)
-            *(float *)(determprob + j) = pj >= 0.5 ? (float)(1.0 - pj) : -(float)pj;
+            *(float *)(determprob + j) = fp32_move(pj);  // (BatchDev::determprob)
         }
         for (int k = tid; k < Sm; k += blockDim.x) {
             d.recombrow32[B.state0 + k] = (float)recombrow[k];
