@@ -74,10 +74,11 @@ template <> struct Fmt<float> {
     __device__ static int expo(float x) { return (__float_as_int(x) >> 23) & 0xff; }
     __device__ static float pow2(int k) { return __int_as_float((k + 127) << 23); }
 };
-// 1023 - E (127 - E), the power that brings the largest exponent to 0; 0 for an empty column
+// 1023 - E (127 - E), the power that brings the largest exponent to 0 (to 1 from the format's last
+// one, whose power would not be a normal number); 0 for an empty column
 template <typename F>
 __device__ __forceinline__ int rescale(int E) {
-    return E == 0 || E == Fmt<F>::top ? 0 : imin(Fmt<F>::bias - E, Fmt<F>::bias - 1);
+    return E == 0 || E == Fmt<F>::top ? 0 : imax(imin(Fmt<F>::bias - E, Fmt<F>::bias - 1), 1 - Fmt<F>::bias);
 }
 
 template <typename F> struct Tab;
@@ -574,7 +575,7 @@ __device__ __forceinline__ void run_chain(const BatchDev &d, const InstDev &I, i
                         F s = sums[q];
                         if (src.x != -1 && rr[q] > F(0)) s += prev[src.x] * rr[q];
                         if (src.y != -1 && cr[q] > F(0)) s += prev[src.y] * cr[q];
-                        s *= factor(abs, q, ek);
+                        s = s * Fmt<F>::pow2(ek) * factor(abs, q, 0);
                         outf[k] = s;
                         cur[k] = base_f[slot[q]] = x_own[q] = s;
                     } else {
@@ -673,10 +674,16 @@ __device__ __forceinline__ void run_chain(const BatchDev &d, const InstDev &I, i
                 const int E = imax(imax(expoS[0], expoS[1]), imax(expoS[2], expoS[3]));
                 sc.see(E);
                 if (!pairs && sc.extra) {  // rare
+                    // (forward: on the values, as a given prior's may be too large for the factor)
+                    const F x = Fmt<F>::pow2(sc.extra);
 #pragma unroll
                     for (int q = 0; q < KPT; q++) {
-                        fac[q] *= Fmt<F>::pow2(sc.extra);
-                        if (FWD) de[q] *= Fmt<F>::pow2(sc.extra);
+                        if constexpr (FWD) {
+                            de[q] = fma(tfS[tq[q]] * x, fac[q], de[q] * x);
+                            fac[q] = F(0);
+                        } else {
+                            fac[q] *= x;
+                        }
                     }
                 }
 #pragma unroll
