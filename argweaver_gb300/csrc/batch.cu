@@ -39,7 +39,8 @@ struct Ctx {
     cudaStream_t stream = nullptr;       // uploads, per-tree kernels, downloads
     cudaStream_t gstream[MAXG] = {};     // per group: forward, traceback, backward (high
                                          // priority, so their CTAs are placed first)
-    cudaStream_t bstream[MAXG] = {};     // per group: the backward pass beside the forward
+    cudaStream_t bstream[MAXG] = {};     // per group: the backward pass beside the forward (made
+                                         // with bev for the first batch that wants marginals)
     char *dev = nullptr;
     size_t dev_cap = 0;
     char *host = nullptr;                // inputs staging (page-locked)
@@ -50,7 +51,7 @@ struct Ctx {
     size_t hout_cap = 0;
     cudaEvent_t ev[8];
     cudaEvent_t gev[2 * MAXG + 2];
-    cudaEvent_t bev[2 * MAXG];           // per group: tables made, backward pass done
+    cudaEvent_t bev[2 * MAXG] = {};      // per group: tables made, backward pass done
     cudaEvent_t done = nullptr;          // end of the last batch's downloads
     Timings last;
     // the captured step of the last batch (kernels, memsets, cross-stream events) and the
@@ -237,17 +238,21 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         CK(cudaStreamCreateWithFlags(&C.stream, cudaStreamNonBlocking));
         int lo = 0, hi = 0;
         CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-        for (int g = 0; g < MAXG; g++) {
+        for (int g = 0; g < MAXG; g++)
             CK(cudaStreamCreateWithPriority(&C.gstream[g], cudaStreamNonBlocking, hi));
-            CK(cudaStreamCreateWithPriority(&C.bstream[g], cudaStreamNonBlocking, hi));
-        }
         for (int i = 0; i < 8; i++) CK(cudaEventCreate(&C.ev[i]));
         for (int i = 0; i < 2 * MAXG + 2; i++)
             CK(cudaEventCreateWithFlags(&C.gev[i], cudaEventDisableTiming));
-        for (int i = 0; i < 2 * MAXG; i++)
-            CK(cudaEventCreateWithFlags(&C.bev[i], cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&C.done, cudaEventDisableTiming));
         C.init = true;
+    }
+    if (!dry && want_post && !C.bev[2 * MAXG - 1]) {
+        int lo = 0, hi = 0;
+        CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+        for (int g = 0; g < MAXG; g++)
+            if (!C.bstream[g]) CK(cudaStreamCreateWithPriority(&C.bstream[g], cudaStreamNonBlocking, hi));
+        for (int i = 0; i < 2 * MAXG; i++)
+            if (!C.bev[i]) CK(cudaEventCreateWithFlags(&C.bev[i], cudaEventDisableTiming));
     }
     cudaStream_t s = C.stream;
 
@@ -870,12 +875,13 @@ void ctx_destroy(Ctx *C) {
         if (C->gexec) cudaGraphExecDestroy(C->gexec);
         for (int g = 0; g < MAXG; g++) {
             cudaStreamDestroy(C->gstream[g]);
-            cudaStreamDestroy(C->bstream[g]);
+            if (C->bstream[g]) cudaStreamDestroy(C->bstream[g]);
         }
         cudaStreamDestroy(C->stream);
         for (int i = 0; i < 8; i++) cudaEventDestroy(C->ev[i]);
         for (int i = 0; i < 2 * MAXG + 2; i++) cudaEventDestroy(C->gev[i]);
-        for (int i = 0; i < 2 * MAXG; i++) cudaEventDestroy(C->bev[i]);
+        for (int i = 0; i < 2 * MAXG; i++)
+            if (C->bev[i]) cudaEventDestroy(C->bev[i]);
         cudaEventDestroy(C->done);
     }
     if (C->dev) cudaFree(C->dev);
@@ -899,7 +905,7 @@ void ctx_sync(Ctx *C) {
     cudaStreamSynchronize(C->stream);
     for (int g = 0; g < MAXG; g++) {
         cudaStreamSynchronize(C->gstream[g]);
-        cudaStreamSynchronize(C->bstream[g]);
+        if (C->bstream[g]) cudaStreamSynchronize(C->bstream[g]);
     }
 }
 

@@ -52,3 +52,16 @@ def test_resampling_behind_a_wanted_table():
         for u, w in zip(us[1:], want[1:]):
             assert np.array_equal(srv.resample(t, u), w)
         srv.release(t)
+
+
+@pytest.mark.parametrize("n", [2, 18])
+def test_marginals_wanted_later_in_a_context(n):
+    """A context's first batch wants none (nothing is made for them), a later one does."""
+    probs, u = _batch(n)
+    want = api.run_batch(probs, precision="fp32", want_forward=False, want_path=True, want_posterior=True, uniforms=u)
+    with api.BatchContext() as c:
+        for post in (False, True, False, True):
+            c.launch(probs, precision="fp32", want_posterior=post, uniforms=u)
+            for r, w in zip(c.finish(), want):
+                assert np.array_equal(r.path, w.path)
+                assert not post or np.array_equal(r.posterior, w.posterior)
