@@ -187,8 +187,16 @@ bool raise_dynamic_smem_fn(const void *kernel, size_t bytes) {
     return true;
 }
 
-// Plans, uploads and enqueues one batch on context C. Synchronous (async false): outputs go
-// straight to the caller's buffers and the call returns when they are there. Asynchronous:
+// Copies from the context's output staging to the callers' buffers.
+static void hand_over(const Ctx &C, const std::vector<Ctx::Copy> &out) {
+    std::vector<HostCopy> copies;
+    for (const Ctx::Copy &c : out) copies.push_back({c.dst, C.hout + c.off, c.bytes});
+    parallel_copy(copies);
+}
+
+// Plans, uploads and enqueues one batch on context C. Synchronous (async false): tables go
+// straight to the caller's buffers, several problems' paths and log-likelihoods through C's
+// page-locked staging, and the call returns when they are there. Asynchronous:
 // outputs go to C's page-locked staging, C.done marks their arrival, and ctx_complete (on
 // the same thread, before C's next batch) checks the device error record and hands them
 // over. timing: 0 off, 1 one compute time, 2 kernels one phase after another. Returns 0,
@@ -748,10 +756,14 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         size_t bytes;
     };
     std::vector<Pending> pend;
-    // several problems' paths and log-likelihoods lie side by side on the device: two copies to
-    // page-locked staging, handed over by ctx_complete (a copy to pageable memory each took 20 ms
-    // for 256 problems of 58,000 columns). A path of 256 MB and more goes as it is.
-    const bool packed = !async && n > 1 && sizeof(int) * COLS <= ((size_t)256 << 20);
+    // several problems' paths and log-likelihoods lie side by side on the device: few copies to
+    // page-locked staging, handed over from there (a copy to pageable memory each took 20 ms for
+    // 256 problems of 58,000 columns). Paths go in pieces through two buffers, a piece to the
+    // callers while the next ones are on their way.
+    const bool packed = !async && n > 1;
+    constexpr size_t PIECE = (size_t)32 << 20;
+    const size_t path_bytes = packed && want_path ? sizeof(int) * COLS : 0;
+    const int pieces = (int)((path_bytes + PIECE - 1) / PIECE);
     for (int q = 0; q < n; q++) {
         const InstDev &I = plan.inst[q];
         const long long cells = (q + 1 < n ? plan.inst[q + 1].cell0 : plan.total_cells) - I.cell0;
@@ -769,14 +781,22 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
         for (const Pending &pd : pend) C.copies.push_back({pd.dst, out_slot(pd.bytes), pd.bytes});
     }
     size_t lnl_at = 0, path_at = 0;
+    // the callers' parts of piece k
+    auto piece = [&](int k, std::vector<Ctx::Copy> &out) {
+        const size_t lo = k * PIECE, hi = std::min(lo + PIECE, path_bytes);
+        for (int q = 0; q < n; q++) {
+            const size_t p0 = sizeof(int) * plan.inst[q].col0, p1 = p0 + sizeof(int) * plan.inst[q].seqlen;
+            const size_t x0 = std::max(p0, lo), x1 = std::min(p1, hi);
+            if (outs[q].path && x0 < x1)
+                out.push_back({(char *)outs[q].path + (x0 - p0), path_at + (k & 1) * PIECE + (x0 - lo), x1 - x0});
+        }
+    };
     if (packed) {
         lnl_at = out_slot(sizeof(double) * n);
-        path_at = out_slot(want_path ? sizeof(int) * COLS : 0);
-        for (int q = 0; q < n; q++) {
-            const InstDev &I = plan.inst[q];
+        path_at = out_slot(std::min(path_bytes, 2 * PIECE));
+        for (int q = 0; q < n; q++)
             if (outs[q].loglik) C.copies.push_back({outs[q].loglik, lnl_at + sizeof(double) * q, sizeof(double)});
-            if (outs[q].path) C.copies.push_back({outs[q].path, path_at + sizeof(int) * I.col0, sizeof(int) * I.seqlen});
-        }
+        for (int k = std::max(pieces - 2, 0); k < pieces; k++) piece(k, C.copies);  // by ctx_complete
     }
     C.err_off = out_slot(4 * sizeof(int));
     if (hout_bytes > C.hout_cap) {
@@ -790,10 +810,19 @@ int ctx_launch(Ctx &C, const awg_problem *probs, awg_outputs *outs, int n, const
     for (size_t i = 0; i < pend.size(); i++)
         CK(cudaMemcpyAsync(async ? (void *)(C.hout + C.copies[i].off) : pend[i].dst, pend[i].src,
                            pend[i].bytes, cudaMemcpyDeviceToHost, s));
-    if (packed) {
-        CK(cudaMemcpyAsync(C.hout + lnl_at, d.lnl, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-        if (want_path)
-            CK(cudaMemcpyAsync(C.hout + path_at, d.path, sizeof(int) * COLS, cudaMemcpyDeviceToHost, s));
+    if (packed) CK(cudaMemcpyAsync(C.hout + lnl_at, d.lnl, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+    for (int k = 0; k < pieces; k++) {
+        cudaEvent_t landed = C.gev[2 * MAXG + (k & 1)];
+        if (k >= 2) {
+            CK(cudaEventSynchronize(landed));
+            std::vector<Ctx::Copy> out;
+            piece(k - 2, out);
+            hand_over(C, out);
+        }
+        const size_t lo = k * PIECE;
+        CK(cudaMemcpyAsync(C.hout + path_at + (k & 1) * PIECE, (char *)d.path + lo, std::min(PIECE, path_bytes - lo),
+                           cudaMemcpyDeviceToHost, s));
+        CK(cudaEventRecord(landed, s));
     }
     CK(cudaMemcpyAsync(C.hout + C.err_off, d.err, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
     if (T) CK(cudaEventRecord(C.ev[7], s));
@@ -836,9 +865,7 @@ int ctx_complete(Ctx &C, std::string &err) {
         C.copies.clear();
         return -4;
     }
-    std::vector<HostCopy> copies;
-    for (const Ctx::Copy &c : C.copies) copies.push_back({c.dst, C.hout + c.off, c.bytes});
-    parallel_copy(copies);
+    hand_over(C, C.copies);
     C.copies.clear();
     return 0;
 }

@@ -65,3 +65,16 @@ def test_marginals_wanted_later_in_a_context(n):
             for r, w in zip(c.finish(), want):
                 assert np.array_equal(r.path, w.path)
                 assert not post or np.array_equal(r.posterior, w.posterior)
+
+
+def test_paths_longer_than_the_staging():
+    """18 problems of a million columns (72 MB of paths, in pieces of 32 MB through two buffers), one
+    of them without a path."""
+    p = simulate(3, 1000003, 9, ntimes=8, rho=1e-11)
+    u = [np.random.default_rng(i).random(p.seqlen) for i in range(18)]
+    bound, outs, got, keep = api._bind_batch([p] * 18, "fp32", False, True, False, u)
+    outs[4].path = None
+    assert capi.load().awg_run_batch(bound, outs, 18, capi.AWG_FP32) == 0
+    for q in (0, 3, 5, 7, 8, 9, 16, 17):  # pieces end in problems 8 and 16
+        assert np.array_equal(got[q][0].path, api.sample_path(p, u[q], precision="fp32"))
+    api.release_memory()
