@@ -246,8 +246,13 @@ __global__ void k_backward(BatchDev d, int maxS, double *bw_out) {
                 float slo = 0.0f;
                 if (j == src.y || j == src.x) {
                     const F *row = (j == src.y) ? cr : rr;
-                    for (int k = 0; k < Sm; k++)
-                        if (row[k] > F(0)) s += row[k] * g[k];
+                    // one thread's: its loads go ahead of the sum (20 of a tree's 220 us at 3,977
+                    // states went to waiting for them one by one)
+#pragma unroll 8
+                    for (int k = 0; k < Sm; k++) {
+                        const F r = row[k], more = s + r * g[k];
+                        s = r > F(0) ? more : s;
+                    }
                 } else if (determ[j] >= 0) {
                     if constexpr (BTab<F>::split) {
                         const F2 x{g[determ[j]], glo[determ[j]]};
