@@ -39,7 +39,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "HMM state-cells/s fwd+traceback, batched FP32 vs plain FP64 @<=1e-5 err; p50/p99"
-FWD_DRAM_BYTES_PER_CELL = 7.26  # forward kernel, ncu capture summarised in profiles/
+FWD_DRAM_BYTES_PER_CELL = 7.13  # k_forward32, ncu capture: profiles/forward_traffic_k64_1e5.md
 UNIT = "state-cells/s"
 
 
@@ -680,7 +680,7 @@ def main():
                      "frac": achieved / hbm,
                      # DRAM bytes of the forward launches: ncu dram__bytes_read.sum +
                      # dram__bytes_write.sum of one k = 64, 100,000-column launch
-                     # (--one-instance 64,100000), 7.26 B per state-cell, scaled to this
+                     # (--one-instance 64,100000), 7.13 B per state-cell, scaled to this
                      # step's cells (profiles/forward_traffic_k64_1e5.md)
                      "traffic": FWD_DRAM_BYTES_PER_CELL * cells, "peak_source": src,
                      "kernel": "forward (k_forward32), 4 B of FP32 table written per cell, "
