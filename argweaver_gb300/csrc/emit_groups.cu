@@ -264,49 +264,49 @@ __device__ void emit_group(const BatchDev &d, const BlockDev &B, const InstDev &
             }
             __syncwarp();
         } else {
-        // two states per lane at a time: independent chains the scheduler can interleave (the
-        // second one repeats the first where it would run past S)
-        df ref = df();
-        for (int k0 = lane; k0 < t.S; k0 += 64) {
-            const int k1 = k0 + 32 < t.S ? k0 + 32 : k0;
-            const df v0 = state_v(k0), v1 = state_v(k1);
-            ed[k0] = v0;
-            ed[k1] = v1;
-            ref = fmax(ref, fmax(v0, v1));
-        }
-        if (penalty < 1.0) {
-            // states that break the infinite-sites model times the penalty (emit.cpp:847-862);
-            // below FP32's range that leaves the ratio 0, written as the smallest negative
-            // value below
-            const df pen(penalty);
-            ref = df();
-            for (int kb = 0; kb < t.S; kb += 32) {
-                const int k = kb + lane;
-                const bool ok = state_ok(vword, k < t.S ? t.states[k].x & 0xffff : 0);
-                if (k < t.S) {
-                    if (!ok) ed[k] = ed[k] * pen;
-                    ref = fmax(ref, ed[k]);
+            // two states per lane at a time: independent chains the scheduler can interleave (the
+            // second one repeats the first where it would run past S)
+            df ref = df();
+            for (int k0 = lane; k0 < t.S; k0 += 64) {
+                const int k1 = k0 + 32 < t.S ? k0 + 32 : k0;
+                const df v0 = state_v(k0), v1 = state_v(k1);
+                ed[k0] = v0;
+                ed[k1] = v1;
+                ref = fmax(ref, fmax(v0, v1));
+            }
+            if (penalty < 1.0) {
+                // states that break the infinite-sites model times the penalty (emit.cpp:847-862);
+                // below FP32's range that leaves the ratio 0, written as the smallest negative
+                // value below
+                const df pen(penalty);
+                ref = df();
+                for (int kb = 0; kb < t.S; kb += 32) {
+                    const int k = kb + lane;
+                    const bool ok = state_ok(vword, k < t.S ? t.states[k].x & 0xffff : 0);
+                    if (k < t.S) {
+                        if (!ok) ed[k] = ed[k] * pen;
+                        ref = fmax(ref, ed[k]);
+                    }
                 }
             }
-        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ref = fmax(ref, __shfl_xor_sync(FULL, ref, o));
-        // 1 / (4 e_ref): the FP32 reciprocal and one Newton step in double-float
-        const df one(1.0f, 0.0f);
-        const df y0(1.0f / ref.hi, 0.0f);
-        const df inv1 = y0 + y0 * (one - ref * y0);
-        float *row = d.var32 + B.var0 + (size_t)vrow * t.S;
-        for (int k = lane; k < t.S; k += 32) {
-            // e_k / e_ref; the largest state's r can round a hair above 1, so its complement
-            // is clamped at +0 (a negative value would read as a ratio, i.e. an emission near
-            // zero)
-            const df r = ed[k] * inv1;
-            float v = r.hi >= 0.5f ? fmaxf((one - r).hi, 0.0f) : -r.hi;
-            if (r.hi < 0.5f && v == 0.0f) v = -__int_as_float(1);  // stays a ratio
-            row[k] = v;
-        }
-        if (lane == 0) d.vref[B.vrow0 + vrow] = .25 * (double)ref;
-        __syncwarp();
+            for (int o = 16; o > 0; o >>= 1) ref = fmax(ref, __shfl_xor_sync(FULL, ref, o));
+            // 1 / (4 e_ref): the FP32 reciprocal and one Newton step in double-float
+            const df one(1.0f, 0.0f);
+            const df y0(1.0f / ref.hi, 0.0f);
+            const df inv1 = y0 + y0 * (one - ref * y0);
+            float *row = d.var32 + B.var0 + (size_t)vrow * t.S;
+            for (int k = lane; k < t.S; k += 32) {
+                // e_k / e_ref; the largest state's r can round a hair above 1, so its complement
+                // is clamped at +0 (a negative value would read as a ratio, i.e. an emission near
+                // zero)
+                const df r = ed[k] * inv1;
+                float v = r.hi >= 0.5f ? fmaxf((one - r).hi, 0.0f) : -r.hi;
+                if (r.hi < 0.5f && v == 0.0f) v = -__int_as_float(1);  // stays a ratio
+                row[k] = v;
+            }
+            if (lane == 0) d.vref[B.vrow0 + vrow] = .25 * (double)ref;
+            __syncwarp();
         }
     }
 }

@@ -109,117 +109,117 @@ __device__ void warp_sample_group(int n, const F *const (&cg)[G], const F *trans
     const int lane = threadIdx.x & 31;
     const int chunk = (n + 31) >> 5;
     const int lo = imin(lane * chunk, n), hi = imin(lo + chunk, n);
-                // every column's chunk sums under the current row, as warp_sample forms them
-                F l0[G], l1[G];
-    #pragma unroll
-                for (int g = 0; g < G; g++) l0[g] = l1[g] = F(0);
-                int j = lo;
-                for (; j + 1 < hi; j += 2) {
-                    const F t0 = trans[j], t1 = trans[j + 1];
-    #pragma unroll
-                    for (int g = 0; g < G; g++) {
-                        l0[g] = fma(cg[g][j], t0, l0[g]);
-                        l1[g] = fma(cg[g][j + 1], t1, l1[g]);
-                    }
+    // every column's chunk sums under the current row, as warp_sample forms them
+    F l0[G], l1[G];
+#pragma unroll
+    for (int g = 0; g < G; g++) l0[g] = l1[g] = F(0);
+    int j = lo;
+    for (; j + 1 < hi; j += 2) {
+        const F t0 = trans[j], t1 = trans[j + 1];
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            l0[g] = fma(cg[g][j], t0, l0[g]);
+            l1[g] = fma(cg[g][j + 1], t1, l1[g]);
+        }
+    }
+    if (j < hi) {
+        const F t0 = trans[j];
+#pragma unroll
+        for (int g = 0; g < G; g++) l0[g] = fma(cg[g][j], t0, l0[g]);
+    }
+    F incl[G];
+#pragma unroll
+    for (int g = 0; g < G; g++) incl[g] = l0[g] + l1[g];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            const F v = __shfl_up_sync(0xffffffffu, incl[g], o);
+            if (lane >= o) incl[g] += v;
+        }
+    }
+    // every column's draw, all G interleaved (finish_sample's steps, column-wise)
+    F pick[G], carry[G];
+    int slo[G], shi[G];
+#pragma unroll
+    for (int g = 0; g < G; g++) {
+        F excl = __shfl_up_sync(0xffffffffu, incl[g], 1);
+        if (lane == 0) excl = 0;
+        const F total = __shfl_sync(0xffffffffu, incl[g], 31);
+        pick[g] = (F)ug[g] * total;
+        const unsigned hit = __ballot_sync(0xffffffffu, incl[g] >= pick[g] && hi > lo);
+        const int src = hit ? __ffs(hit) - 1 : 0;
+        slo[g] = imin(src * chunk, n);
+        shi[g] = hit ? imin(slo[g] + chunk, n) : slo[g];  // empty: no rescan
+        carry[g] = __shfl_sync(0xffffffffu, excl, src);
+        res[g] = hit ? shi[g] - 1 : n - 1;
+    }
+    unsigned open = 0;  // columns whose pick is not found yet
+#pragma unroll
+    for (int g = 0; g < G; g++)
+        if (shi[g] > slo[g]) open |= 1u << g;
+    if (chunk <= 16) {
+        // short chunks: lane g rescans column g's chosen chunk in order, one product
+        // and one add per state, the G columns side by side (a 32-lane scan per column
+        // costs five warp-wide adds however few states the chunk holds: on the FP64
+        // path each holds the sub-partition's FP64 pipe for about 64 cycles)
+        int mine = 0;
+        if (lane < G) {
+            F mpick = 0, run = 0;
+            int mslo = 0, mshi = 0;
+            const F *mc = cg[0];
+#pragma unroll
+            for (int g = 0; g < G; g++)
+                if (lane == g) {
+                    mpick = pick[g];
+                    run = carry[g];
+                    mslo = slo[g];
+                    mshi = (open >> g) & 1 ? shi[g] : slo[g];
+                    mine = res[g];
+                    mc = cg[g];
                 }
-                if (j < hi) {
-                    const F t0 = trans[j];
-    #pragma unroll
-                    for (int g = 0; g < G; g++) l0[g] = fma(cg[g][j], t0, l0[g]);
+            for (int jj = mslo; jj < mshi; jj++) {
+                run += mc[jj] * trans[jj];
+                if (run >= mpick) {
+                    mine = jj;
+                    break;
                 }
-                F incl[G];
-    #pragma unroll
-                for (int g = 0; g < G; g++) incl[g] = l0[g] + l1[g];
-    #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-    #pragma unroll
-                    for (int g = 0; g < G; g++) {
-                        const F v = __shfl_up_sync(0xffffffffu, incl[g], o);
-                        if (lane >= o) incl[g] += v;
-                    }
-                }
-                // every column's draw, all G interleaved (finish_sample's steps, column-wise)
-                F pick[G], carry[G];
-                int slo[G], shi[G];
-    #pragma unroll
-                for (int g = 0; g < G; g++) {
-                    F excl = __shfl_up_sync(0xffffffffu, incl[g], 1);
-                    if (lane == 0) excl = 0;
-                    const F total = __shfl_sync(0xffffffffu, incl[g], 31);
-                    pick[g] = (F)ug[g] * total;
-                    const unsigned hit = __ballot_sync(0xffffffffu, incl[g] >= pick[g] && hi > lo);
-                    const int src = hit ? __ffs(hit) - 1 : 0;
-                    slo[g] = imin(src * chunk, n);
-                    shi[g] = hit ? imin(slo[g] + chunk, n) : slo[g];  // empty: no rescan
-                    carry[g] = __shfl_sync(0xffffffffu, excl, src);
-                    res[g] = hit ? shi[g] - 1 : n - 1;
-                }
-                unsigned open = 0;  // columns whose pick is not found yet
-    #pragma unroll
-                for (int g = 0; g < G; g++)
-                    if (shi[g] > slo[g]) open |= 1u << g;
-                if (chunk <= 16) {
-                    // short chunks: lane g rescans column g's chosen chunk in order, one product
-                    // and one add per state, the G columns side by side (a 32-lane scan per column
-                    // costs five warp-wide adds however few states the chunk holds: on the FP64
-                    // path each holds the sub-partition's FP64 pipe for about 64 cycles)
-                    int mine = 0;
-                    if (lane < G) {
-                        F mpick = 0, run = 0;
-                        int mslo = 0, mshi = 0;
-                        const F *mc = cg[0];
-    #pragma unroll
-                        for (int g = 0; g < G; g++)
-                            if (lane == g) {
-                                mpick = pick[g];
-                                run = carry[g];
-                                mslo = slo[g];
-                                mshi = (open >> g) & 1 ? shi[g] : slo[g];
-                                mine = res[g];
-                                mc = cg[g];
-                            }
-                        for (int jj = mslo; jj < mshi; jj++) {
-                            run += mc[jj] * trans[jj];
-                            if (run >= mpick) {
-                                mine = jj;
-                                break;
-                            }
-                        }
-                    }
-    #pragma unroll
-                    for (int g = 0; g < G; g++) res[g] = __shfl_sync(0xffffffffu, mine, g);
-                    open = 0;
-                }
-                for (int b = 0; open; b += 32) {
-                    F x[G];
-    #pragma unroll
-                    for (int g = 0; g < G; g++) {
-                        const int jj = slo[g] + b + lane;
-                        x[g] = ((open >> g) & 1) && jj < shi[g] ? cg[g][jj] * trans[jj] : F(0);
-                    }
-    #pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-    #pragma unroll
-                        for (int g = 0; g < G; g++) {
-                            const F v = __shfl_up_sync(0xffffffffu, x[g], o);
-                            if (lane >= o) x[g] += v;
-                        }
-                    }
-    #pragma unroll
-                    for (int g = 0; g < G; g++) {
-                        if (!((open >> g) & 1)) continue;
-                        const int jj = slo[g] + b + lane;
-                        const unsigned got =
-                            __ballot_sync(0xffffffffu, jj < shi[g] && carry[g] + x[g] >= pick[g]);
-                        if (got) {
-                            res[g] = slo[g] + b + __ffs(got) - 1;
-                            open &= ~(1u << g);
-                        } else {
-                            carry[g] += __shfl_sync(0xffffffffu, x[g], 31);
-                            if (slo[g] + b + 32 >= shi[g]) open &= ~(1u << g);
-                        }
-                    }
-                }
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < G; g++) res[g] = __shfl_sync(0xffffffffu, mine, g);
+        open = 0;
+    }
+    for (int b = 0; open; b += 32) {
+        F x[G];
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            const int jj = slo[g] + b + lane;
+            x[g] = ((open >> g) & 1) && jj < shi[g] ? cg[g][jj] * trans[jj] : F(0);
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                const F v = __shfl_up_sync(0xffffffffu, x[g], o);
+                if (lane >= o) x[g] += v;
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            if (!((open >> g) & 1)) continue;
+            const int jj = slo[g] + b + lane;
+            const unsigned got =
+                __ballot_sync(0xffffffffu, jj < shi[g] && carry[g] + x[g] >= pick[g]);
+            if (got) {
+                res[g] = slo[g] + b + __ffs(got) - 1;
+                open &= ~(1u << g);
+            } else {
+                carry[g] += __shfl_sync(0xffffffffu, x[g], 31);
+                if (slo[g] + b + 32 >= shi[g]) open &= ~(1u << g);
+            }
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1034,10 +1034,10 @@ __global__ void __launch_bounds__(32 * TW) k_traceback_lots(BatchDev d, int buf_
                     const double *cp = column(mc);
                     double before = 0.0, after = 0.0;
                     int j = q;
-    #pragma unroll 4
+#pragma unroll 4
                     for (; j < k; j += lanes) before = fma(cp[j], trans[j], before);
                     j += j == k ? lanes : 0;
-    #pragma unroll 4
+#pragma unroll 4
                     for (; j < S; j += lanes) after = fma(cp[j], trans[j], after);
                     for (int o = 1; o < lanes; o <<= 1) {
                         before += __shfl_xor_sync(FULL, before, o);
